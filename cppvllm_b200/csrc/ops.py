@@ -7,6 +7,7 @@ tensor that is not on a CUDA device, or a missing compiler, raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 import sys
@@ -1114,6 +1115,97 @@ def lru_step(out: torch.Tensor, packed: torch.Tensor, y_off: int, x_off: int, bi
         _ptr(neg_softplus), sp, sf, c_int(n_slots), _ptr(cu_seqlens), _ptr(state_slots), _ptr(positions), c_int(num_seqs), c_int(W), c_int(parts),
         c_int(taps), c_int(packed.stride(0)), c_int(y_off), c_int(x_off), c_int(dtype_code(packed.dtype)), _ptr(error_flag(out.device)),
         _stream()), "lru_step")
+    return out
+
+
+# ---- prompt portions over cache entries on the tcgen05 tensor cores ---------------------------------------------------
+
+_attn_entries = None
+
+
+def _attn_entries_lib():
+    global _attn_entries
+    if _attn_entries is None:
+        lib = load_library("attn_entries")
+        P, i, f = c_void_p, c_int, c_float      # declared, so that a call converts plain numbers itself (48 objects a call cost 5 us)
+        lib.cvb_attn_entries_tcgen05.argtypes = [P, i, P, i, P, P, i, P, P] + [i] * 14 + [f, f, P, i, P, P, i, P, P, i, i, f, i, i, P, c_int64, P, P, P]
+        lib.cvb_attn_entries_tcgen05.restype = c_int
+        lib.cvb_attn_entries_supported.restype = c_int
+        _attn_entries = lib
+    return _attn_entries
+
+
+@functools.lru_cache(maxsize=256)
+def _attn_entries_shape(num_heads: int, num_kv_heads: int, dim: int, vdim: int, shared: bool, page_size: int, table_len: int) -> bool:
+    return bool(_attn_entries_lib().cvb_attn_entries_supported(c_int(num_heads), c_int(num_kv_heads), c_int(dim), c_int(vdim),
+                                                               c_int(1 if shared else 0), c_int(page_size), c_int(table_len)))
+
+
+# What a block costs outside its tiles (tensor memory, barriers, the query tiles, the output through shared memory) is more than an
+# mma.sync block's, so a step whose tokens all see less than one tile of entries stays there.  Measured, a layer of 64 tokens of a new
+# prompt / 4 tokens behind 124 / 128 tokens of a new prompt, us, mma.sync against tcgen05: chunks with cap, distance term and gate at
+# 32/8 heads 31 / 36 / 41 against 39 / 40 / 42, a bias per distance at 16/8 heads 22 / 24 / 27 against 26 / 24 / 27, keys that are values at
+# 32/8 heads 28 / 28 / 34.5 against 29.5 / 24 / 32, chunks with a gate at 16/8 heads 27 / 27 / 33 against 23 / 21 / 25.
+ENTRIES_MIN_VISIBLE = 128
+
+
+def attn_entries_supported(q: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor], num_heads: int, num_kv_heads: int, dim: int, vdim: int,
+                           page_size: int, visible: int, shared: bool = False, table_len: int = 0) -> bool:
+    """Whether the tcgen05 kernel takes a portion (csrc/attention_entries_tcgen05.cu): bf16, keys of 64 or 128 elements and values as wide
+    (`shared`: the entry is key and value; 96 of 128 too), pages of 2^n >= 16 tokens, a distance table of `table_len` entries per head that
+    fits beside its tiles, rows of q, out and a gate per element on 16-byte boundaries (the mma.sync kernels ask for less), and tokens that
+    see at least ENTRIES_MIN_VISIBLE entries at most."""
+    def rows16(t):
+        return t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    return (visible >= ENTRIES_MIN_VISIBLE and q.dtype == torch.bfloat16
+            and _attn_entries_shape(num_heads, num_kv_heads, dim, vdim, shared, page_size, table_len)
+            and rows16(q) and rows16(out) and (gate is None or gate.shape[1] == num_heads or rows16(gate)))
+
+
+def attn_entries_tcgen05(out: torch.Tensor, q: torch.Tensor, pages: torch.Tensor, block_tables: torch.Tensor, cu_seqlens: torch.Tensor,
+                         positions: torch.Tensor, q_lens, num_heads: int, num_kv_heads: int, dim: int, vdim: int, page_size: int, scale: float,
+                         visible: int, workspace=None, shared: bool = False, planes: int = 1, chunk: int = 0, window: int = 0, pool: int = 0,
+                         keep_first: int = 0, softcap: float = 0.0, bias: Optional[torch.Tensor] = None, r1: Optional[torch.Tensor] = None,
+                         r2: Optional[torch.Tensor] = None, table_len: int = 0, sink: Optional[torch.Tensor] = None,
+                         gate: Optional[torch.Tensor] = None, out_scale: float = 1.0, pieces: int = 0,
+                         min_rounds: int = 0) -> torch.Tensor:
+    """Attention of prompt portions (and single tokens among them) over pages [plane, kv head, slot, dim + vdim] of entries that hold a key and
+    its value, or (`shared`) [kv head, slot, dim] whose first vdim elements are the value: the masks and terms of attn_masked_bf16,
+    attn_bias_bf16 (`bias`) and attn_keys_bf16.  `table_len`: distances that `bias` or `r1`, `r2` distinguish (r1, r2: at least as many as
+    the mask lets through).  `visible`: the most entries a token can see (it decides whether long query blocks are worked on by several
+    blocks, whose shares go through scratch of the `workspace`; `pieces`, `min_rounds` > 0 force that choice)."""
+    H, G, bf, f32 = num_heads, num_kv_heads, torch.bfloat16, torch.float32
+    for t, dtype in ((out, bf), (q, bf), (gate, bf), (pages, bf), (block_tables, torch.int32), (cu_seqlens, torch.int32), (positions, torch.int32),
+                     (bias, f32), (r1, f32), (r2, f32), (sink, f32)):
+        if t is not None and (t.dtype != dtype or not t.is_cuda or not (t is out or t is q or t is gate or t.is_contiguous())):
+            raise KernelError("attn_entries_tcgen05: CUDA tensors; queries, pages, gate and output bf16, tables and positions int32, terms float32; "
+                              "all but queries, gate and output contiguous")
+    if block_tables.dim() != 2 or any(t is not None and t.numel() != H for t in (r1, r2, sink)) or (bias is not None and (bias.dim() != 2 or bias.shape[0] != H)):
+        raise KernelError("attn_entries_tcgen05: block_tables [S, W]; r1, r2 and sink [H], bias [H, L]")
+    if q.dim() != 2 or q.shape[1] < H * dim or q.stride(1) != 1 or out.dim() != 2 or out.shape[1] != H * vdim or out.stride(1) != 1:
+        raise KernelError("attn_entries_tcgen05: q [T, >= H * dim], out [T, H * vdim]")
+    if gate is not None and (gate.shape[1] not in (H, H * vdim) or gate.stride(1) != 1):
+        raise KernelError("attn_entries_tcgen05: gate bf16 [T, H] or [T, H * vdim]")
+    num_tiles = prefill_tiles_tcgen05(q_lens, H, G, skip_single=False)
+    pieces = pieces or prefill_pieces_tcgen05(num_tiles, G, visible)
+    scratch = counts = None
+    if workspace is not None:
+        # as for attn_prefill_tcgen05: a grid that is cut has at most one block per SM after the cut
+        scratch = workspace.flat(f"attn_entries_pieces_{vdim}", PREFILL_SMS * 2 * (vdim + 2) * 128, f32)
+        counts = workspace.flat("attn_prefill_piece_counts", PREFILL_SMS, torch.int32)
+    if pieces > 1 and (scratch is None or counts.numel() < num_tiles * G):
+        raise KernelError("attn_entries_tcgen05: pieces need a workspace and at most as many query blocks as there are SMs")
+    num_pages = pages.numel() // (planes * G * page_size * (dim if shared else dim + vdim))
+
+    def at(t):
+        return t.data_ptr() if t is not None else None
+    _check(_attn_entries_lib().cvb_attn_entries_tcgen05(
+        out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
+        cu_seqlens.data_ptr(), positions.data_ptr(), len(q_lens), num_tiles, H, G, dim, vdim, 1 if shared else 0, page_size, planes, num_pages, chunk,
+        window, pool, keep_first, scale, softcap, at(bias), bias.shape[1] if bias is not None else 0, at(r1), at(r2), table_len, at(sink), at(gate),
+        gate.stride(0) if gate is not None else 0, 1 if gate is not None and gate.shape[1] != H else 0, out_scale, pieces,
+        min_rounds or PREFILL_MIN_ROUNDS, at(scratch), scratch.numel() if scratch is not None else 0, at(counts),
+        error_flag(q.device).data_ptr(), _stream()), "attn_entries_tcgen05", kernels=2 if pieces > 1 else 1)
     return out
 
 

@@ -83,9 +83,13 @@ class KeysAttention(Mixer):
         if not self.force_general and ops.attn_keys_supported(qk.dtype, H, KV, hd, qk.shape[1]):
             q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             single = ctx.all_decode and ctx.num_tokens == ctx.num_seqs
+            visible = min(ctx.max_kv_len, self.window + self.keep_first) if self.window > 0 else ctx.max_kv_len
+            if not single and ops.attn_entries_supported(qk, att, None, H, KV, hd, hd, g.page_size, visible, shared=True):
+                ops.attn_entries_tcgen05(att, qk, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, KV, hd, hd, g.page_size,
+                                         self.scale, visible, workspace=self.rt.workspace, shared=True, window=self.window, keep_first=self.keep_first)
+                return
             splits, scratch = 1, None
             if single:
-                visible = min(ctx.max_kv_len, self.window + self.keep_first) if self.window > 0 else ctx.max_kv_len
                 splits = ops.attn_keys_decode_splits(ctx.num_seqs, KV, visible)
                 if splits > 1:
                     most = ops.attn_keys_scratch_floats(self.rt.workspace.max_seqs, KV, hd, 8)

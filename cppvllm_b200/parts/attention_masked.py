@@ -15,8 +15,8 @@
 
 The cache holds, per token and kv head, the key and behind it the value; with pooled blocks a second plane of the same pages
 holds the blocks' means at the place of position b (pages [plane, kv head, slot, dim + vdim]), written by the step that
-brings a block's last token.  float32 and any sizes run on the general kernel; bf16 with sizes the tensor-core kernel takes
-runs there (csrc/attention_masked.cu).
+brings a block's last token.  float32 and any sizes run on the general kernel; bf16 with sizes the tensor-core kernels take
+runs there (csrc/attention_masked.cu, portions at heads of 64 or 128 csrc/attention_entries_tcgen05.cu).
 """
 from __future__ import annotations
 
@@ -149,20 +149,33 @@ class MaskedAttention(Mixer):
         self.attend(out, q, gate, ctx, cache, g, scale)
         return out
 
+    def _visible(self, ctx) -> int:
+        """What a token can see at most: its chunk, or its window and the pooled blocks before it."""
+        seen = ctx.max_kv_len
+        if self.chunk:
+            seen = min(seen, self.chunk)
+        if self.window:
+            seen = min(seen, self.window + self.keep_first + (ctx.max_kv_len // self.pool if self.pool else 0))
+        return seen
+
     def attend(self, att, q, gate, ctx, cache, g, out_scale=1.0):
         H, G, dk, dv = self.num_heads, self.num_kv_heads, self.dim, self.vdim
+        # distances that the mask lets through, for the tcgen05 kernel's table; without a bound the term goes to the other kernels
+        reach = min([n for n in (self.chunk, self.window if not self.keep_first else 0) if n], default=0) if self.r1 is not None else 0
+        if (not self.force_general and not (ctx.all_decode and ctx.num_tokens == ctx.num_seqs) and (self.r1 is None or reach)
+                and ops.attn_entries_supported(q, att, gate, H, G, dk, dv, g.page_size, self._visible(ctx), table_len=reach)):
+            q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
+            ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv, g.page_size,
+                                     self.scale, self._visible(ctx), workspace=self.rt.workspace, planes=self.planes, chunk=self.chunk,
+                                     window=self.window, pool=self.pool, keep_first=self.keep_first, softcap=self.softcap, r1=self.r1, r2=self.r2,
+                                     table_len=reach, sink=self.sinks, gate=gate, out_scale=out_scale)
+            return
         if not self.force_general and ops.attn_masked_supported(q.dtype, H, G, dk, dv) and ops.attn_masked_pairs(att, gate, H):
             q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             single = ctx.all_decode and ctx.num_tokens == ctx.num_seqs and H // G <= 16
             splits, scratch = 1, None
             if single:
-                # what a decoded token can see at most: its chunk, or its window and the pooled blocks before it
-                seen = ctx.max_kv_len
-                if self.chunk:
-                    seen = min(seen, self.chunk)
-                if self.window:
-                    seen = min(seen, self.window + self.keep_first + (ctx.max_kv_len // self.pool if self.pool else 0))
-                splits = ops.attn_masked_decode_splits(ctx.num_seqs, G, seen)
+                splits = ops.attn_masked_decode_splits(ctx.num_seqs, G, self._visible(ctx))
                 if splits > 1:
                     most = ops.attn_keys_scratch_floats(self.rt.workspace.max_seqs, G, dv, 8)
                     scratch = self.rt.workspace.flat(f"attn_masked_parts_{G}_{dv}", most, torch.float32)
