@@ -44,6 +44,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "moe": ["moe.cu"],
     "latent": ["latent.cu"],
     "recurrent": ["recurrent.cu"],
+    "delta": ["delta_chunks.cu"],
     "lru": ["lru.cu"],
     "linear": ["linear.cu"],
     "ssd": ["ssd.cu"],

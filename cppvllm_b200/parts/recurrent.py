@@ -215,7 +215,11 @@ class HeadDeltaMixer(Mixer):
                        ctx.seq_of_token, ctx.cu_seqlens, ctx.state_slots, H, G, dk, dv, decay_dim=1)
         ops.conv_history(state, self.matrix_floats, packed, 0, self.channels, self.taps, ctx.cu_seqlens, ctx.state_slots, S)
         o = ws.rows("rec_o", T, H * dv, f32)
-        ops.delta_scan(o, qn, kn, vv, gg, bb, state, ctx.cu_seqlens, ctx.state_slots, S, H, G, dk, dv, decay_dim=1)
+        q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * S
+        if not self.rt.plain_kernels and ops.delta_chunks_supported(x.dtype, dk, dv, state, q_lens):
+            ops.delta_chunks(o, qn, kn, vv, gg, bb, state, ctx.cu_seqlens, ctx.state_slots, q_lens, H, G, dk, dv, ws)
+        else:
+            ops.delta_scan(o, qn, kn, vv, gg, bb, state, ctx.cu_seqlens, ctx.state_slots, S, H, G, dk, dv, decay_dim=1)
         y = ops.gated_norm(ws.rows("rec_y", T, H * dv, x.dtype), o, packed[:, self.g_off:self.g_off + H * dv], self.w_norm, H, self.eps,
                            gate_act="silu")
         return _project(self.rt, y, self.w_o, ws.rows("attn_proj", T, self.hidden_size, x.dtype), T)
