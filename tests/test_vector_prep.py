@@ -44,3 +44,29 @@ def test_head_gate_and_turned_queries(dtype, per_element):
     assert bool((got[..., :rank] == 0).all())
     bound = r.abs().amax(-1, keepdim=True) * 1.5
     assert bool(((got[..., rank:] - want).abs() <= tol * bound + 1e-30).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, BF])
+@pytest.mark.parametrize("nq,G,dk,dv,write", [(512, 2, 64, 32, True), (2048, 8, 128, 128, True), (6144, 2, 128, 128, True), (8192, 8, 64, 64, False)])
+def test_norm_over_whole_projections(dtype, nq, G, dk, dv, write):
+    from cppvllm_b200.csrc import ops
+    gen = torch.Generator().manual_seed(nq)
+    T, page, eps = 9, 16, 1e-5
+    packed = rnd(gen, T, nq + (G * (dk + dv) if write else 0) + 8, dtype=dtype)
+    wq, wk = rnd(gen, nq) * 0.1 + 1, rnd(gen, G * dk) * 0.1 + 1
+    q, pages = torch.zeros(T, nq, dtype=dtype, device=DEV), torch.zeros(2, G, page, dk + dv, dtype=dtype, device=DEV)
+    slots, pos = torch.randperm(2 * page, generator=gen)[:T], torch.arange(T) * 50
+    ops.wide_qk_prep(q, packed, wq, i32(pos), eps, 0.25, 128, G, dk, dv, **(dict(pages=pages, k_weight=wk, slots=i32(slots), page_size=page) if write else {}))
+    ops.check_device_errors(torch.device(DEV))
+
+    def norm(x, w):
+        return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w.double()
+    temp = torch.tensor([1 + 0.25 * math.log((int(p) + 1) // 128 + 1) for p in pos], dtype=torch.float64, device=DEV)[:, None]
+    tol = 2 ** -8 if dtype == BF else 2e-6
+    want = norm(packed[:, :nq].double(), wq) * temp
+    assert bool(((q.double() - want).abs() <= tol * want.abs() + 1e-30).all())
+    if write:
+        k = norm(packed[:, nq:nq + G * dk].double(), wk).view(T, G, dk)
+        v = packed[:, nq + G * dk:nq + G * (dk + dv)].double().view(T, G, dv)
+        got = pages.double().movedim(2, 1)[slots.to(DEV) // page, slots.to(DEV) % page]
+        assert bool(((got[..., :dk] - k).abs() <= tol * k.abs() + 1e-30).all()) and torch.equal(got[..., dk:], v)
