@@ -70,3 +70,21 @@ def test_norm_over_whole_projections(dtype, nq, G, dk, dv, write):
         v = packed[:, nq + G * dk:nq + G * (dk + dv)].double().view(T, G, dv)
         got = pages.double().movedim(2, 1)[slots.to(DEV) // page, slots.to(DEV) % page]
         assert bool(((got[..., :dk] - k).abs() <= tol * k.abs() + 1e-30).all()) and torch.equal(got[..., dk:], v)
+
+
+@pytest.mark.parametrize("T,D,top,weighted", [(5, 1032, 2, True), (3, 8, 6, True), (2, 2048, 1, False), (4, 20, 3, True)])
+def test_sum_of_a_tokens_expert_rows(T, D, top, weighted):
+    from ctypes import c_int
+    from cppvllm_b200.csrc import ops
+    gen = torch.Generator().manual_seed(D)
+    rows, x, y = rnd(gen, T * top + 3, D, dtype=BF), rnd(gen, T, D, dtype=BF), torch.zeros(T, D, dtype=BF, device=DEV)
+    slot = torch.randperm(T * top + 3, generator=gen)[:T * top].view(T, top)
+    slot[-1, -1] = -1                                    # the input itself
+    w = torch.rand(T, top, generator=gen)
+    wd, sd = w.to(DEV), i32(slot)
+    assert ops._moe_lib().cvb_combine_pairs_bf16(ops._ptr(y), ops._ptr(rows), ops._ptr(x), ops._ptr(sd), ops._ptr(wd if weighted else None), c_int(T),
+                                                 c_int(D), c_int(top), ops._stream()) == 0
+    src = torch.where((slot >= 0)[..., None], rows.cpu().double()[slot.clamp(min=0)], x.cpu().double()[:, None])
+    terms = src * (w.double()[..., None] if weighted else 1.0)
+    # one rounding to bf16 behind float sums of a few terms
+    assert bool(((y.cpu().double() - terms.sum(1)).abs() <= 2 ** -8 * terms.sum(1).abs() + 1e-6 * terms.abs().sum(1)).all())
