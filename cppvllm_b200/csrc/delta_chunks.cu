@@ -7,16 +7,15 @@
 // in front of it, a chunk's tokens are one triangular system
 //   (I + L) U = b (V - e K S_0),  L_ij = b_i D_ij (k_i . k_j) for j < i          W = (I + L)^-1 b e K,  U~ = (I + L)^-1 b V
 //   U = U~ - W S_0;   O = e Q S_0 + A U,  A_ij = D_ij (q_i . k_j) for j <= i;     S = e_31 S_0 + K^T (D_31,j U_j)
-// delta_prepare_kernel makes W, U~, A, e and D_31 of every (chunk, head) side by side; delta_chain_kernel walks the chunks of a
-// (request, head, slice of value columns) with S in registers, two barriers and about 24 + 12 products a warp and chunk.  Decays are
+// delta_prepare_kernel makes W, U~, A, e and D_31 of every (chunk, head) side by side, from the packed projection; delta_chain_kernel walks the chunks of a
+// (request, head, slice of value columns) with S in registers, half of its warps on the chain and half on the outputs beside it.  Decays are
 // running products (never logarithms: g may be 0).
 //
 // Products run as `mma.sync.m16n8k16` with every float operand split into two bf16 (x = hi + lo, hi hi + hi lo + lo hi, float
 // accumulation): 2^-17 of an operand is lost, 1 / 64 of what the bf16 projection in front of the rule has rounded already.  W and U~ come
 // from a float substitution, one thread per column.  Steps in float32 stay on the scan.
 // Chunk images in scratch are laid out as the chain kernel wants them in shared memory (rows padded against ldmatrix conflicts), so a
-// chunk arrives by three bulk copies, two chunks ahead.  What bounds the chain: the mma.sync rate and the copies from the L2 (57 KB a
-// chunk and block).
+// chunk arrives by a few bulk copies, two chunks ahead.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "mma_tiles.cuh"
@@ -32,11 +31,13 @@ constexpr int kDHeadBytes = 2 * kDRowsBytes + 2 * kDC * kDLA * 2 + 2 * kDC * 4; 
 constexpr int kDKvBytes = 4 * kDRowsBytes;               // K hi, lo | Q hi, lo
 
 struct DeltaChunkParams {
-    const float* qn;                                     // [T, G * 128]
-    const float* kn;
-    const float* vv;                                     // [T, H * dv]
-    const float* gg;                                     // [T, H]
-    const float* bb;                                     // [T, H]
+    const __nv_bfloat16* packed;                         // rows of `stride` elements; from column qkv_off on q [G * 128], k [G * 128], v [H * dv]
+    int stride, qkv_off;
+    const float* conv_w;                                 // [channels, taps]
+    const float* ba;                                     // [T, 2 H]: the input strengths' logits, then the decays'
+    const float* dt_bias;                                // [H]
+    const float* a_log;
+    int64_t conv_off;                                    // where the convolution's history lies in a slot
     float* out;                                          // [T, H * dv]
     float* state;
     int64_t state_floats;
@@ -62,10 +63,6 @@ __device__ __forceinline__ float* u_image(const DeltaChunkParams& p, int lc, int
     return reinterpret_cast<float*>(base) + ((static_cast<int64_t>(lc) * p.H + h) * (p.dv / NB) + cb) * (kDC * (NB + 8));
 }
 
-__device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bfloat16& lo) {
-    hi = __float2bfloat16_rn(x);
-    lo = __float2bfloat16_rn(x - __bfloat162float(hi));
-}
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
     const float2 f = __bfloat1622float2(h);
@@ -73,21 +70,32 @@ __device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint3
     lo = pack2(x - f.x, y - f.y);
 }
 
-// Grid (chunk, head), 128 + dv threads: thread c < 128 solves for column c of W, the others for a column of U~.
-template <int NB>
+__device__ __forceinline__ float delta_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
+
+constexpr int kDLF = kDK + 4;                            // floats of a padded row of convolved channels
+constexpr int kDPair = 2;                                // heads of a kv head worked on together
+constexpr size_t kDPrepBytes = static_cast<size_t>(kDKvBytes) + 3 * kDC * kDLF * sizeof(float) +
+                               kDPair * (kDC * 36 + kDC * 33 + 2 * kDC) * sizeof(float);
+
+// Grid (chunk, kv head).  From the packed projection: convolutions, silu, unit vectors, decays and input strengths as recurrent.cu's delta_prep
+// makes them, then the kv head's image and, two heads at a time, the heads' images; nothing between the projection and the images travels
+// through memory.  (With delta_prep in front, a block per (chunk, head) and the heads' float rows read back, it was 66 + 49 us for 2,048
+// tokens of 16/8 heads; now 58, bound by instruction issue: 0.41 a cycle and scheduler with two blocks an SM.)
+template <int NB, int TAPS>
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const DeltaChunkParams p) {
     pdl_trigger();
     extern __shared__ __align__(128) unsigned char smem[];
     __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem);                    // hi, lo
     __nv_bfloat16* sQ = sK + 2 * kDC * kDLD;                                       // hi, lo
-    float* sL = reinterpret_cast<float*>(sQ + 2 * kDC * kDLD);                     // L transposed: [j][i], rows of 36
-    float* sD = sL + kDC * 36;                                                     // [i][j], rows of 33
-    float* sG = sD + kDC * 33;                                                     // g, b, e
-    float* sBeta = sG + kDC;
-    float* sE = sBeta + kDC;
+    float* sKf = reinterpret_cast<float*>(sQ + 2 * kDC * kDLD);                    // k, convolved, then of unit length
+    float* sV0 = sKf + kDC * kDLF;
+    float* sV1 = sV0 + kDC * kDLF;                                                 // the second head's v; before that, q
+    float* sL = sV1 + kDC * kDLF;                                                  // [head of the pair] L transposed: [j][i], rows of 36
+    float* sD = sL + kDPair * kDC * 36;                                            // [i][j], rows of 33
+    float* sG = sD + kDPair * kDC * 33;                                            // [head][b | e][32]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lc = blockIdx.x, h = blockIdx.y, share = p.H / p.G, kvh = h / share;
+    const int lc = blockIdx.x, kvh = blockIdx.y, share = p.H / p.G;
     // which request the chunk belongs to: the lanes of a warp take a request each (every warp does the same)
     const int chunk = p.c_first + lc;
     int seq = -1, ci = 0, before = 0;
@@ -111,141 +119,241 @@ delta_prepare_kernel(const DeltaChunkParams p) {
     }
     if (seq < 0) return;
     const int t0 = p.cu_seqlens[seq] + ci * kDC, n = min(kDC, p.cu_seqlens[seq + 1] - t0);
+    const int slot = p.state_slots[seq];
+    if (slot < 0 || slot >= p.num_slots) {
+        if (tid == 0) atomicExch(p.err, 2);
+        return;
+    }
+    const int QK = p.G * kDK, C = 2 * QK + p.H * p.dv;
+    const float* hist = p.state + static_cast<int64_t>(slot) * p.state_floats + p.conv_off;
     pdl_wait();
-    // tokens past the portion: k, q, v, b zero and g one, which leaves the state as it is
-    for (int idx = tid; idx < 2 * kDC * (kDK / 4); idx += blockDim.x) {
-        const int which = idx / (kDC * (kDK / 4)), r = idx / (kDK / 4) % kDC, c = idx % (kDK / 4) * 4;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < n) x = *reinterpret_cast<const float4*>((which ? p.qn : p.kn) + (static_cast<int64_t>(t0 + r) * p.G + kvh) * kDK + c);
-        uint2 hi, lo;
-        split_pair(x.x, x.y, hi.x, lo.x);
-        split_pair(x.z, x.w, hi.y, lo.y);
-        __nv_bfloat16* dst = (which ? sQ : sK) + r * kDLD + c;
-        *reinterpret_cast<uint2*>(dst) = hi;
-        *reinterpret_cast<uint2*>(dst + kDC * kDLD) = lo;
-    }
-    if (tid < kDC) {
-        sG[tid] = tid < n ? p.gg[static_cast<int64_t>(t0 + tid) * p.H + h] : 1.f;
-        sBeta[tid] = tid < n ? p.bb[static_cast<int64_t>(t0 + tid) * p.H + h] : 0.f;
-    }
-    // the thread's right-hand side, asked for now and used after the products
-    const int col = tid < kDK ? tid : tid - kDK;
-    const bool is_w = tid < kDK;
-    float x[kDC];
+    // Two neighbouring channels of eight tokens per thread.  The rows of all channels are asked for first, without a branch between them (a load in a
+    // branch of its own is waited for there: eleven trips to memory, one after the other); rows past the portion stand in for themselves with its
+    // first one and count as zeros.
+    const int cp = (tid & 63) * 2, r0 = (tid >> 6) * 8;
+    constexpr int kRows = 8 + TAPS - 1;
+    auto fetch = [&](uint32_t (&raw)[kRows], float (&w)[2 * TAPS], int c0, int width) {      // w: [channel][tap]
+        const int c = c0 + (cp < width ? cp : 0);
 #pragma unroll
-    for (int i = 0; i < kDC; ++i) {
-        const float* src = is_w ? p.kn + (static_cast<int64_t>(t0 + i) * p.G + kvh) * kDK + col : p.vv + (static_cast<int64_t>(t0 + i) * p.H + h) * p.dv + col;
-        x[i] = i < n ? *src : 0.f;
+        for (int i = 0; i < 2 * TAPS; ++i) w[i] = p.conv_w[static_cast<int64_t>(c) * TAPS + i];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) {
+            const int r = r0 + i - (TAPS - 1);                                     // the token's place in the chunk
+            const bool in = r < n && ci * kDC + r >= 0;
+            raw[i] = *reinterpret_cast<const uint32_t*>(p.packed + static_cast<int64_t>(t0 + (in ? r : 0)) * p.stride + p.qkv_off + c);
+        }
+    };
+    auto convolve = [&](float* dst, const uint32_t (&raw)[kRows], const float (&w)[2 * TAPS], int c0, int width) {
+        if (cp >= width) return;
+        float2 x[kRows];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) x[i] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[i]));
+        if (ci == 0 && r0 == 0) {                                                  // before the portion: the request's history, oldest first
+#pragma unroll
+            for (int i = 0; i < TAPS - 1; ++i) {
+                x[i].x = hist[static_cast<int64_t>(i) * C + c0 + cp];
+                x[i].y = hist[static_cast<int64_t>(i) * C + c0 + cp + 1];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float ax = 0.f, ay = 0.f;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                ax = fmaf(w[j], x[i + j].x, ax);
+                ay = fmaf(w[TAPS + j], x[i + j].y, ay);
+            }
+            const bool in = r0 + i < n;
+            *reinterpret_cast<float2*>(dst + (r0 + i) * kDLF + cp) = make_float2(in ? ax / (1.f + expf(-ax)) : 0.f, in ? ay / (1.f + expf(-ay)) : 0.f);
+        }
+    };
+    const int v_col = 2 * QK + kvh * share * p.dv;
+    uint32_t raw_v1[kRows];
+    float w_v1[2 * TAPS];
+    {
+        uint32_t raw_q[kRows], raw_k[kRows], raw_v[kRows];
+        float w_q[2 * TAPS], w_k[2 * TAPS], w_v[2 * TAPS];
+        fetch(raw_q, w_q, kvh * kDK, kDK);
+        fetch(raw_k, w_k, QK + kvh * kDK, kDK);
+        fetch(raw_v, w_v, v_col, p.dv);
+        if (share > 1) fetch(raw_v1, w_v1, v_col + p.dv, p.dv);
+        convolve(sV1, raw_q, w_q, kvh * kDK, kDK);
+        convolve(sKf, raw_k, w_k, QK + kvh * kDK, kDK);
+        convolve(sV0, raw_v, w_v, v_col, p.dv);
     }
     __syncthreads();
-    if (warp == 0) {                                                               // D, a column per lane
-        float d = 1.f;
-        for (int i = 0; i < kDC; ++i) {
-            if (i > lane) d *= sG[i];
-            sD[i * 33 + lane] = d;                                                 // read for j <= i only
+#pragma unroll
+    for (int i = 0; i < kDC / 8; ++i) {                                            // unit vectors, split; a warp per row
+        const int r = warp * (kDC / 8) + i;
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            float* row = (which ? sV1 : sKf) + r * kDLF + lane * 4;
+            float4 x = *reinterpret_cast<const float4*>(row);
+            const float ss = warp_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))));
+            float inv = 1.f / sqrtf(ss + 1e-6f);
+            if (which) inv *= 1.f / sqrtf(static_cast<float>(kDK));
+            x = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+            if (!which) *reinterpret_cast<float4*>(row) = x;
+            uint2 hi, lo;
+            split_pair(x.x, x.y, hi.x, lo.x);
+            split_pair(x.z, x.w, hi.y, lo.y);
+            __nv_bfloat16* dst = (which ? sQ : sK) + r * kDLD + lane * 4;
+            *reinterpret_cast<uint2*>(dst) = hi;
+            *reinterpret_cast<uint2*>(dst + kDC * kDLD) = lo;
         }
-    } else if (warp == 1) {
-        float e = 1.f;
-        for (int s = 0; s <= lane; ++s) e *= sG[s];
-        sE[lane] = e;
     }
-    if (h % share == 0) {                                                          // the kv head's image, once
+    __syncthreads();
+    {                                                                              // the rows' pads are never read
         const uint4* src = reinterpret_cast<const uint4*>(smem);
         uint4* dst = reinterpret_cast<uint4*>(kv_image(p, lc, kvh));
-        for (int i = tid; i < kDKvBytes / 16; i += blockDim.x) dst[i] = src[i];
+        for (int i = tid; i < kDKvBytes / 16; i += 256) dst[i] = src[i];
     }
-    __syncthreads();
-    unsigned char* img = head_image(p, lc, h);
-    // K K^T and Q K^T: 2 x 2 x 4 tiles of 16 x 8 for eight warps (six, where a head's values are 64 wide: some warps take two)
-    for (int tile = warp; tile < 8; tile += blockDim.x >> 5) {
-        const int m = (tile & 1) * 16, nn = (tile >> 1) * 8;
-        float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
+    // K K^T and Q K^T, one tile of 16 x 8 of either per warp, the same for all heads of the group
+    const int m = (warp & 1) * 16, nn = (warp >> 1) * 8;
+    float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < kDK / 16; ++k) {
-            const int ao = (m + (lane & 15)) * kDLD + k * 16 + (lane >> 4) * 8;
-            uint32_t kh[4], kl[4], qh[4], ql[4], b[4];
-            ldm_x4(kh, sK + ao); ldm_x4(kl, sK + kDC * kDLD + ao);
-            ldm_x4(qh, sQ + ao); ldm_x4(ql, sQ + kDC * kDLD + ao);
-            // b[0], b[1]: hi, columns k*16 and k*16 + 8 of the eight rows; b[2], b[3]: lo
-            ldm_x4(b, sK + (lane >> 4) * kDC * kDLD + (nn + (lane & 7)) * kDLD + k * 16 + ((lane >> 3) & 1) * 8);
-            mma_16816(kk, kh, b[0], b[1]); mma_16816(kk, kh, b[2], b[3]); mma_16816(kk, kl, b[0], b[1]);
-            mma_16816(qk, qh, b[0], b[1]); mma_16816(qk, qh, b[2], b[3]); mma_16816(qk, ql, b[0], b[1]);
-        }
-        __nv_bfloat16* a_img = reinterpret_cast<__nv_bfloat16*>(img + 2 * kDRowsBytes);
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int i = m + (lane >> 2) + half * 8, j = nn + (lane & 3) * 2;
-            sL[j * 36 + i] = j < i ? sBeta[i] * sD[i * 33 + j] * kk[half * 2] : 0.f;
-            sL[(j + 1) * 36 + i] = j + 1 < i ? sBeta[i] * sD[i * 33 + j + 1] * kk[half * 2 + 1] : 0.f;
-            uint32_t hi, lo;
-            split_pair(j <= i ? sD[i * 33 + j] * qk[half * 2] : 0.f, j + 1 <= i ? sD[i * 33 + j + 1] * qk[half * 2 + 1] : 0.f, hi, lo);
-            *reinterpret_cast<uint32_t*>(a_img + i * kDLA + j) = hi;
-            *reinterpret_cast<uint32_t*>(a_img + kDC * kDLA + i * kDLA + j) = lo;
-        }
+    for (int k = 0; k < kDK / 16; ++k) {
+        const int ao = (m + (lane & 15)) * kDLD + k * 16 + (lane >> 4) * 8;
+        uint32_t kh[4], kl[4], qh[4], ql[4], b[4];
+        ldm_x4(kh, sK + ao); ldm_x4(kl, sK + kDC * kDLD + ao);
+        ldm_x4(qh, sQ + ao); ldm_x4(ql, sQ + kDC * kDLD + ao);
+        // b[0], b[1]: hi, columns k * 16 and k * 16 + 8 of the eight rows; b[2], b[3]: lo
+        ldm_x4(b, sK + (lane >> 4) * kDC * kDLD + (nn + (lane & 7)) * kDLD + k * 16 + ((lane >> 3) & 1) * 8);
+        mma_16816(kk, kh, b[0], b[1]); mma_16816(kk, kh, b[2], b[3]); mma_16816(kk, kl, b[0], b[1]);
+        mma_16816(qk, qh, b[0], b[1]); mma_16816(qk, qh, b[2], b[3]); mma_16816(qk, ql, b[0], b[1]);
     }
-    if (tid < kDC) {
-        float* v = reinterpret_cast<float*>(img + 2 * kDRowsBytes + 2 * kDC * kDLA * 2);
-        v[tid] = sE[tid];
-        v[kDC + tid] = sD[(kDC - 1) * 33 + tid];
-    }
-    __syncthreads();
-    // forward substitution, column by column of L: x_i -= L_ij x_j
-#pragma unroll
-    for (int i = 0; i < kDC; ++i) x[i] *= is_w ? sBeta[i] * sE[i] : sBeta[i];
-#pragma unroll
-    for (int j = 0; j < kDC - 1; ++j) {
-#pragma unroll
-        for (int i4 = (j + 1) / 4 * 4; i4 < kDC; i4 += 4) {
-            const float4 l = *reinterpret_cast<const float4*>(sL + j * 36 + i4);   // zero on and above the diagonal
-            x[i4] = fmaf(-l.x, x[j], x[i4]);
-            x[i4 + 1] = fmaf(-l.y, x[j], x[i4 + 1]);
-            x[i4 + 2] = fmaf(-l.z, x[j], x[i4 + 2]);
-            x[i4 + 3] = fmaf(-l.w, x[j], x[i4 + 3]);
+    for (int h0 = 0; h0 < share; h0 += kDPair) {
+        const int heads = min(kDPair, share - h0), hbase = kvh * share + h0;
+        const int c0 = v_col + h0 * p.dv;
+        if (h0 > 0) {
+            uint32_t raw[kRows];
+            float w[2 * TAPS];
+            fetch(raw, w, c0, p.dv);
+            if (heads > 1) fetch(raw_v1, w_v1, c0 + p.dv, p.dv);
+            convolve(sV0, raw, w, c0, p.dv);
         }
-    }
-    if (is_w) {
-        __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(img);
+        if (heads > 1) convolve(sV1, raw_v1, w_v1, c0 + p.dv, p.dv);               // q has become its image
+        if (warp < heads) {                                                        // a head per warp, a token per lane
+            const int h = hbase + warp;
+            float g = 1.f, be = 0.f;
+            if (lane < n) {
+                const float* ba = p.ba + static_cast<int64_t>(t0 + lane) * 2 * p.H + h;
+                const float z = ba[p.H] + p.dt_bias[h], sp = z > 20.f ? z : log1pf(expf(z));
+                g = expf(-expf(p.a_log[h]) * sp);
+                be = delta_sigmoid(ba[0]);
+            }
+            float* G = sG + warp * 2 * kDC;
+            G[lane] = be;
+            float d = 1.f, e = 1.f, mine = 1.f;                                    // D_i,lane and e_i: running products
 #pragma unroll
-        for (int i = 0; i < kDC; ++i) {
-            __nv_bfloat16 hi, lo;
-            split_bf16(x[i], hi, lo);
-            w[i * kDLD + col] = hi;
-            w[kDC * kDLD + i * kDLD + col] = lo;
+            for (int i = 0; i < kDC; ++i) {
+                const float gi = __shfl_sync(0xffffffffu, g, i);
+                e *= gi;
+                if (i > lane) d *= gi;
+                if (i == lane) mine = e;
+                sD[warp * kDC * 33 + i * 33 + lane] = d;                           // read for j <= i only
+            }
+            G[kDC + lane] = mine;
         }
-    } else {
-        float* u = u_image<NB>(p, lc, h, col / NB) + col % NB;
+        __syncthreads();
+        for (int x = 0; x < heads; ++x) {
+            unsigned char* img = head_image(p, lc, hbase + x);
+            __nv_bfloat16* a_img = reinterpret_cast<__nv_bfloat16*>(img + 2 * kDRowsBytes);
+            const float* D = sD + x * kDC * 33;
+            const float* G = sG + x * 2 * kDC;
+            float* Lt = sL + x * kDC * 36;
 #pragma unroll
-        for (int i = 0; i < kDC; ++i) u[i * (NB + 8)] = x[i];
+            for (int half = 0; half < 2; ++half) {
+                const int i = m + (lane >> 2) + half * 8, j = nn + (lane & 3) * 2;
+                Lt[j * 36 + i] = j < i ? G[i] * D[i * 33 + j] * kk[half * 2] : 0.f;
+                Lt[(j + 1) * 36 + i] = j + 1 < i ? G[i] * D[i * 33 + j + 1] * kk[half * 2 + 1] : 0.f;
+                uint32_t hi, lo;
+                split_pair(j <= i ? D[i * 33 + j] * qk[half * 2] : 0.f, j + 1 <= i ? D[i * 33 + j + 1] * qk[half * 2 + 1] : 0.f, hi, lo);
+                *reinterpret_cast<uint32_t*>(a_img + i * kDLA + j) = hi;
+                *reinterpret_cast<uint32_t*>(a_img + kDC * kDLA + i * kDLA + j) = lo;
+            }
+            if (tid < kDC) {
+                float* v = reinterpret_cast<float*>(img + 2 * kDRowsBytes + 2 * kDC * kDLA * 2);
+                v[tid] = G[kDC + tid];
+                v[kDC + tid] = D[(kDC - 1) * 33 + tid];
+            }
+        }
+        __syncthreads();
+        // forward substitution, column by column of L: x_i -= L_ij x_j; threads 0 .. 127 a column of W, the others of U~
+        const bool is_w = tid < kDK;
+        const int col = tid & (kDK - 1);
+        for (int x2 = 0; x2 < heads; ++x2) {
+            if (!is_w && col >= p.dv) continue;
+            const float* Lt = sL + x2 * kDC * 36;
+            const float* G = sG + x2 * 2 * kDC;
+            const float* rhs = (is_w ? sKf : (x2 ? sV1 : sV0)) + col;
+            float x[kDC];
+#pragma unroll
+            for (int i = 0; i < kDC; ++i) x[i] = rhs[i * kDLF] * (is_w ? G[i] * G[kDC + i] : G[i]);
+#pragma unroll
+            for (int j = 0; j < kDC - 1; ++j) {
+#pragma unroll
+                for (int i4 = (j + 1) / 4 * 4; i4 < kDC; i4 += 4) {
+                    const float4 l = *reinterpret_cast<const float4*>(Lt + j * 36 + i4);   // zero on and above the diagonal
+                    x[i4] = fmaf(-l.x, x[j], x[i4]);
+                    x[i4 + 1] = fmaf(-l.y, x[j], x[i4 + 1]);
+                    x[i4 + 2] = fmaf(-l.z, x[j], x[i4 + 2]);
+                    x[i4 + 3] = fmaf(-l.w, x[j], x[i4 + 3]);
+                }
+            }
+            if (is_w) {                                                            // of two neighbouring columns one thread stores hi, the other lo
+                __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(head_image(p, lc, hbase + x2)) + (col & 1) * kDC * kDLD + (col & ~1);
+#pragma unroll
+                for (int i = 0; i < kDC; ++i) {
+                    const float other = __shfl_xor_sync(0xffffffffu, x[i], 1);
+                    uint32_t hi, lo;
+                    split_pair((col & 1) ? other : x[i], (col & 1) ? x[i] : other, hi, lo);
+                    *reinterpret_cast<uint32_t*>(w + i * kDLD) = (col & 1) ? lo : hi;
+                }
+            } else {
+                float* u = u_image<NB>(p, lc, hbase + x2, col / NB) + col % NB;
+#pragma unroll
+                for (int i = 0; i < kDC; ++i) u[i * (NB + 8)] = x[i];
+            }
+        }
+        __syncthreads();
     }
 }
 
 template <int NB>
 struct DeltaChainSmem {
     static constexpr int kU = kDC * (NB + 8) * 4;
-    static constexpr int kStage = kDHeadBytes + kDKvBytes + kU;
+    static constexpr int kStageW = 2 * kDRowsBytes + 2 * kDRowsBytes + kU + 2 * kDC * 4;       // W hi, lo | K hi, lo | U~ | e, D_31
+    static constexpr int kStageQ = 2 * kDRowsBytes + 2 * kDC * kDLA * 2 + 2 * kDC * 4;         // Q hi, lo | A hi, lo | e, D_31
     static constexpr int kS = 2 * kDK * (NB + 8) * 2;                              // S hi, lo
-    static constexpr int kUb = 4 * kDC * (NB + 8) * 2;                             // U hi, lo | D U hi, lo
-    static constexpr size_t kBytes = static_cast<size_t>(2) * kStage + kS + kUb + 2 * 8;
+    static constexpr int kUb = 2 * kDC * (NB + 8) * 2;                             // U hi, lo
+    static constexpr size_t kBytes = static_cast<size_t>(2) * (kStageW + kStageQ + kS + kUb) + kUb + 4 * 8;
 };
 
-// Grid (request, head, NB value columns); NB / 2 warps: one half makes W S, the other Q S (tiles of 16 x 8), then every warp two tiles of S.
+// Grid (request, head, NB value columns); NB / 2 warps in two halves.  The first half carries the chain: W S, U = U~ - W S, S = e_31 S + K^T (D_31 U),
+// with two barriers of its own a chunk.  The second half makes the outputs e Q S + A U beside it, up to a chunk behind: S and U have two
+// buffers, `ready` (U of the chunk is there, S was before) and `done` (the outputs have been made) hand them over.  Each half fetches for itself, two
+// chunks ahead.  What bounds it are the shared-memory reads of the split operands (528 ldmatrix of 512 bytes a chunk at 32 columns, 2,100
+// cycles); with all warps in step through both parts a chunk took 4,000 cycles, now
+// 3,400 (1,511 + 537 tokens, 16 heads: 96 -> 84 us); the rest is the chain's own latencies.
 template <int NB>
 __global__ void __launch_bounds__(NB * 16, 1)
 delta_chain_kernel(const DeltaChunkParams p) {
     pdl_trigger();
     extern __shared__ __align__(128) unsigned char smem[];
     using L = DeltaChainSmem<NB>;
-    constexpr int LS = NB + 8, kWarps = NB / 2, kHalf = kWarps / 2;
-    unsigned char* sStage = smem;
-    __nv_bfloat16* sS = reinterpret_cast<__nv_bfloat16*>(smem + 2 * L::kStage);
-    __nv_bfloat16* sU = sS + 2 * kDK * LS;
-    __nv_bfloat16* sDU = sU + 2 * kDC * LS;
-    uint64_t* full = reinterpret_cast<uint64_t*>(sDU + 2 * kDC * LS);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int LS = NB + 8, kHalf = NB / 4, kThreads = NB * 16;                 // warps of a half, threads of the block
+    unsigned char* sStageW = smem;
+    unsigned char* sStageQ = smem + 2 * L::kStageW;
+    __nv_bfloat16* sS = reinterpret_cast<__nv_bfloat16*>(sStageQ + 2 * L::kStageQ);             // two buffers of S hi, lo
+    __nv_bfloat16* sU = sS + 2 * 2 * kDK * LS;                                     // two buffers of U hi, lo
+    __nv_bfloat16* sDU = sU + 2 * 2 * kDC * LS;                                    // D_31 U hi, lo
+    uint64_t* full = reinterpret_cast<uint64_t*>(sDU + 2 * kDC * LS);              // [2] of the first half, [2] of the second
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.x, h = blockIdx.y, cb = blockIdx.z, kvh = h / (p.H / p.G);
     const int slot = p.state_slots[s];
     if (slot < 0 || slot >= p.num_slots) {
-        if (tid == 0) atomicExch(p.err, 2);
+        if (threadIdx.x == 0) atomicExch(p.err, 2);
         return;
     }
     int first = 0;                                                                 // the request's first chunk among all
@@ -253,75 +361,52 @@ delta_chain_kernel(const DeltaChunkParams p) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
     const int begin = p.cu_seqlens[s], end = p.cu_seqlens[s + 1];
-    const int c0 = max(first, p.c_first), c1 = min(first + chunks_of(p, s), p.c_first + p.c_count);
-    if (c0 >= c1) return;
-    if (tid == 0) {
-        mbar_init(full, 1);
-        mbar_init(full + 1, 1);
+    const int c0 = max(first, p.c_first), n = min(first + chunks_of(p, s), p.c_first + p.c_count) - c0;      // chunks here
+    if (n <= 0) return;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; ++i) mbar_init(full + i, 1);
         mbar_fence_init();
     }
     pdl_wait();
-    auto fetch = [&](int c) {                                                      // one thread: chunk c into its stage
-        const int st = (c - c0) & 1, lc = c - p.c_first;
-        unsigned char* dst = sStage + st * L::kStage;
-        mbar_expect_tx(full + st, L::kStage);
-        const void* src[3] = {head_image(p, lc, h), kv_image(p, lc, kvh), u_image<NB>(p, lc, h, cb)};
-        const int bytes[3] = {kDHeadBytes, kDKvBytes, L::kU};
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                         ::"r"(smem_u32(dst)), "l"(src[i]), "r"(bytes[i]), "r"(smem_u32(full + st)) : "memory");
-            dst += bytes[i];
-        }
-    };
-    if (tid == 0) {
-        fetch(c0);
-        if (c0 + 1 < c1) fetch(c0 + 1);
-    }
-    // S: this warp's two tiles of 16 rows x 8 columns
-    const int sm = (NB == 16 ? warp : warp & 7) * 16, sn = NB == 16 ? 0 : (warp >> 3) * 16;
-    float* st_base = p.state + static_cast<int64_t>(slot) * p.state_floats + static_cast<int64_t>(h) * kDK * p.dv + cb * NB;
-    float S[2][4];
-    auto write_s = [&]() {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t hi, lo;
-                split_pair(S[t][half * 2], S[t][half * 2 + 1], hi, lo);
-                __nv_bfloat16* dst = sS + (sm + (lane >> 2) + half * 8) * LS + sn + t * 8 + (lane & 3) * 2;
-                *reinterpret_cast<uint32_t*>(dst) = hi;
-                *reinterpret_cast<uint32_t*>(dst + kDK * LS) = lo;
-            }
-        }
-    };
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const float2 v = *reinterpret_cast<const float2*>(st_base + static_cast<int64_t>(sm + (lane >> 2) + half * 8) * p.dv + sn + t * 8 + (lane & 3) * 2);
-            S[t][half * 2] = v.x;
-            S[t][half * 2 + 1] = v.y;
-        }
-    }
-    write_s();
     __syncthreads();
     const bool is_q = warp >= kHalf;
-    const int w = is_q ? warp - kHalf : warp, m = (w & 1) * 16, nn = (w >> 1) * 8;
-    for (int c = c0; c < c1; ++c) {
-        const int st = (c - c0) & 1;
-        const unsigned char* base = sStage + st * L::kStage;
-        const __nv_bfloat16* sW = reinterpret_cast<const __nv_bfloat16*>(base);
-        const __nv_bfloat16* sA = sW + 2 * kDC * kDLD;
-        const float* sE = reinterpret_cast<const float*>(sA + 2 * kDC * kDLA);
-        const __nv_bfloat16* sK = reinterpret_cast<const __nv_bfloat16*>(base + kDHeadBytes);
-        const __nv_bfloat16* sQ = sK + 2 * kDC * kDLD;
-        const float* sUt = reinterpret_cast<const float*>(base + kDHeadBytes + kDKvBytes);
-        mbar_wait(full + st, ((c - c0) >> 1) & 1, p.err);
-        // W S (first half of the warps) or Q S: chains of their own for the three parts of the split
-        float a0[4] = {0.f, 0.f, 0.f, 0.f}, a1[4] = {0.f, 0.f, 0.f, 0.f}, a2[4] = {0.f, 0.f, 0.f, 0.f};
-        const __nv_bfloat16* lhs = (is_q ? sQ : sW) + (m + (lane & 15)) * kDLD + (lane >> 4) * 8;
-        const __nv_bfloat16* rhs = sS + lane * LS + nn;
+    const int w = is_q ? warp - kHalf : warp, m = (w & 1) * 16, nn = (w >> 1) * 8; // the warp's tile of W S or Q S
+    auto bulk = [&](unsigned char*& dst, const void* src, int bytes, uint64_t* bar) {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                     ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+        dst += bytes;
+    };
+    constexpr int kABytes = 2 * kDC * kDLA * 2, kVecBytes = 2 * kDC * 4;
+    auto fetch = [&](int c) {                                                      // one thread of a half: chunk c0 + c into the half's stage
+        const int st = c & 1, lc = c0 + c - p.c_first;
+        const unsigned char* head = head_image(p, lc, h);
+        const unsigned char* kv = kv_image(p, lc, kvh);
+        uint64_t* bar = full + (is_q ? 2 : 0) + st;
+        if (is_q) {
+            unsigned char* dst = sStageQ + st * L::kStageQ;
+            mbar_expect_tx(bar, L::kStageQ);
+            bulk(dst, kv + 2 * kDRowsBytes, 2 * kDRowsBytes, bar);
+            bulk(dst, head + 2 * kDRowsBytes, kABytes + kVecBytes, bar);
+        } else {
+            unsigned char* dst = sStageW + st * L::kStageW;
+            mbar_expect_tx(bar, L::kStageW);
+            bulk(dst, head, 2 * kDRowsBytes, bar);
+            bulk(dst, kv, 2 * kDRowsBytes, bar);
+            bulk(dst, u_image<NB>(p, lc, h, cb), L::kU, bar);
+            bulk(dst, head + 2 * kDRowsBytes + kABytes, kVecBytes, bar);
+        }
+    };
+    if (w == 0 && lane == 0) {
+        fetch(0);
+        if (n > 1) fetch(1);
+    }
+    // lhs (32 rows of 128, hi and lo) times the chunk's S: the warp's tile, the three parts of the split in chains of their own
+    auto times_s = [&](float (&a0)[4], const __nv_bfloat16* lhs, const __nv_bfloat16* rhs) {
+        float a1[4] = {0.f, 0.f, 0.f, 0.f}, a2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a0[i] = 0.f;
+        lhs += (m + (lane & 15)) * kDLD + (lane >> 4) * 8;
+        rhs += lane * LS + nn;
 #pragma unroll
         for (int k = 0; k < kDK / 16; k += 2) {
             uint32_t bh[4], bl[4];
@@ -339,67 +424,127 @@ delta_chain_kernel(const DeltaChunkParams p) {
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) a0[i] += a1[i] + a2[i];
-        if (!is_q) {                                                               // U = U~ - W S, and D_31 U
+    };
+    // named barriers: 1 the first half; 2, 3 `ready` and 4, 5 `done` of even and odd chunks
+    if (!is_q) {
+        // S: four tiles of 16 rows x 8 columns a warp
+        auto tile_m = [&](int t) { return (NB == 32 ? w : 2 * w + (t >> 1)) * 16; };
+        auto tile_n = [&](int t) { return (NB == 32 ? t : t & 1) * 8; };
+        float* st_base = p.state + static_cast<int64_t>(slot) * p.state_floats + static_cast<int64_t>(h) * kDK * p.dv + cb * NB;
+        float S[4][4];
+        auto write_s = [&](__nv_bfloat16* dst0) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t hi, lo;
+                    split_pair(S[t][half * 2], S[t][half * 2 + 1], hi, lo);
+                    __nv_bfloat16* dst = dst0 + (tile_m(t) + (lane >> 2) + half * 8) * LS + tile_n(t) + (lane & 3) * 2;
+                    *reinterpret_cast<uint32_t*>(dst) = hi;
+                    *reinterpret_cast<uint32_t*>(dst + kDK * LS) = lo;
+                }
+            }
+        };
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
+                const float2 v = *reinterpret_cast<const float2*>(st_base + static_cast<int64_t>(tile_m(t) + (lane >> 2) + half * 8) * p.dv + tile_n(t) + (lane & 3) * 2);
+                S[t][half * 2] = v.x;
+                S[t][half * 2 + 1] = v.y;
+            }
+        }
+        write_s(sS);
+        asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads / 2) : "memory");
+        for (int c = 0; c < n; ++c) {
+            const int st = c & 1;
+            const unsigned char* base = sStageW + st * L::kStageW;
+            const __nv_bfloat16* sW = reinterpret_cast<const __nv_bfloat16*>(base);
+            const __nv_bfloat16* sK = sW + 2 * kDC * kDLD;
+            const float* sUt = reinterpret_cast<const float*>(base + 4 * kDRowsBytes);
+            const float* sE = sUt + kDC * LS;
+            __nv_bfloat16* u_buf = sU + st * 2 * kDC * LS;
+            mbar_wait(full + st, (c >> 1) & 1, p.err);
+            float a[4];
+            times_s(a, sW, sS + st * 2 * kDK * LS);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {                                 // U = U~ - W S, and D_31 U
                 const int i = m + (lane >> 2) + half * 8, j = nn + (lane & 3) * 2;
                 const float2 ut = *reinterpret_cast<const float2*>(sUt + i * LS + j);
-                const float ux = ut.x - a0[half * 2], uy = ut.y - a0[half * 2 + 1], d = sE[kDC + i];
+                const float ux = ut.x - a[half * 2], uy = ut.y - a[half * 2 + 1], d = sE[kDC + i];
                 uint32_t hi, lo;
-                split_pair(ux, uy, hi, lo);
-                *reinterpret_cast<uint32_t*>(sU + i * LS + j) = hi;
-                *reinterpret_cast<uint32_t*>(sU + (kDC + i) * LS + j) = lo;
                 split_pair(d * ux, d * uy, hi, lo);
                 *reinterpret_cast<uint32_t*>(sDU + i * LS + j) = hi;
                 *reinterpret_cast<uint32_t*>(sDU + (kDC + i) * LS + j) = lo;
+                split_pair(ux, uy, hi, lo);
+                *reinterpret_cast<uint32_t*>(u_buf + i * LS + j) = hi;
+                *reinterpret_cast<uint32_t*>(u_buf + (kDC + i) * LS + j) = lo;
             }
-        }
-        __syncthreads();                                                           // U is there; nobody reads the old S any more
-        {                                                                          // S = e_31 S + K^T (D_31 U)
-            const float e = sE[kDC - 1];
-            float acc[2][4];
+            asm volatile("bar.arrive %0, %1;\n" ::"r"(2 + st), "n"(kThreads) : "memory");        // ready
+            asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads / 2) : "memory");
+            const float e = sE[kDC - 1];                                           // S = e_31 S + K^T (D_31 U)
+            float acc[4][4];
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
+            for (int t = 0; t < 4; ++t) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
             }
-            const int ko = ((lane & 7) + (lane >> 4) * 8) * kDLD + sm + ((lane >> 3) & 1) * 8;
-            uint32_t bh[2][4], bl[2][4];
+            constexpr int kN = NB / 8, kM = 4 / kN;                                // the warp's column and row tiles
+            uint32_t bh[kN][4], bl[kN][4];
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
-                ldm_x4_trans(bh[t], sDU + lane * LS + sn + t * 8);
-                ldm_x4_trans(bl[t], sDU + (kDC + lane) * LS + sn + t * 8);
+            for (int t = 0; t < kN; ++t) {
+                ldm_x4_trans(bh[t], sDU + lane * LS + t * 8);
+                ldm_x4_trans(bl[t], sDU + (kDC + lane) * LS + t * 8);
             }
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                uint32_t kh[4], kl[4];
-                ldm_x4_trans(kh, sK + k * 16 * kDLD + ko);
-                ldm_x4_trans(kl, sK + (kDC + k * 16) * kDLD + ko);
+            for (int mt = 0; mt < kM; ++mt) {
+                const __nv_bfloat16* kt = sK + ((lane & 7) + (lane >> 4) * 8) * kDLD + tile_m(mt * kN) + ((lane >> 3) & 1) * 8;
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    mma_16816(acc[t], kh, bh[t][2 * k], bh[t][2 * k + 1]);
-                    mma_16816(acc[t], kh, bl[t][2 * k], bl[t][2 * k + 1]);
-                    mma_16816(acc[t], kl, bh[t][2 * k], bh[t][2 * k + 1]);
+                for (int k = 0; k < 2; ++k) {
+                    uint32_t kh[4], kl[4];
+                    ldm_x4_trans(kh, kt + k * 16 * kDLD);
+                    ldm_x4_trans(kl, kt + (kDC + k * 16) * kDLD);
+#pragma unroll
+                    for (int t = 0; t < kN; ++t) {
+                        mma_16816(acc[mt * kN + t], kh, bh[t][2 * k], bh[t][2 * k + 1]);
+                        mma_16816(acc[mt * kN + t], kh, bl[t][2 * k], bl[t][2 * k + 1]);
+                        mma_16816(acc[mt * kN + t], kl, bh[t][2 * k], bh[t][2 * k + 1]);
+                    }
                 }
             }
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
+            for (int t = 0; t < 4; ++t) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) S[t][i] = fmaf(e, S[t][i], acc[t][i]);
             }
-            if (c + 1 < c1) write_s();
+            if (c > 0) asm volatile("bar.sync %0, %1;\n" ::"r"(4 + (st ^ 1)), "n"(kThreads) : "memory");     // done with the chunk before
+            if (c + 1 < n) write_s(sS + (st ^ 1) * 2 * kDK * LS);
+            asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads / 2) : "memory");      // the new S is there; the stage may be filled again
+            if (threadIdx.x == 0 && c + 2 < n) fetch(c + 2);
         }
-        if (is_q) {                                                                // O = e Q S + A U
-            float o[4];
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const float e = sE[m + (lane >> 2) + half * 8];
-                o[half * 2] = e * a0[half * 2];
-                o[half * 2 + 1] = e * a0[half * 2 + 1];
-            }
+        for (int t = 0; t < 4; ++t) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                *reinterpret_cast<float2*>(st_base + static_cast<int64_t>(tile_m(t) + (lane >> 2) + half * 8) * p.dv + tile_n(t) + (lane & 3) * 2) =
+                    make_float2(S[t][half * 2], S[t][half * 2 + 1]);
+        }
+    } else {
+        for (int c = 0; c < n; ++c) {
+            const int st = c & 1;
+            const __nv_bfloat16* sQ = reinterpret_cast<const __nv_bfloat16*>(sStageQ + st * L::kStageQ);
+            const __nv_bfloat16* sA = sQ + 2 * kDC * kDLD;
+            const float* sE = reinterpret_cast<const float*>(sA + 2 * kDC * kDLA);
+            const __nv_bfloat16* u_buf = sU + st * 2 * kDC * LS;
+            mbar_wait(full + 2 + st, (c >> 1) & 1, p.err);
+            asm volatile("bar.sync %0, %1;\n" ::"r"(2 + st), "n"(kThreads) : "memory");          // ready
+            float o[4];
+            times_s(o, sQ, sS + st * 2 * kDK * LS);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] *= sE[m + (lane >> 2) + (i >> 1) * 8];
             uint32_t bh[4], bl[4];
-            ldm_x4_trans(bh, sU + lane * LS + nn);
-            ldm_x4_trans(bl, sU + (kDC + lane) * LS + nn);
+            ldm_x4_trans(bh, u_buf + lane * LS + nn);
+            ldm_x4_trans(bl, u_buf + (kDC + lane) * LS + nn);
             const __nv_bfloat16* al = sA + (m + (lane & 15)) * kDLA + (lane >> 4) * 8;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -410,23 +555,17 @@ delta_chain_kernel(const DeltaChunkParams p) {
                 mma_16816(o, xh, bl[2 * k], bl[2 * k + 1]);
                 mma_16816(o, xl, bh[2 * k], bh[2 * k + 1]);
             }
-            const int t0 = begin + (c - first) * kDC;
+            if (c + 1 < n) asm volatile("bar.arrive %0, %1;\n" ::"r"(4 + st), "n"(kThreads) : "memory");     // done
+            const int t0 = begin + (c0 + c - first) * kDC;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 const int t = t0 + m + (lane >> 2) + half * 8;
                 if (t < end)
                     *reinterpret_cast<float2*>(p.out + (static_cast<int64_t>(t) * p.H + h) * p.dv + cb * NB + nn + (lane & 3) * 2) = make_float2(o[half * 2], o[half * 2 + 1]);
             }
+            asm volatile("bar.sync 6, %0;\n" ::"n"(kThreads / 2) : "memory");      // the whole half: the stage may be filled again
+            if (w == 0 && lane == 0 && c + 2 < n) fetch(c + 2);
         }
-        __syncthreads();                                                           // the new S is there; the stage may be filled again
-        if (tid == 0 && c + 2 < c1) fetch(c + 2);
-    }
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half)
-            *reinterpret_cast<float2*>(st_base + static_cast<int64_t>(sm + (lane >> 2) + half * 8) * p.dv + sn + t * 8 + (lane & 3) * 2) =
-                make_float2(S[t][half * 2], S[t][half * 2 + 1]);
     }
 }
 
@@ -435,12 +574,11 @@ int64_t delta_chunk_bytes(int H, int G, int dv) {
     return static_cast<int64_t>(H) * kDHeadBytes + static_cast<int64_t>(G) * kDKvBytes + static_cast<int64_t>(H) * (dv / NB) * kDC * (NB + 8) * 4;
 }
 
-template <int NB>
+template <int NB, int TAPS>
 int launch_delta_chunks(DeltaChunkParams p, int total, int held, cudaStream_t stream) {
-    const size_t prep = static_cast<size_t>(kDKvBytes) + (kDC * 36 + kDC * 33 + 3 * kDC) * sizeof(float);
     static bool set = false;
     if (!set) {
-        if (cudaFuncSetAttribute(delta_prepare_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(prep)) != cudaSuccess ||
+        if (cudaFuncSetAttribute(delta_prepare_kernel<NB, TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDPrepBytes)) != cudaSuccess ||
             cudaFuncSetAttribute(delta_chain_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(DeltaChainSmem<NB>::kBytes)) != cudaSuccess)
             return launch_status();
         set = true;
@@ -449,7 +587,7 @@ int launch_delta_chunks(DeltaChunkParams p, int total, int held, cudaStream_t st
     for (int c = 0; c < total; c += held) {
         p.c_first = c;
         p.c_count = total - c < held ? total - c : held;
-        launch_kernel(delta_prepare_kernel<NB>, dim3(p.c_count, p.H), dim3(kDK + p.dv), prep, stream, p);
+        launch_kernel(delta_prepare_kernel<NB, TAPS>, dim3(p.c_count, p.G), dim3(256), kDPrepBytes, stream, p);
         launch_kernel(delta_chain_kernel<NB>, dim3(p.S, p.H, p.dv / NB), dim3(NB * 16), DeltaChainSmem<NB>::kBytes, stream, p);
     }
     return launch_status();
@@ -463,26 +601,37 @@ using namespace cvb;
 extern "C" int64_t cvb_delta_chunks_scratch(int chunks, int H, int G, int dv) { return static_cast<int64_t>(chunks) * delta_chunk_bytes<16>(H, G, dv); }
 
 // total: the sum over the requests of ceil(tokens / 32).
-extern "C" int cvb_delta_chunks(float* out, const float* qn, const float* kn, const float* vv, const float* gg, const float* bb, float* state,
-                                int64_t state_floats, const int* cu_seqlens, const int* state_slots, int num_slots, int S, int total, int H, int G,
-                                int dk, int dv, void* scratch, int64_t scratch_bytes, int* err_flag, cudaStream_t stream) {
+extern "C" int cvb_delta_chunks(float* out, const void* packed, int stride, int qkv_off, const float* conv_w, int taps, const float* ba,
+                                const float* dt_bias, const float* a_log, float* state, int64_t state_floats, int64_t conv_off,
+                                const int* cu_seqlens, const int* state_slots, int num_slots, int S, int total, int H, int G, int dk, int dv,
+                                void* scratch, int64_t scratch_bytes, int* err_flag, cudaStream_t stream) {
     if (S == 0 || total == 0) return CVB_OK;
     if (S < 0 || total < 0 || H <= 0 || H > 65535 || G <= 0 || num_slots <= 0) return CVB_E_SIZE;
-    if (dk != kDK || (dv != 64 && dv != 128)) return CVB_E_UNSUPPORTED;
-    if (H % G || state_floats < static_cast<int64_t>(H) * dk * dv) return CVB_E_SHAPE;
-    for (const void* p : {static_cast<const void*>(qn), static_cast<const void*>(kn), static_cast<const void*>(vv), static_cast<const void*>(out),
-                          static_cast<const void*>(state), static_cast<const void*>(scratch)})
+    if (dk != kDK || (dv != 64 && dv != 128) || taps < 1 || taps > 4) return CVB_E_UNSUPPORTED;
+    const int64_t C = 2LL * G * dk + static_cast<int64_t>(H) * dv, mat = static_cast<int64_t>(H) * dk * dv;
+    if (H % G || qkv_off < 0 || stride < qkv_off + C || conv_off < mat || state_floats < conv_off + (taps - 1) * C) return CVB_E_SHAPE;
+    for (const void* p : {static_cast<const void*>(out), static_cast<const void*>(state), static_cast<const void*>(scratch)})
         if (reinterpret_cast<uintptr_t>(p) & 15) return CVB_E_ALIGN;
-    if (state_floats % 2) return CVB_E_ALIGN;                                      // a slot's matrices start on whole pairs
+    // pairs of channels, and a slot's matrices start on whole pairs
+    if (state_floats % 2 || stride % 2 || qkv_off % 2 || (reinterpret_cast<uintptr_t>(packed) & 3)) return CVB_E_ALIGN;
     DeltaChunkParams p{};
-    p.qn = qn; p.kn = kn; p.vv = vv; p.gg = gg; p.bb = bb; p.out = out; p.state = state; p.state_floats = state_floats;
+    p.packed = static_cast<const __nv_bfloat16*>(packed); p.stride = stride; p.qkv_off = qkv_off; p.conv_w = conv_w;
+    p.ba = ba; p.dt_bias = dt_bias; p.a_log = a_log; p.conv_off = conv_off;
+    p.out = out; p.state = state; p.state_floats = state_floats;
     p.cu_seqlens = cu_seqlens; p.state_slots = state_slots; p.num_slots = num_slots; p.S = S; p.H = H; p.G = G; p.dv = dv;
     p.scratch = static_cast<unsigned char*>(scratch); p.err = err_flag;
     // slices of 16 columns while the chain's blocks fit the SMs at once (each holds an SM's shared memory), else of 32
     const bool narrow = static_cast<int64_t>(S) * H * (dv / 16) <= 148;
     const int64_t per = narrow ? delta_chunk_bytes<16>(H, G, dv) : delta_chunk_bytes<32>(H, G, dv);
-    const int64_t held = scratch_bytes / per;
-    if (held < 1) return CVB_E_SCRATCH;
-    const int h32 = static_cast<int>(held < total ? held : total);
-    return narrow ? launch_delta_chunks<16>(p, total, h32, stream) : launch_delta_chunks<32>(p, total, h32, stream);
+    const int64_t fits = scratch_bytes / per;
+    if (fits < 1) return CVB_E_SCRATCH;
+    const int held = static_cast<int>(fits < total ? fits : total);
+#define CALL(T) return narrow ? launch_delta_chunks<16, T>(p, total, held, stream) : launch_delta_chunks<32, T>(p, total, held, stream)
+    switch (taps) {
+        case 1: CALL(1);
+        case 2: CALL(2);
+        case 3: CALL(3);
+        default: CALL(4);
+    }
+#undef CALL
 }

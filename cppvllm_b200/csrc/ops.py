@@ -768,7 +768,7 @@ def _delta_lib():
     if _delta is None:
         lib = load_library("delta")
         P, i, n = c_void_p, c_int, c_int64
-        lib.cvb_delta_chunks.argtypes = [P] * 7 + [n, P, P] + [i] * 7 + [P, n, P, P]
+        lib.cvb_delta_chunks.argtypes = [P, P, i, i, P, i] + [P] * 4 + [n, n, P, P] + [i] * 7 + [P, n, P, P]
         lib.cvb_delta_chunks.restype = c_int
         lib.cvb_delta_chunks_scratch.argtypes = [i, i, i, i]
         lib.cvb_delta_chunks_scratch.restype = n
@@ -780,31 +780,37 @@ DELTA_CHUNK = 32              # tokens
 DELTA_CHUNKS_HELD = 96        # chunks whose images the scratch holds (170 MB at 32 heads of 128 x 128); longer steps go through it in turns
 
 
-def delta_chunks_supported(dtype: torch.dtype, dim: int, vdim: int, state: torch.Tensor, q_lens) -> bool:
+def delta_chunks_supported(packed: torch.Tensor, qkv_off: int, taps: int, num_heads: int, num_kv_heads: int, dim: int, vdim: int, state: torch.Tensor,
+                           q_lens) -> bool:
     """Whether portions of the rule with one decay per head go through the tensor cores (csrc/delta_chunks.cu): activations in bf16 (float32 stays
-    on the token-by-token scan), keys of 128 and values of 64 or 128 elements, states that start on whole pairs, and a portion longer than a
-    chunk: the scan takes 0.41 us a token of the longest portion, the two chunk kernels 11 us for up to a chunk and 0.7 us for a further one."""
-    return (dtype == torch.bfloat16 and dim == 128 and vdim in (64, 128) and state.shape[1] % 2 == 0 and max(q_lens) > DELTA_CHUNK)
+    on the token-by-token scan), keys of 128 and values of 64 or 128 elements, up to four taps, channels and states that start on whole pairs, and
+    a long portion.  The scan takes 0.41 us a token of the longest portion; the chunks cost 25 us at two heads a kv head and 17 us more for every
+    further pair of them before the first token is done.  Measured, a layer, chunks against scan, us: 16/8 heads 64 tokens 46 / 47, 128 tokens 49 /
+    69, 33 tokens 45 / 39; 32/8 heads 128 tokens 100 / 105, 64 tokens 94 / 79."""
+    least = 24 + 40 * ((num_heads // num_kv_heads + 1) // 2)
+    return (packed.dtype == torch.bfloat16 and dim == 128 and vdim in (64, 128) and 1 <= taps <= 4 and state.shape[1] % 2 == 0
+            and packed.stride(0) % 2 == 0 and qkv_off % 2 == 0 and packed.data_ptr() % 4 == 0 and max(q_lens) >= least)
 
 
-def delta_chunks(out, qn, kn, vv, gg, bb, state: torch.Tensor, cu_seqlens, state_slots, q_lens, num_heads: int, num_kv_heads: int, dim: int,
-                 vdim: int, workspace) -> torch.Tensor:
-    """delta_scan with `decay_dim` = 1 in chunks of 32 tokens."""
+def delta_chunks(out, packed, qkv_off: int, conv_w, ba, dt_bias, a_log, state: torch.Tensor, conv_off: int, cu_seqlens, state_slots, q_lens,
+                 num_heads: int, num_kv_heads: int, dim: int, vdim: int, workspace) -> torch.Tensor:
+    """delta_prep and delta_scan with `decay_dim` = 1 in one, in chunks of 32 tokens; `ba` [T, 2 H]: the logits of b, then of the decays."""
     f32, i32 = torch.float32, torch.int32
-    for t, dtype in ((out, f32), (qn, f32), (kn, f32), (vv, f32), (gg, f32), (bb, f32), (cu_seqlens, i32), (state_slots, i32)):
+    for t, dtype in ((out, f32), (packed, torch.bfloat16), (conv_w, f32), (ba, f32), (dt_bias, f32), (a_log, f32), (state, f32),
+                     (cu_seqlens, i32), (state_slots, i32)):
         if t.dtype != dtype or not t.is_cuda or not t.is_contiguous():
-            raise KernelError("delta_chunks: contiguous CUDA tensors, float32; cu_seqlens and state_slots int32")
-    T, H, G = out.shape[0], num_heads, num_kv_heads
-    if (out.numel() != T * H * vdim or vv.numel() != out.numel() or qn.numel() != T * G * dim or kn.numel() != qn.numel() or gg.numel() != T * H
-            or bb.numel() != T * H or state.dtype != f32 or not state.is_contiguous() or state.dim() != 2):
-        raise KernelError("delta_chunks: out, v [T, H * vdim], q, k [T, G * dim], g, b [T, H], state float32 [slots, floats]")
+            raise KernelError("delta_chunks: contiguous CUDA tensors, packed bf16, cu_seqlens and state_slots int32, the others float32")
+    T, H, G = packed.shape[0], num_heads, num_kv_heads
+    if (out.numel() != T * H * vdim or ba.numel() != T * 2 * H or dt_bias.numel() != H or a_log.numel() != H or conv_w.dim() != 2
+            or conv_w.shape[0] != 2 * G * dim + H * vdim or state.dim() != 2):
+        raise KernelError("delta_chunks: out [T, H * vdim], ba [T, 2 H], dt_bias, a_log [H], conv_w [channels, taps], state [slots, floats]")
     lib = _delta_lib()
     total = sum((n + DELTA_CHUNK - 1) // DELTA_CHUNK for n in q_lens)
     scratch = workspace.flat(f"delta_chunks_{H}_{G}_{vdim}", lib.cvb_delta_chunks_scratch(DELTA_CHUNKS_HELD, H, G, vdim), torch.uint8)
-    _check(lib.cvb_delta_chunks(out.data_ptr(), qn.data_ptr(), kn.data_ptr(), vv.data_ptr(), gg.data_ptr(), bb.data_ptr(), state.data_ptr(),
-                                state.shape[1], cu_seqlens.data_ptr(), state_slots.data_ptr(), state.shape[0], len(q_lens), total, H, G, dim, vdim,
-                                scratch.data_ptr(), scratch.numel(), error_flag(out.device).data_ptr(), _stream()), "delta_chunks",
-           kernels=2 * -(-total // DELTA_CHUNKS_HELD))
+    _check(lib.cvb_delta_chunks(out.data_ptr(), packed.data_ptr(), packed.stride(0), qkv_off, conv_w.data_ptr(), conv_w.shape[1], ba.data_ptr(),
+                                dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), state.shape[1], conv_off, cu_seqlens.data_ptr(),
+                                state_slots.data_ptr(), state.shape[0], len(q_lens), total, H, G, dim, vdim, scratch.data_ptr(), scratch.numel(),
+                                error_flag(out.device).data_ptr(), _stream()), "delta_chunks", kernels=2 * -(-total // DELTA_CHUNKS_HELD))
     return out
 
 

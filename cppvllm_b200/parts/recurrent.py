@@ -194,6 +194,7 @@ class HeadDeltaMixer(Mixer):
         self.w_in = _cat_rows([t("q"), t("k"), t("v"), t("g")])
         self.g_off = self.channels
         self.w_b, self.w_a, self.w_o = t("b"), t("a"), t("o")
+        self.w_ba = _cat_rows([self.w_b, self.w_a])          # one product where the chunk kernels take both
         self.conv_w = torch.cat([t("q.conv"), t("k.conv"), t("v.conv")], dim=0).contiguous()
         self.dt_bias, self.a_log, self.w_norm = t("dt_bias"), t("A_log"), t("norm")
 
@@ -206,19 +207,22 @@ class HeadDeltaMixer(Mixer):
         ws = self.rt.workspace
         f32 = torch.float32
         packed = _project(self.rt, x, self.w_in, ws.rows("rec_in", T, self.w_in.shape[0], x.dtype), T)
-        # what enters the recurrence leaves its product unrounded
-        b = ops.linear(x, self.w_b, out=ws.rows("delta_b", T, H, f32), out_dtype=f32)
-        a = ops.linear(x, self.w_a, out=ws.rows("delta_a1", T, H, f32), out_dtype=f32)
-        qn, kn = ws.rows("delta_q", T, G * dk, f32), ws.rows("delta_k", T, G * dk, f32)
-        vv, gg, bb = ws.rows("delta_v", T, H * dv, f32), ws.rows("delta_g1", T, H, f32), ws.rows("delta_beta", T, H, f32)
-        ops.delta_prep(qn, kn, vv, gg, bb, packed, 0, self.conv_w, a, self.dt_bias, self.a_log, b, state, self.matrix_floats,
-                       ctx.seq_of_token, ctx.cu_seqlens, ctx.state_slots, H, G, dk, dv, decay_dim=1)
-        ops.conv_history(state, self.matrix_floats, packed, 0, self.channels, self.taps, ctx.cu_seqlens, ctx.state_slots, S)
         o = ws.rows("rec_o", T, H * dv, f32)
         q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * S
-        if not self.rt.plain_kernels and ops.delta_chunks_supported(x.dtype, dk, dv, state, q_lens):
-            ops.delta_chunks(o, qn, kn, vv, gg, bb, state, ctx.cu_seqlens, ctx.state_slots, q_lens, H, G, dk, dv, ws)
+        if not self.rt.plain_kernels and ops.delta_chunks_supported(packed, 0, self.taps, H, G, dk, dv, state, q_lens):
+            # what enters the recurrence leaves its product unrounded
+            ba = ops.linear(x, self.w_ba, out=ws.rows("delta_ba", T, 2 * H, f32), out_dtype=f32)
+            ops.delta_chunks(o, packed, 0, self.conv_w, ba, self.dt_bias, self.a_log, state, self.matrix_floats, ctx.cu_seqlens, ctx.state_slots,
+                             q_lens, H, G, dk, dv, ws)
+            ops.conv_history(state, self.matrix_floats, packed, 0, self.channels, self.taps, ctx.cu_seqlens, ctx.state_slots, S)
         else:
+            b = ops.linear(x, self.w_b, out=ws.rows("delta_b", T, H, f32), out_dtype=f32)
+            a = ops.linear(x, self.w_a, out=ws.rows("delta_a1", T, H, f32), out_dtype=f32)
+            qn, kn = ws.rows("delta_q", T, G * dk, f32), ws.rows("delta_k", T, G * dk, f32)
+            vv, gg, bb = ws.rows("delta_v", T, H * dv, f32), ws.rows("delta_g1", T, H, f32), ws.rows("delta_beta", T, H, f32)
+            ops.delta_prep(qn, kn, vv, gg, bb, packed, 0, self.conv_w, a, self.dt_bias, self.a_log, b, state, self.matrix_floats,
+                           ctx.seq_of_token, ctx.cu_seqlens, ctx.state_slots, H, G, dk, dv, decay_dim=1)
+            ops.conv_history(state, self.matrix_floats, packed, 0, self.channels, self.taps, ctx.cu_seqlens, ctx.state_slots, S)
             ops.delta_scan(o, qn, kn, vv, gg, bb, state, ctx.cu_seqlens, ctx.state_slots, S, H, G, dk, dv, decay_dim=1)
         y = ops.gated_norm(ws.rows("rec_y", T, H * dv, x.dtype), o, packed[:, self.g_off:self.g_off + H * dv], self.w_norm, H, self.eps,
                            gate_act="silu")

@@ -18,40 +18,50 @@ def rule(q, k, v, g, b, S):
     return o, S
 
 
-@pytest.mark.parametrize("H,G,dv,lens,held,decay", [
-    (2, 1, 128, [[33], [64], [1]], 96, "mixed"), (4, 2, 64, [[31, 65, 1], [40, 2, 97]], 96, "mixed"), (3, 3, 128, [[200, 70]], 2, "mixed"),
-    (2, 2, 128, [[100]], 96, "one"), (2, 2, 128, [[100]], 96, "zero"), (6, 3, 128, [[50] * 8], 96, "mixed")])
-def test_against_the_rule_token_by_token(H, G, dv, lens, held, decay):
+@pytest.mark.parametrize("H,G,dv,taps,lens,held,decay", [
+    (2, 1, 128, 4, [[33], [64], [1]], 96, "mixed"), (4, 2, 64, 3, [[31, 65, 1], [40, 2, 97]], 96, "mixed"), (3, 3, 128, 1, [[200, 70]], 2, "mixed"),
+    (2, 2, 128, 2, [[100]], 96, "one"), (2, 2, 128, 4, [[100]], 96, "zero"), (9, 3, 128, 4, [[50] * 8, [3] * 8], 96, "mixed")])
+def test_against_the_rule_token_by_token(H, G, dv, taps, lens, held, decay):
     from cppvllm_b200.csrc import ops
     from cppvllm_b200.parts.base import Workspace
     dk, d = 128, torch.device("cuda:0")
     gen = torch.Generator().manual_seed(H * 1000 + dv)
     S, extra = len(lens[0]), 6
-    slots = [(3 * s + 1) % (S + 1) for s in range(S)] if S % 3 != 2 else list(range(S - 1, -1, -1))
-    state = torch.randn(S + 1, H * dk * dv + extra, generator=gen) * 0.1
+    slots = list(range(S, 0, -1))
+    mat, C = H * dk * dv, 2 * G * dk + H * dv
+    state = torch.randn(S + 1, mat + (taps - 1) * C + extra, generator=gen) * 0.1
+    conv, dt_bias = torch.randn(C, taps, generator=gen) * 0.6, torch.randn(H, generator=gen)
+    a_log = {"mixed": torch.randn(H, generator=gen) - 1, "one": torch.full((H,), -60.0), "zero": torch.full((H,), 8.0)}[decay]
     want_state = state.to(F).clone()
     on_gpu = state.to(d)
     ws = Workspace(d, 1024, 8)
     before, ops.DELTA_CHUNKS_HELD = ops.DELTA_CHUNKS_HELD, held
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=d)             # noqa: E731
     try:
         for step in lens:                                            # portions, one after the other
-            T = sum(step)
-            unit = lambda x: x / x.norm(dim=-1, keepdim=True)        # noqa: E731
-            q, k = unit(torch.randn(T, G, dk, generator=gen)) * dk ** -0.5, unit(torch.randn(T, G, dk, generator=gen))
-            v, b = torch.randn(T, H, dv, generator=gen), torch.rand(T, H, generator=gen)
-            g = {"mixed": torch.rand(T, H, generator=gen) ** 0.2, "one": torch.ones(T, H), "zero": torch.zeros(T, H)}[decay]
+            T, off = sum(step), 2
+            packed = torch.randn(T, off + C + 4, generator=gen).to(torch.bfloat16)
+            a, b = torch.randn(T, H, generator=gen), torch.randn(T, H, generator=gen)
             cu, want = [0], []
             for s, n in enumerate(step):
-                a, e = cu[-1], cu[-1] + n
-                cu.append(e)
-                share = H // G
-                M = want_state[slots[s], :H * dk * dv].view(H, dk, dv)
-                o, M = rule(q[a:e].to(F).repeat_interleave(share, 1), k[a:e].to(F).repeat_interleave(share, 1), v[a:e].to(F), g[a:e].to(F), b[a:e].to(F), M)
-                want_state[slots[s], :H * dk * dv] = M.reshape(-1)
+                e = slice(cu[-1], cu[-1] + n)
+                cu.append(cu[-1] + n)
+                hist = want_state[slots[s], mat:mat + (taps - 1) * C].view(taps - 1, C)
+                u = torch.cat([hist, packed[e, off:off + C].to(F)])
+                y = sum(u[j:j + n] * conv[:, j].to(F) for j in range(taps))
+                y = y / (1 + torch.exp(-y))
+                unit = lambda x: x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6)        # noqa: E731
+                q, k, v = unit(y[:, :G * dk].view(n, G, dk)) * dk ** -0.5, unit(y[:, G * dk:2 * G * dk].view(n, G, dk)), y[:, 2 * G * dk:].view(n, H, dv)
+                g = torch.exp(-torch.exp(a_log.to(F)) * torch.nn.functional.softplus(a[e].to(F) + dt_bias.to(F), threshold=60.0))
+                M = want_state[slots[s], :mat].view(H, dk, dv)
+                o, M = rule(q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1), v, g, torch.sigmoid(b[e].to(F)), M)
+                want_state[slots[s], :mat] = M.reshape(-1)
+                want_state[slots[s], mat:mat + (taps - 1) * C] = u[n:].reshape(-1)
                 want.append(o)
             out = torch.full((T, H * dv), 9.0, device=d)
-            i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=d)     # noqa: E731
-            ops.delta_chunks(out, *(t.reshape(T, -1).contiguous().to(d) for t in (q, k, v, g, b)), on_gpu, i32(cu), i32(slots), step, H, G, dk, dv, ws)
+            dev = packed.to(d)
+            ops.delta_chunks(out, dev, off, conv.to(d), torch.cat([b, a], 1).to(d), dt_bias.to(d), a_log.to(d), on_gpu, mat, i32(cu), i32(slots), step, H, G, dk, dv, ws)
+            ops.conv_history(on_gpu, mat, dev, off, C, taps, i32(cu), i32(slots), S)
             torch.cuda.synchronize()
             ops.check_device_errors(d)
             got, want = out.cpu().to(F), torch.cat(want).reshape(T, -1)
@@ -67,7 +77,10 @@ def test_against_the_rule_token_by_token(H, G, dv, lens, held, decay):
 
 def test_what_the_rule_leaves_to_the_scan():
     from cppvllm_b200.csrc import ops
-    state = torch.zeros(2, 128 * 128 + 1)
-    ok = lambda dt=torch.bfloat16, dk=128, dv=128, w=128 * 128, n=33: ops.delta_chunks_supported(dt, dk, dv, state[:, :w], [1, n])     # noqa: E731
-    assert ok() and ok(dv=64)
-    assert not ok(dt=torch.float32) and not ok(dk=64) and not ok(dv=96) and not ok(w=128 * 128 + 1) and not ok(n=32)
+    state, row = torch.zeros(2, 128 * 128 + 1), torch.zeros(40, 513, dtype=torch.bfloat16)
+
+    def ok(packed=row[:, :512].contiguous(), off=0, taps=4, H=4, dk=128, dv=128, w=128 * 128, n=64):
+        return ops.delta_chunks_supported(packed, off, taps, H, 2, dk, dv, state[:, :w], [1, n])
+    assert ok() and ok(dv=64) and ok(off=2)
+    assert not ok(packed=row[:, :512].float()) and not ok(packed=row) and not ok(off=1) and not ok(taps=5)
+    assert not ok(dk=64) and not ok(dv=96) and not ok(w=128 * 128 + 1) and not ok(n=63) and not ok(H=8)
