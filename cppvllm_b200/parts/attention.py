@@ -207,6 +207,11 @@ class PagedAttention(Mixer):
                 ops.attn_decode_bf16(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, S, H, KV, hd,
                                      g.page_size, self.scale, splits, scratch, window=self.window)
             return
+        q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
+        if not self.force_general and ops.attn_prefill_f32_supported(q.dtype, H, KV, hd, q_lens):
+            ops.attn_prefill_f32(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, KV, hd, g.page_size, self.scale,
+                                 window=self.window)
+            return
         ops.paged_attention_general(att, q, cache.pages, g.block_tables, ctx.seq_of_token, ctx.positions,
                                     self.num_heads, self.num_kv_heads, self.head_dim, g.page_size, self.scale,
                                     window=self.window, num_tokens=ctx.num_tokens)
