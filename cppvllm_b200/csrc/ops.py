@@ -115,6 +115,9 @@ _err_flags = {}
 
 def error_flag(device) -> torch.Tensor:
     """One int32 per device that kernels set when they meet an index they refuse to follow."""
+    f = _err_flags.get(device.index) if type(device) is torch.device else None
+    if f is not None:
+        return f
     device = torch.device(device)
     key = device.index if device.index is not None else torch.cuda.current_device()
     f = _err_flags.get(key)
@@ -389,6 +392,8 @@ def _sandwich_lib():
         lib = load_library("sandwich")
         for name in ("cvb_input_conv", "cvb_gated_norm_add", "cvb_glu_act", "cvb_add_gated_rows", "cvb_wide_qk_prep"):
             getattr(lib, name).restype = c_int
+        lib.cvb_wide_qk_prep.argtypes = ([c_void_p] * 3 + [c_int] * 2 + [c_void_p] * 4 + [c_int] * 5 + [c_int64, c_float, c_float] + [c_int] * 3
+                                         + [c_void_p] * 2)              # declared, so that a call converts plain numbers itself
         _sandwich = lib
     return _sandwich
 
@@ -489,10 +494,10 @@ def wide_qk_prep(q_out: torch.Tensor, packed: torch.Tensor, q_weight: torch.Tens
         raise KernelError("wide_qk_prep: q_out [T, nq] and pages like packed; weights float32; positions, slots int32")
     num_pages = pages.numel() // (num_kv_heads * page_size * (dim + vdim)) if write else 0
     _check(_sandwich_lib().cvb_wide_qk_prep(
-        _ptr(q_out), _ptr(pages), _ptr(packed), c_int(T), c_int(packed.shape[1]), _ptr(q_weight), _ptr(k_weight), _ptr(positions),
-        _ptr(slots), c_int(nq), c_int(num_kv_heads), c_int(dim), c_int(vdim), c_int(page_size), c_int64(num_pages), c_float(eps),
-        c_float(temp_coef), c_int(temp_every), c_int(1 if write else 0), c_int(dtype_code(packed.dtype)),
-        _ptr(error_flag(packed.device)), _stream()), "wide_qk_prep")
+        q_out.data_ptr(), pages.data_ptr() if pages is not None else None, packed.data_ptr(), T, packed.shape[1], q_weight.data_ptr(),
+        k_weight.data_ptr() if k_weight is not None else None, positions.data_ptr(), slots.data_ptr() if slots is not None else None, nq,
+        num_kv_heads, dim, vdim, page_size, num_pages, eps, temp_coef, temp_every, 1 if write else 0, dtype_code(packed.dtype),
+        error_flag(packed.device).data_ptr(), _stream()), "wide_qk_prep")
     return q_out
 
 
@@ -1228,13 +1233,20 @@ def attn_entries_tcgen05(out: torch.Tensor, q: torch.Tensor, pages: torch.Tensor
     attn_bias_bf16 (`bias`) and attn_keys_bf16.  `table_len`: distances that `bias` or `r1`, `r2` distinguish (r1, r2: at least as many as
     the mask lets through).  `visible`: the most entries a token can see (it decides whether long query blocks are worked on by several
     blocks, whose shares go through scratch of the `workspace`; `pieces`, `min_rounds` > 0 force that choice)."""
-    H, G, bf, f32 = num_heads, num_kv_heads, torch.bfloat16, torch.float32
-    for t, dtype in ((out, bf), (q, bf), (gate, bf), (pages, bf), (block_tables, torch.int32), (cu_seqlens, torch.int32), (positions, torch.int32),
-                     (bias, f32), (r1, f32), (r2, f32), (sink, f32)):
-        if t is not None and (t.dtype != dtype or not t.is_cuda or not (t is out or t is q or t is gate or t.is_contiguous())):
-            raise KernelError("attn_entries_tcgen05: CUDA tensors; queries, pages, gate and output bf16, tables and positions int32, terms float32; "
-                              "all but queries, gate and output contiguous")
-    if block_tables.dim() != 2 or any(t is not None and t.numel() != H for t in (r1, r2, sink)) or (bias is not None and (bias.dim() != 2 or bias.shape[0] != H)):
+    H, G, bf, f32, i32 = num_heads, num_kv_heads, torch.bfloat16, torch.float32, torch.int32
+
+    def bad_term(t):
+        return t.dtype != f32 or not t.is_cuda or not t.is_contiguous()
+    # written out: as a loop over eleven pairs the checks took as long as the launch, which a step of a few short portions waits for
+    if (out.dtype != bf or q.dtype != bf or pages.dtype != bf or block_tables.dtype != i32 or cu_seqlens.dtype != i32 or positions.dtype != i32
+            or not (out.is_cuda and q.is_cuda and pages.is_cuda and block_tables.is_cuda and cu_seqlens.is_cuda and positions.is_cuda)
+            or not (pages.is_contiguous() and block_tables.is_contiguous() and cu_seqlens.is_contiguous() and positions.is_contiguous())
+            or (gate is not None and (gate.dtype != bf or not gate.is_cuda)) or (bias is not None and bad_term(bias))
+            or (r1 is not None and bad_term(r1)) or (r2 is not None and bad_term(r2)) or (sink is not None and bad_term(sink))):
+        raise KernelError("attn_entries_tcgen05: CUDA tensors; queries, pages, gate and output bf16, tables and positions int32, terms float32; "
+                          "all but queries, gate and output contiguous")
+    if (block_tables.dim() != 2 or (bias is not None and (bias.dim() != 2 or bias.shape[0] != H)) or (r1 is not None and r1.numel() != H)
+            or (r2 is not None and r2.numel() != H) or (sink is not None and sink.numel() != H)):
         raise KernelError("attn_entries_tcgen05: block_tables [S, W]; r1, r2 and sink [H], bias [H, L]")
     if q.dim() != 2 or q.shape[1] < H * dim or q.stride(1) != 1 or out.dim() != 2 or out.shape[1] != H * vdim or out.stride(1) != 1:
         raise KernelError("attn_entries_tcgen05: q [T, >= H * dim], out [T, H * vdim]")
