@@ -126,7 +126,8 @@ __device__ __forceinline__ float2 tanh_small2(float2 x) {
 }
 __device__ __forceinline__ float tanh_exponential(float x) { return 1.f - __fdividef(2.f, 1.f + __expf(2.f * x)); }
 
-// SHARED: one entry is key and value.  TERMS: a cap or a distance table (else the scale joins the exponent's multiply-add).
+// SHARED: one entry is key and value.  TERMS: a cap or a distance table (else the scale joins the exponent's multiply-add, behind the mask and
+// the maximum: it must be above 0).
 template <int HD, int DV, bool SHARED, bool TERMS>
 __global__ void __launch_bounds__(kEThreads, 1)
 attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const EntryAttnParams p) {
@@ -735,6 +736,7 @@ extern "C" int cvb_attn_entries_tcgen05(void* out, int out_stride, const void* q
     if ((bias != nullptr && bias_len != table_len) || ((bias != nullptr || r1 != nullptr) != (table_len > 0)) || (r1 != nullptr) != (r2 != nullptr)) return CVB_E_SHAPE;
     const bool terms = softcap > 0.f || table_len > 0;
     if (shared && terms) return CVB_E_UNSUPPORTED;
+    if (!terms && !(scale > 0.f)) return CVB_E_UNSUPPORTED;         // such scores are masked and their maximum taken before the scale
     if (q_stride < H * dk || out_stride < H * dv || q_stride % 8 || out_stride % 8) return CVB_E_ALIGN;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(pages) | reinterpret_cast<uintptr_t>(out)) & 15) return CVB_E_ALIGN;
     if (gate != nullptr && gate_element && (gate_stride % 8 || (reinterpret_cast<uintptr_t>(gate) & 15))) return CVB_E_ALIGN;

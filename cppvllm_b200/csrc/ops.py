@@ -1209,14 +1209,15 @@ ENTRIES_MIN_VISIBLE = 128
 
 
 def attn_entries_supported(q: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor], num_heads: int, num_kv_heads: int, dim: int, vdim: int,
-                           page_size: int, visible: int, shared: bool = False, table_len: int = 0) -> bool:
+                           page_size: int, visible: int, shared: bool = False, table_len: int = 0, scale: float = 1.0, softcap: float = 0.0) -> bool:
     """Whether the tcgen05 kernel takes a portion (csrc/attention_entries_tcgen05.cu): bf16, keys of 64 or 128 elements and values as wide
     (`shared`: the entry is key and value; 96 of 128 too), pages of 2^n >= 16 tokens, a distance table of `table_len` entries per head that
-    fits beside its tiles, rows of q, out and a gate per element on 16-byte boundaries (the mma.sync kernels ask for less), and tokens that
+    fits beside its tiles, rows of q, out and a gate per element on 16-byte boundaries (the mma.sync kernels ask for less), a scale above 0
+    where no cap or distance term follows it (such scores are masked and compared before the scale, which joins the exponent), and tokens that
     see at least ENTRIES_MIN_VISIBLE entries at most."""
     def rows16(t):
         return t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
-    return (visible >= ENTRIES_MIN_VISIBLE and q.dtype == torch.bfloat16
+    return (visible >= ENTRIES_MIN_VISIBLE and q.dtype == torch.bfloat16 and (scale > 0 or softcap > 0 or table_len > 0)
             and _attn_entries_shape(num_heads, num_kv_heads, dim, vdim, shared, page_size, table_len)
             and rows16(q) and rows16(out) and (gate is None or gate.shape[1] == num_heads or rows16(gate)))
 

@@ -163,7 +163,8 @@ class MaskedAttention(Mixer):
         # distances that the mask lets through, for the tcgen05 kernel's table; without a bound the term goes to the other kernels
         reach = min([n for n in (self.chunk, self.window if not self.keep_first else 0) if n], default=0) if self.r1 is not None else 0
         if (not self.force_general and not (ctx.all_decode and ctx.num_tokens == ctx.num_seqs) and (self.r1 is None or reach)
-                and ops.attn_entries_supported(q, att, gate, H, G, dk, dv, g.page_size, self._visible(ctx), table_len=reach)):
+                and ops.attn_entries_supported(q, att, gate, H, G, dk, dv, g.page_size, self._visible(ctx), table_len=reach, scale=self.scale,
+                                               softcap=self.softcap)):
             q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv, g.page_size,
                                      self.scale, self._visible(ctx), workspace=self.rt.workspace, planes=self.planes, chunk=self.chunk,
