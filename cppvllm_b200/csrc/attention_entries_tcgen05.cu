@@ -618,12 +618,12 @@ attn_entries_merge_kernel(const EntryAttnParams p, const int dv) {
     float m_all = p.sink != nullptr ? p.sink[head] * kELog2e : -INFINITY, l = 0.f;
 #pragma unroll
     for (int k = 0; k < kEMaxPieces; ++k) {
-        if (!(sum[k] > 0.f)) w[k] = -INFINITY;                      // a piece without a key for this row
+        if (sum[k] == 0.f) w[k] = -INFINITY;                        // a piece without a key for this row; a NaN stays
         m_all = fmaxf(m_all, w[k]);
     }
 #pragma unroll
     for (int k = 0; k < kEMaxPieces; ++k) {
-        w[k] = w[k] == -INFINITY ? 0.f : ex2(w[k] - m_all);
+        w[k] = sum[k] == 0.f ? 0.f : ex2(w[k] - m_all);
         l = __fadd_rn(l, __fmul_rn(sum[k], w[k]));
     }
     if (p.sink != nullptr) l += ex2(p.sink[head] * kELog2e - m_all);
@@ -632,12 +632,12 @@ attn_entries_merge_kernel(const EntryAttnParams p, const int dv) {
     for (int c = 0; c < 32; ++c) acc[c] = 0.f;
 #pragma unroll
     for (int k = 0; k < kEMaxPieces; ++k) {
-        if (k >= n_pieces || w[k] == 0.f) continue;
+        if (sum[k] == 0.f) continue;                                // never written
         const float* share = p.part_o + ((first + k) * 2 + x) * (static_cast<int64_t>(dv) * 128) + static_cast<int64_t>(c0) * 128 + r;
 #pragma unroll
         for (int c = 0; c < 32; ++c) acc[c] = __fadd_rn(acc[c], __fmul_rn(__ldcg(share + c * 128), w[k]));
     }
-    float inv = l > 0.f ? p.out_scale / l : 0.f;
+    float inv = l == 0.f ? 0.f : p.out_scale / l;
     if (p.gate != nullptr) {
         const __nv_bfloat16* grow = p.gate + t_abs * p.gate_stride;
         if (p.gate_element) {

@@ -181,3 +181,42 @@ def test_what_the_rule_leaves_to_the_other_kernels():
     assert not takes(q, wide[:, 4:], None, 128, 128, 32)
     assert not takes(q, out, wide[:, 4:], 128, 128, 32)
     assert not takes(q, out, None, 128, 96, 32)                      # 96 of 128 only where one entry is key and value
+
+
+def one_request(H, G, dim, shared, n, cached, page=32, seed=3):
+    """A request's queries and pages (in order, all in use), bf16 on the host."""
+    gen = torch.Generator().manual_seed(seed)
+    pages = torch.randn(-(-(n + cached) // page), 1, G, page, dim if shared else 2 * dim, generator=gen).to(torch.bfloat16)
+    return torch.randn(n, H * dim, generator=gen).to(torch.bfloat16), pages
+
+
+def run_one(q, pages, H, G, dim, shared, n, cached, pieces=1, scale=0.1, **kw):
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.parts.base import Workspace
+    d = dev()
+
+    def i32(x):
+        return torch.as_tensor(x, dtype=torch.int32).to(d)
+    out = torch.zeros(n, H * dim, dtype=torch.bfloat16, device=d)
+    ops.attn_entries_tcgen05(out, q.to(d), pages.to(d), i32([list(range(pages.shape[0]))]), i32([0, n]), i32(range(cached, cached + n)), [n], H, G, dim, dim,
+                             pages.shape[3], scale, 1 << 20 if pieces > 1 else 1, workspace=Workspace(d, 1024, 8), shared=shared, pieces=pieces,
+                             min_rounds=2, **kw)
+    torch.cuda.synchronize()
+    ops.check_device_errors(d)
+    return out.cpu().view(n, H, dim)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("pieces", [1, 4])
+def test_a_nan_is_answered_with_nan(shared, pieces):
+    """A NaN in a key spoils the rows that see it, a NaN in a query its own row, and no other, whether the query block is cut or not."""
+    H, G, dim, n, cached = 4, 2, 128, 40, 2100
+    q, pages = one_request(H, G, dim, shared, n, cached)
+    pages[700 // 32, 0, 1, 700 % 32, 3] = math.nan
+    q[5, 7] = math.nan
+    out = run_one(q, pages, H, G, dim, shared, n, cached, pieces)
+    want = torch.zeros(n, H, dtype=torch.bool)
+    want[:, 2:] = True
+    want[5, 0] = True
+    assert torch.equal(torch.isnan(out).all(-1), want) and not torch.isnan(out[~want]).any()
