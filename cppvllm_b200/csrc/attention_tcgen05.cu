@@ -541,12 +541,12 @@ attn_prefill_merge_kernel(const TcAttnParams p, const int skip_single, const int
     float m_all = -INFINITY, l = 0.f;
 #pragma unroll
     for (int k = 0; k < kMaxPieces; ++k) {
-        if (!(sum[k] > 0.f)) w[k] = -INFINITY;                      // a piece without a key for this row
+        if (sum[k] == 0.f) w[k] = -INFINITY;                        // a piece without a key for this row; a NaN stays
         m_all = fmaxf(m_all, w[k]);
     }
 #pragma unroll
     for (int k = 0; k < kMaxPieces; ++k) {
-        w[k] = w[k] == -INFINITY ? 0.f : ex2(w[k] - m_all);
+        w[k] = sum[k] == 0.f ? 0.f : ex2(w[k] - m_all);
         l = __fadd_rn(l, __fmul_rn(sum[k], w[k]));
     }
     float acc[32];
@@ -554,12 +554,12 @@ attn_prefill_merge_kernel(const TcAttnParams p, const int skip_single, const int
     for (int c = 0; c < 32; ++c) acc[c] = 0.f;
 #pragma unroll
     for (int k = 0; k < kMaxPieces; ++k) {
-        if (k >= n_pieces || w[k] == 0.f) continue;
+        if (sum[k] == 0.f) continue;                                // never written
         const float* share = p.part_o + ((first + k) * 2 + x) * (static_cast<int64_t>(hd) * 128) + static_cast<int64_t>(c0) * 128 + r;
 #pragma unroll
         for (int c = 0; c < 32; ++c) acc[c] = __fadd_rn(acc[c], __fmul_rn(__ldcg(share + c * 128), w[k]));
     }
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    const float inv = l == 0.f ? 0.f : 1.f / l;
 #pragma unroll
     for (int k = 0; k < 32; k += 8) {
         uint4 t;

@@ -475,6 +475,29 @@ def test_tcgen05_prefill_shares_the_keys_of_long_query_blocks_among_blocks(ops, 
         assert torch.isfinite(got).all() and (got[rows] - rnd(ref, dt)[rows]).abs().max() < 2e-2
 
 
+@pytest.mark.parametrize("pieces", [1, 4])
+def test_attention_tcgen05_answers_a_nan_with_nan_in_pieces_too(pieces):
+    """A NaN in a key of kv head 1 spoils the rows that see it (its query heads', from its position on), a NaN in a query that row, and no other."""
+    from cppvllm_b200.csrc import ops
+    H, KV, hd, page, c, n, dt, d = 4, 2, 128, 32, 900, 200, torch.bfloat16, dev()
+    g = torch.Generator().manual_seed(11)
+    k, v = (torch.randn(c + n, KV, hd, generator=g).to(dt) for _ in range(2))
+    q = torch.randn(n, H, hd, generator=g).to(dt)
+    k[950, 1, 3], q[5, 0, 7] = float("nan"), float("nan")
+    cache, tables = build_paged([k], [v], page, (c + n + page - 1) // page + 1, KV, hd, dt, g)
+    tiles = ops.prefill_tiles_tcgen05([n], H, KV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=d)                                 # noqa: E731
+    scratch = torch.full((ops.attn_prefill_tcgen05_scratch_floats(tiles, KV, hd, pieces),), float("nan"), device=d)
+    out = ops.attn_prefill_tcgen05(torch.zeros(n, H * hd, dtype=dt, device=d), q.view(n, -1).to(d), cache.to(d), tables.to(d), i32([0, n]),
+                                   i32(list(range(c, c + n))), 1, tiles, H, KV, hd, page, 0.1, pieces=pieces, min_rounds=2, scratch=scratch,
+                                   piece_counts=i32([0] * (tiles * KV)))
+    ops.check_device_errors(d)
+    want = torch.zeros(n, H, dtype=torch.bool)
+    want[50:, 2:], want[5, 0] = True, True
+    bad = torch.isnan(out.cpu().view(n, H, hd))
+    assert torch.equal(bad.all(-1), want) and not bad[~want].any()
+
+
 @pytest.mark.parametrize("seed", [0, 1, 2, 3, 4, 5])
 def test_tcgen05_prefill_pieces_at_random_shapes(ops, seed):
     """Random requests (tokens in the cache, tokens in the step), heads, pages, windows, piece counts and piece lengths:
