@@ -286,10 +286,12 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                 // nearest box that does stands in for it.
                 int key = first_key(it) + box * p.box_rows;
                 if (pooled) key = min(key, nb_max - 1);
-                else if (key >= keep) {
-                    if (it < n_pool + n_kept) key = keep - 1;
-                    else if (key + p.box_rows <= key_lo) key = key_lo;
-                    else key = min(key, key_hi);
+                else {
+                    key = min(key, key_hi);                          // a request may be shorter than the kept first tokens
+                    if (key >= keep) {
+                        if (it < n_pool + n_kept) key = keep - 1;
+                        else if (key + p.box_rows <= key_lo) key = key_lo;
+                    }
                 }
                 key &= ~(p.box_rows - 1);
                 const int slot = key >> page_shift;

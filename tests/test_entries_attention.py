@@ -70,6 +70,10 @@ CASES = [
     (3, 3, 64, 64, True, 16, {"window": 300, "keep": 200}, None, [(260, 500)], 2),
     (4, 2, 128, 128, False, 32, {"bias": 33}, None, [(300, 0), (5, 77)], 0),
     (8, 2, 64, 64, False, 32, {"bias": 1025}, None, [(200, 2000)], 4),
+    # requests shorter than what is kept: the block tables hold nothing behind them
+    (4, 2, 128, 128, False, 32, {"window": 1024, "keep": 200}, None, [(130, 0)], 0),
+    (8, 2, 128, 128, True, 16, {"window": 1024, "keep": 200}, None, [(5, 0), (300, 0)], 0),
+    (4, 2, 64, 64, False, 64, {"window": 90, "keep": 500, "cap": 2.0}, "head", [(150, 0), (3, 190), (70, 400)], 0),
 ]
 
 
