@@ -734,6 +734,7 @@ extern "C" int cvb_attn_entries_tcgen05(void* out, int out_stride, const void* q
     if (num_tiles == 0) return CVB_OK;
     if (num_tiles < 0 || num_tiles > 65535 || S <= 0 || table_width <= 0 || num_pages <= 0 || planes < 1 || planes > 2 || bias_len < 0) return CVB_E_SIZE;
     if (chunk < 0 || window < 0 || pool < 0 || keep < 0 || (pool > 0 && planes != 2)) return CVB_E_SIZE;
+    if ((pool > 0 || keep > 0) && window == 0) return CVB_E_SHAPE;  // they stand beside a window
     if (!cvb_attn_entries_supported(H, G, dk, dv, shared, page_size, table_len)) return CVB_E_UNSUPPORTED;
     if ((bias != nullptr && bias_len != table_len) || ((bias != nullptr || r1 != nullptr) != (table_len > 0)) || (r1 != nullptr) != (r2 != nullptr)) return CVB_E_SHAPE;
     const bool terms = softcap > 0.f || table_len > 0;

@@ -161,7 +161,8 @@ class MaskedAttention(Mixer):
     def attend(self, att, q, gate, ctx, cache, g, out_scale=1.0):
         H, G, dk, dv = self.num_heads, self.num_kv_heads, self.dim, self.vdim
         # distances that the mask lets through, for the tcgen05 kernel's table; without a bound the term goes to the other kernels
-        reach = min([n for n in (self.chunk, self.window if not self.keep_first else 0) if n], default=0) if self.r1 is not None else 0
+        # (kept first tokens are seen from any distance)
+        reach = min([n for n in (self.chunk, self.window) if n], default=0) if self.r1 is not None and not self.keep_first else 0
         if (not self.force_general and not (ctx.all_decode and ctx.num_tokens == ctx.num_seqs) and (self.r1 is None or reach)
                 and ops.attn_entries_supported(q, att, gate, H, G, dk, dv, g.page_size, self._visible(ctx), table_len=reach, scale=self.scale,
                                                softcap=self.softcap)):

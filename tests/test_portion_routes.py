@@ -154,3 +154,9 @@ def test_the_kernel_refuses_a_scale_it_would_apply_behind_the_mask():
         assert ops.attn_entries_supported(q, out, None, 4, 2, 128, 128, PAGE, 1000, scale=scale, softcap=1.0)
         with pytest.raises(ops.KernelError):
             ops.attn_entries_tcgen05(out, q, pages, i32([[0, 1]]), i32([0, 8]), i32(range(8)), [8], 4, 2, 128, 128, PAGE, scale, 8, Workspace(dev, 64, 4))
+
+
+def test_kept_first_tokens_with_a_distance_term(monkeypatch):
+    """They are seen from beyond the chunk and the window: no table of distances is long enough, and the step stays with the other kernels."""
+    diffs = both(monkeypatch, "attn_masked_bf16", "masked_attention", chunk=150, window=140, keep_first=20, distance_bias=True)
+    assert max(diffs) < BF16, diffs
