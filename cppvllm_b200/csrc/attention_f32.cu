@@ -12,6 +12,8 @@
 #include "common.cuh"
 #include "sm100.cuh"
 
+#include <cuda/std/type_traits>
+
 namespace cvb {
 
 constexpr int kFRows = 64;
@@ -82,6 +84,7 @@ attn_prefill_f32_kernel(const F32AttnParams p) {
     const int pos0 = p.positions[cu0 + q0];
     const int key_hi = pos0 + n_tok - 1;                  // a request's tokens of a step sit at consecutive positions
     const int key_lo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+    const int last_lo = p.window > 0 ? max(0, key_hi - p.window + 1) : 0;                 // where the last token's window begins
     const int tile0 = key_lo / kFKeys, n_tiles = key_hi / kFKeys - tile0 + 1;
     pdl_wait();
     for (int i = threadIdx.x; i < kFRows * CPR; i += 2 * kFThreads) {
@@ -191,27 +194,34 @@ attn_prefill_f32_kernel(const F32AttnParams p) {
         cp_async_wait<0>();
         half_sync();                                      // the values are there, and nobody reads the keys any more
         load_tile(it + 2, false);
+        auto weigh = [&](auto edge) {
 #pragma unroll 2
-        for (int j = 0; j < kFKeys; j += 4) {
-            float4 a[4];
+            for (int j = 0; j < kFKeys; j += 4) {
+                float4 a[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sP + (ty * 4 + i) * LP + j);
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(sP + (ty * 4 + i) * LP + j);
 #pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
+                for (int jj = 0; jj < 4; ++jj) {
 #pragma unroll
-                for (int c = 0; c < HD / 64; ++c) {
-                    const float4 v = *reinterpret_cast<const float4*>(sV + (j + jj) * LD + c * 64 + tx * 4);
+                    for (int c = 0; c < HD / 64; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(sV + (j + jj) * LD + c * 64 + tx * 4);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float pj = jj == 0 ? a[i].x : jj == 1 ? a[i].y : jj == 2 ? a[i].z : a[i].w;
-                        o[i][c * 4] = fmaf(pj, v.x, o[i][c * 4]);
-                        o[i][c * 4 + 1] = fmaf(pj, v.y, o[i][c * 4 + 1]);
-                        o[i][c * 4 + 2] = fmaf(pj, v.z, o[i][c * 4 + 2]);
-                        o[i][c * 4 + 3] = fmaf(pj, v.w, o[i][c * 4 + 3]);
+                        for (int i = 0; i < 4; ++i) {
+                            if (decltype(edge)::value && (key0 + j + jj > row_pos[i] || key0 + j + jj < row_lo[i])) continue;
+                            const float pj = jj == 0 ? a[i].x : jj == 1 ? a[i].y : jj == 2 ? a[i].z : a[i].w;
+                            o[i][c * 4] = fmaf(pj, v.x, o[i][c * 4]);
+                            o[i][c * 4 + 1] = fmaf(pj, v.y, o[i][c * 4 + 1]);
+                            o[i][c * 4 + 2] = fmaf(pj, v.z, o[i][c * 4 + 2]);
+                            o[i][c * 4 + 3] = fmaf(pj, v.w, o[i][c * 4 + 3]);
+                        }
                     }
                 }
             }
-        }
+        };
+        // Where some row of the block does not see a key of the tile, that key's value is left out of the row's sum, not weighed with 0: an
+        // infinity or a NaN in a later token's value must not reach the tokens before it.
+        if (key0 + kFKeys - 1 <= pos0 && key0 >= last_lo) weigh(cuda::std::false_type{});
+        else weigh(cuda::std::true_type{});
         half_sync();                                      // nobody reads the values any more
         load_tile(it + 2, true);
     }

@@ -56,3 +56,27 @@ def test_what_stays_with_the_general_kernel():
     ok = ops.attn_prefill_f32_supported
     assert ok(torch.float32, 4, 2, 128, [1, 32]) and not ok(torch.float32, 4, 2, 128, [1, 31]) and not ok(torch.float32, 4, 2, 32, [32])
     assert not ok(torch.bfloat16, 4, 2, 128, [32]) and not ok(torch.float32, 65, 1, 64, [32])
+
+
+@pytest.mark.parametrize("window", [0, 20])
+@pytest.mark.parametrize("plane", [0, 1])
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+def test_a_bad_token_reaches_no_token_that_does_not_see_it(window, plane, bad):
+    from cppvllm_b200.csrc import ops
+    gen, d = torch.Generator().manual_seed(5), torch.device("cuda:0")
+    H, KV, hd, n, page, at = 4, 2, 128, 100, 32, 40
+    pages, q = torch.randn(4, 2, KV, page, hd, generator=gen), torch.randn(n, H * hd, generator=gen)
+    i32 = lambda x: torch.as_tensor(x, dtype=torch.int32).to(d)      # noqa: E731
+
+    def run(p):
+        out = torch.empty(n, H * hd, device=d)
+        ops.attn_prefill_f32(out, q.to(d), p.to(d), i32([[0, 1, 2, 3]]), i32([0, n]), i32(range(n)), [n], H, KV, hd, page, 0.1, window)
+        return out.cpu()
+    clean = run(pages)
+    pages[at // page, plane, :, at % page] = bad
+    got = run(pages)
+    sees = torch.zeros(n, dtype=torch.bool)
+    sees[at:at + window if window else n] = True
+    assert torch.equal(got[~sees], clean[~sees])
+    if plane == 1:
+        assert not torch.isfinite(got[sees]).any()
