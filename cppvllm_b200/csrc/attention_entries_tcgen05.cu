@@ -721,16 +721,21 @@ extern "C" int64_t cvb_attn_entries_scratch_floats(int num_tiles, int G, int dv,
     return static_cast<int64_t>(num_tiles) * G * pieces * 2 * (dv + 2) * 128;
 }
 
+// What a layer asks of the kernel whatever the step.
+struct EntryAttnShape {
+    int H, G, dk, dv, shared, page_size, planes, chunk, window, pool, keep, table_len;
+    float scale, softcap, out_scale;
+};
+
 // num_tiles: per request ceil(tokens / (2 * (128 / group))) query blocks.  `table_len` > 0: distances 0 .. table_len - 1 have an entry,
 // of `bias` [H, bias_len] (bias_len = table_len) or of r1, r2; larger distances take the last one (with r1, r2 the mask must rule them
 // out).  With pieces > 1 a query block of at least 2 * min_rounds tiles is worked on by up to `pieces` blocks.
-extern "C" int cvb_attn_entries_tcgen05(void* out, int out_stride, const void* q, int q_stride, const void* pages, const int* block_tables,
-                                        int table_width, const int* cu_seqlens, const int* positions, int S, int num_tiles, int H, int G, int dk,
-                                        int dv, int shared, int page_size, int planes, int num_pages, int chunk, int window, int pool, int keep,
-                                        float scale, float softcap, const float* bias, int bias_len, const float* r1, const float* r2,
-                                        int table_len, const float* sink, const void* gate, int gate_stride, int gate_element, float out_scale,
-                                        int pieces, int min_rounds, float* scratch, int64_t scratch_floats, int* piece_counts, int* err_flag,
-                                        cudaStream_t stream) {
+extern "C" int cvb_attn_entries_tcgen05(const EntryAttnShape* shape, void* out, int out_stride, const void* q, int q_stride, const void* pages,
+                                        int num_pages, const int* block_tables, int table_width, const int* cu_seqlens, const int* positions, int S,
+                                        int num_tiles, const float* bias, const float* r1, const float* r2, const float* sink, const void* gate,
+                                        int bias_len, int gate_stride, int gate_element, int pieces, int min_rounds, float* scratch,
+                                        int64_t scratch_floats, int* piece_counts, int* err_flag, cudaStream_t stream) {
+    const auto [H, G, dk, dv, shared, page_size, planes, chunk, window, pool, keep, table_len, scale, softcap, out_scale] = *shape;
     if (num_tiles == 0) return CVB_OK;
     if (num_tiles < 0 || num_tiles > 65535 || S <= 0 || table_width <= 0 || num_pages <= 0 || planes < 1 || planes > 2 || bias_len < 0) return CVB_E_SIZE;
     if (chunk < 0 || window < 0 || pool < 0 || keep < 0 || (pool > 0 && planes != 2)) return CVB_E_SIZE;

@@ -1186,18 +1186,28 @@ def _attn_entries_lib():
     global _attn_entries
     if _attn_entries is None:
         lib = load_library("attn_entries")
-        P, i, f = c_void_p, c_int, c_float      # declared, so that a call converts plain numbers itself (48 objects a call cost 5 us)
-        lib.cvb_attn_entries_tcgen05.argtypes = [P, i, P, i, P, P, i, P, P] + [i] * 14 + [f, f, P, i, P, P, i, P, P, i, i, f, i, i, P, c_int64, P, P, P]
+        P, i = c_void_p, c_int                  # declared, so that a call converts plain numbers itself
+        lib.cvb_attn_entries_tcgen05.argtypes = [P, P, i, P, i, P, i, P, i, P, P, i, i] + [P] * 5 + [i] * 5 + [P, c_int64, P, P, P]
         lib.cvb_attn_entries_tcgen05.restype = c_int
         lib.cvb_attn_entries_supported.restype = c_int
         _attn_entries = lib
     return _attn_entries
 
 
+class _EntriesShape(ctypes.Structure):
+    """What a layer asks of the kernel whatever the step (csrc/attention_entries_tcgen05.cu: EntryAttnShape)."""
+    _fields_ = [(n, c_int) for n in ("H", "G", "dk", "dv", "shared", "page_size", "planes", "chunk", "window", "pool", "keep", "table_len")] + [
+        (n, c_float) for n in ("scale", "softcap", "out_scale")]
+
+
 @functools.lru_cache(maxsize=256)
-def _attn_entries_shape(num_heads: int, num_kv_heads: int, dim: int, vdim: int, shared: bool, page_size: int, table_len: int) -> bool:
-    return bool(_attn_entries_lib().cvb_attn_entries_supported(c_int(num_heads), c_int(num_kv_heads), c_int(dim), c_int(vdim),
-                                                               c_int(1 if shared else 0), c_int(page_size), c_int(table_len)))
+def _attn_entries_shape(H, G, dk, dv, shared, page_size, planes, chunk, window, pool, keep, table_len, scale, softcap, out_scale):
+    """The shape as the kernel reads it, or None where it does not take it; kept, because a step asks for the same few again and again."""
+    if not _attn_entries_lib().cvb_attn_entries_supported(c_int(H), c_int(G), c_int(dk), c_int(dv), c_int(1 if shared else 0), c_int(page_size),
+                                                          c_int(table_len)) or not (scale > 0 or softcap > 0 or table_len > 0):
+        return None
+    shape = _EntriesShape(H, G, dk, dv, 1 if shared else 0, page_size, planes, chunk, window, pool, keep, table_len, scale, softcap, out_scale)
+    return shape, ctypes.addressof(shape)
 
 
 # What a block costs outside its tiles (tensor memory, barriers, the query tiles, the output through shared memory) is more than an
@@ -1217,8 +1227,8 @@ def attn_entries_supported(q: torch.Tensor, out: torch.Tensor, gate: Optional[to
     see at least ENTRIES_MIN_VISIBLE entries at most."""
     def rows16(t):
         return t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
-    return (visible >= ENTRIES_MIN_VISIBLE and q.dtype == torch.bfloat16 and (scale > 0 or softcap > 0 or table_len > 0)
-            and _attn_entries_shape(num_heads, num_kv_heads, dim, vdim, shared, page_size, table_len)
+    return (visible >= ENTRIES_MIN_VISIBLE and q.dtype == torch.bfloat16
+            and _attn_entries_shape(num_heads, num_kv_heads, dim, vdim, shared, page_size, 1, 0, 0, 0, 0, table_len, scale, softcap, 1.0) is not None
             and rows16(q) and rows16(out) and (gate is None or gate.shape[1] == num_heads or rows16(gate)))
 
 
@@ -1227,53 +1237,86 @@ def attn_entries_tcgen05(out: torch.Tensor, q: torch.Tensor, pages: torch.Tensor
                          visible: int, workspace=None, shared: bool = False, planes: int = 1, chunk: int = 0, window: int = 0, pool: int = 0,
                          keep_first: int = 0, softcap: float = 0.0, bias: Optional[torch.Tensor] = None, r1: Optional[torch.Tensor] = None,
                          r2: Optional[torch.Tensor] = None, table_len: int = 0, sink: Optional[torch.Tensor] = None,
-                         gate: Optional[torch.Tensor] = None, out_scale: float = 1.0, pieces: int = 0,
-                         min_rounds: int = 0) -> torch.Tensor:
+                         gate: Optional[torch.Tensor] = None, out_scale: float = 1.0, pieces: int = 0, min_rounds: int = 0,
+                         optional: bool = False) -> Optional[torch.Tensor]:
     """Attention of prompt portions (and single tokens among them) over pages [plane, kv head, slot, dim + vdim] of entries that hold a key and
     its value, or (`shared`) [kv head, slot, dim] whose first vdim elements are the value: the masks and terms of attn_masked_bf16,
     attn_bias_bf16 (`bias`) and attn_keys_bf16.  `table_len`: distances that `bias` or `r1`, `r2` distinguish (r1, r2: at least as many as
     the mask lets through).  `visible`: the most entries a token can see (it decides whether long query blocks are worked on by several
-    blocks, whose shares go through scratch of the `workspace`; `pieces`, `min_rounds` > 0 force that choice)."""
-    H, G, bf, f32, i32 = num_heads, num_kv_heads, torch.bfloat16, torch.float32, torch.int32
+    blocks, whose shares go through scratch of the `workspace`; `pieces`, `min_rounds` > 0 force that choice).  `optional`: a step that
+    attn_entries_supported leaves to the other kernels launches nothing and is answered with None.
 
-    def bad_term(t):
-        return t.dtype != f32 or not t.is_cuda or not t.is_contiguous()
-    # written out: as a loop over eleven pairs the checks took as long as the launch, which a step of a few short portions waits for
-    if (out.dtype != bf or q.dtype != bf or pages.dtype != bf or block_tables.dtype != i32 or cu_seqlens.dtype != i32 or positions.dtype != i32
-            or not (out.is_cuda and q.is_cuda and pages.is_cuda and block_tables.is_cuda and cu_seqlens.is_cuda and positions.is_cuda)
-            or not (pages.is_contiguous() and block_tables.is_contiguous() and cu_seqlens.is_contiguous() and positions.is_contiguous())
-            or (gate is not None and (gate.dtype != bf or not gate.is_cuda)) or (bias is not None and bad_term(bias))
-            or (r1 is not None and bad_term(r1)) or (r2 is not None and bad_term(r2)) or (sink is not None and bad_term(sink))):
-        raise KernelError("attn_entries_tcgen05: CUDA tensors; queries, pages, gate and output bf16, tables and positions int32, terms float32; "
-                          "all but queries, gate and output contiguous")
-    if (block_tables.dim() != 2 or (bias is not None and (bias.dim() != 2 or bias.shape[0] != H)) or (r1 is not None and r1.numel() != H)
-            or (r2 is not None and r2.numel() != H) or (sink is not None and sink.numel() != H)):
-        raise KernelError("attn_entries_tcgen05: block_tables [S, W]; r1, r2 and sink [H], bias [H, L]")
-    if q.dim() != 2 or q.shape[1] < H * dim or q.stride(1) != 1 or out.dim() != 2 or out.shape[1] != H * vdim or out.stride(1) != 1:
-        raise KernelError("attn_entries_tcgen05: q [T, >= H * dim], out [T, H * vdim]")
-    if gate is not None and (gate.shape[1] not in (H, H * vdim) or gate.stride(1) != 1):
-        raise KernelError("attn_entries_tcgen05: gate bf16 [T, H] or [T, H * vdim]")
-    num_tiles = prefill_tiles_tcgen05(q_lens, H, G, skip_single=False)
-    pieces = pieces or prefill_pieces_tcgen05(num_tiles, G, visible)
-    scratch = counts = None
+    A step of a few short portions waits for the host here.  So the rule and the call are one, alignment is left to the kernel's own check, and what
+    does not change between steps crosses to C as one structure.  On one core of the build machine the two take 9.4 us, as a rule of its own
+    and a call with 42 arguments they took 20.8; attn_keys_bf16, which such a step went to before, takes 10.6."""
+    shape = _attn_entries_shape(num_heads, num_kv_heads, dim, vdim, shared, page_size, planes, chunk, window, pool, keep_first, table_len, scale,
+                                softcap, out_scale)
+    bf, f32, i32 = torch.bfloat16, torch.float32, torch.int32
+    if shape is None or q.dtype is not bf:
+        if optional:
+            return None
+        raise KernelError("attn_entries_tcgen05: bf16, and a shape and a scale that attn_entries_supported names")
+    scratch = None
     if workspace is not None:
-        # as for attn_prefill_tcgen05: a grid that is cut has at most one block per SM after the cut
-        scratch = workspace.flat(f"attn_entries_pieces_{vdim}", PREFILL_SMS * 2 * (vdim + 2) * 128, f32)
-        counts = workspace.flat("attn_prefill_piece_counts", PREFILL_SMS, torch.int32)
-    if pieces > 1 and (scratch is None or counts.numel() < num_tiles * G):
-        raise KernelError("attn_entries_tcgen05: pieces need a workspace and at most as many query blocks as there are SMs")
-    num_pages = pages.numel() // (planes * G * page_size * (dim if shared else dim + vdim))
-
-    def at(t):
-        return t.data_ptr() if t is not None else None
-    _check(_attn_entries_lib().cvb_attn_entries_tcgen05(
-        out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), pages.data_ptr(), block_tables.data_ptr(), block_tables.shape[1],
-        cu_seqlens.data_ptr(), positions.data_ptr(), len(q_lens), num_tiles, H, G, dim, vdim, 1 if shared else 0, page_size, planes, num_pages, chunk,
-        window, pool, keep_first, scale, softcap, at(bias), bias.shape[1] if bias is not None else 0, at(r1), at(r2), table_len, at(sink), at(gate),
-        gate.stride(0) if gate is not None else 0, 1 if gate is not None and gate.shape[1] != H else 0, out_scale, pieces,
-        min_rounds or PREFILL_MIN_ROUNDS, at(scratch), scratch.numel() if scratch is not None else 0, at(counts),
-        error_flag(q.device).data_ptr(), _stream()), "attn_entries_tcgen05", kernels=2 if pieces > 1 else 1)
+        # As for attn_prefill_tcgen05: a grid that is cut has at most one block per SM after the cut.  Made at the layer's first step with a portion,
+        # whether it stays here or not: a graph that is captured later is captured for the longest context and finds it.
+        scratch = workspace.entry_pieces.get(vdim) or _entry_pieces(workspace, vdim)
+    num_tiles = prefill_tiles_tcgen05(q_lens, num_heads, num_kv_heads, skip_single=False)
+    if optional and (visible < ENTRIES_MIN_VISIBLE or num_tiles > 65535):
+        return None
+    # written out: as a loop over eleven pairs the checks took as long as the launch
+    if (out.dtype is not bf or pages.dtype is not bf or block_tables.dtype is not i32 or cu_seqlens.dtype is not i32 or positions.dtype is not i32
+            or not (out.is_cuda and q.is_cuda and pages.is_cuda and block_tables.is_cuda and cu_seqlens.is_cuda and positions.is_cuda)
+            or not (pages.is_contiguous() and block_tables.is_contiguous() and cu_seqlens.is_contiguous() and positions.is_contiguous())):
+        raise KernelError("attn_entries_tcgen05: CUDA tensors; queries, pages and output bf16, tables and positions int32; all but queries and output "
+                          "contiguous")
+    width, q_stride, out_stride = block_tables.shape, q.stride(), out.stride()
+    if (len(width) != 2 or len(q_stride) != 2 or q.shape[1] < num_heads * dim or q_stride[1] != 1 or len(out_stride) != 2
+            or out.shape[1] != num_heads * vdim or out_stride[1] != 1):
+        raise KernelError("attn_entries_tcgen05: block_tables [S, W], q [T, >= H * dim], out [T, H * vdim]")
+    bias_p = r1_p = r2_p = sink_p = gate_p = scratch_p = counts_p = None
+    bias_len = gate_stride = gate_element = floats = 0
+    if bias is not None:
+        bias_p, bias_len = _entries_term(bias, num_heads, 2), bias.shape[1]
+    if r1 is not None:
+        r1_p = _entries_term(r1, num_heads, 1)
+    if r2 is not None:
+        r2_p = _entries_term(r2, num_heads, 1)
+    if sink is not None:
+        sink_p = _entries_term(sink, num_heads, 1)
+    if gate is not None:
+        cols = gate.shape[1]
+        if gate.dtype is not bf or not gate.is_cuda or gate.stride(1) != 1 or (cols != num_heads and cols != num_heads * vdim):
+            raise KernelError("attn_entries_tcgen05: gate bf16 [T, H] or [T, H * vdim] on the GPU")
+        gate_p, gate_stride, gate_element = gate.data_ptr(), gate.stride(0), 0 if cols == num_heads else 1
+    pieces = pieces or prefill_pieces_tcgen05(num_tiles, num_kv_heads, visible)
+    if pieces > 1:
+        if scratch is None or scratch[1].numel() < num_tiles * num_kv_heads:
+            raise KernelError("attn_entries_tcgen05: pieces need a workspace and at most as many query blocks as there are SMs")
+        scratch_p, counts_p, floats = scratch[0].data_ptr(), scratch[1].data_ptr(), scratch[0].numel()
+    num_pages = pages.numel() // (planes * num_kv_heads * page_size * (dim if shared else dim + vdim))
+    status = _attn_entries_lib().cvb_attn_entries_tcgen05(
+        shape[1], out.data_ptr(), out_stride[0], q.data_ptr(), q_stride[0], pages.data_ptr(), num_pages, block_tables.data_ptr(), width[1],
+        cu_seqlens.data_ptr(), positions.data_ptr(), len(q_lens), num_tiles, bias_p, r1_p, r2_p, sink_p, gate_p, bias_len, gate_stride, gate_element,
+        pieces, min_rounds or PREFILL_MIN_ROUNDS, scratch_p, floats, counts_p, error_flag(q.device).data_ptr(), _stream())
+    if status == -3 and optional:                # rows that start off 16 bytes: the mma.sync kernels ask for less
+        return None
+    _check(status, "attn_entries_tcgen05", kernels=2 if pieces > 1 else 1)
     return out
+
+
+def _entries_term(t: torch.Tensor, num_heads: int, dims: int) -> int:
+    shape = t.shape
+    if t.dtype is not torch.float32 or not t.is_cuda or not t.is_contiguous() or len(shape) != dims or shape[0] != num_heads:
+        raise KernelError("attn_entries_tcgen05: contiguous float32 terms on the GPU: r1, r2 and sink [H], bias [H, L]")
+    return t.data_ptr()
+
+
+def _entry_pieces(workspace, vdim: int):
+    pair = (workspace.flat(f"attn_entries_pieces_{vdim}", PREFILL_SMS * 2 * (vdim + 2) * 128, torch.float32),
+            workspace.flat("attn_prefill_piece_counts", PREFILL_SMS, torch.int32))
+    workspace.entry_pieces[vdim] = pair
+    return pair
 
 
 # ---- attention over keys that are also the values ------------------------------------------------------------------

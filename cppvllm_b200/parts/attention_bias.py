@@ -111,9 +111,9 @@ class BiasedAttention(Mixer):
             q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             single = ctx.all_decode and ctx.num_tokens == ctx.num_seqs
             table = self.bias_table.shape[1]
-            if not single and ops.attn_entries_supported(q, att, None, H, G, dk, dv, g.page_size, ctx.max_kv_len, table_len=table, scale=self.scale):
-                ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv, g.page_size,
-                                         self.scale, ctx.max_kv_len, workspace=self.rt.workspace, bias=self.bias_table, table_len=table)
+            if not single and ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv,
+                                                       g.page_size, self.scale, ctx.max_kv_len, workspace=self.rt.workspace, bias=self.bias_table,
+                                                       table_len=table, optional=True) is not None:
                 return
             splits, scratch = 1, None
             if single:

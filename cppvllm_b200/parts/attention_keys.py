@@ -84,9 +84,9 @@ class KeysAttention(Mixer):
             q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             single = ctx.all_decode and ctx.num_tokens == ctx.num_seqs
             visible = min(ctx.max_kv_len, self.window + self.keep_first) if self.window > 0 else ctx.max_kv_len
-            if not single and ops.attn_entries_supported(qk, att, None, H, KV, hd, hd, g.page_size, visible, shared=True, scale=self.scale):
-                ops.attn_entries_tcgen05(att, qk, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, KV, hd, hd, g.page_size,
-                                         self.scale, visible, workspace=self.rt.workspace, shared=True, window=self.window, keep_first=self.keep_first)
+            if not single and ops.attn_entries_tcgen05(att, qk, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, KV, hd, hd,
+                                                       g.page_size, self.scale, visible, workspace=self.rt.workspace, shared=True, window=self.window,
+                                                       keep_first=self.keep_first, optional=True) is not None:
                 return
             splits, scratch = 1, None
             if single:

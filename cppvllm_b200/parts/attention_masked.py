@@ -163,17 +163,14 @@ class MaskedAttention(Mixer):
         # distances that the mask lets through, for the tcgen05 kernel's table; without a bound the term goes to the other kernels
         # (kept first tokens are seen from any distance)
         reach = min([n for n in (self.chunk, self.window) if n], default=0) if self.r1 is not None and not self.keep_first else 0
+        q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
         if (not self.force_general and not (ctx.all_decode and ctx.num_tokens == ctx.num_seqs) and (self.r1 is None or reach)
-                and ops.attn_entries_supported(q, att, gate, H, G, dk, dv, g.page_size, self._visible(ctx), table_len=reach, scale=self.scale,
-                                               softcap=self.softcap)):
-            q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
-            ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv, g.page_size,
-                                     self.scale, self._visible(ctx), workspace=self.rt.workspace, planes=self.planes, chunk=self.chunk,
-                                     window=self.window, pool=self.pool, keep_first=self.keep_first, softcap=self.softcap, r1=self.r1, r2=self.r2,
-                                     table_len=reach, sink=self.sinks, gate=gate, out_scale=out_scale)
+                and ops.attn_entries_tcgen05(att, q, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, G, dk, dv, g.page_size,
+                                             self.scale, self._visible(ctx), workspace=self.rt.workspace, planes=self.planes, chunk=self.chunk,
+                                             window=self.window, pool=self.pool, keep_first=self.keep_first, softcap=self.softcap, r1=self.r1, r2=self.r2,
+                                             table_len=reach, sink=self.sinks, gate=gate, out_scale=out_scale, optional=True) is not None):
             return
         if not self.force_general and ops.attn_masked_supported(q.dtype, H, G, dk, dv) and ops.attn_masked_pairs(att, gate, H):
-            q_lens = ctx.q_lens if ctx.q_lens is not None else [1] * ctx.num_seqs
             single = ctx.all_decode and ctx.num_tokens == ctx.num_seqs and H // G <= 16
             splits, scratch = 1, None
             if single:

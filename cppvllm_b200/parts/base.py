@@ -127,6 +127,7 @@ class Workspace:
         self.max_seqs = max_seqs or max_tokens
         self._buffers: Dict[str, torch.Tensor] = {}
         self._views: Dict[tuple, torch.Tensor] = {}
+        self.entry_pieces: Dict[int, tuple] = {}      # ops.attn_entries_tcgen05: scratch of its pieces, by value width
 
     def rows(self, name: str, n_rows: int, width, dtype: torch.dtype) -> torch.Tensor:
         hit = self._views.get((name, n_rows, width, dtype))       # the same view object for the same request

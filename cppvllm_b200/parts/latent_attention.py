@@ -164,9 +164,9 @@ class LatentAttention(Mixer):
                                    ctx.num_seqs, H, groups, HD, g.page_size, self.scale, all_single=True, splits=splits,
                                    scratch=scratch, value_dim=R, kv_heads_in_pages=1, sink=self.sinks, out_scale=out_scale)
                 return
-            if ops.attn_entries_supported(q_att, o_lat, None, H, 1, HD, R, g.page_size, ctx.max_kv_len, shared=True, scale=self.scale):
-                ops.attn_entries_tcgen05(o_lat, q_att, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, 1, HD, R, g.page_size,
-                                         self.scale, ctx.max_kv_len, workspace=self.rt.workspace, shared=True, sink=self.sinks, out_scale=out_scale)
+            if ops.attn_entries_tcgen05(o_lat, q_att, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, q_lens, H, 1, HD, R, g.page_size,
+                                        self.scale, ctx.max_kv_len, workspace=self.rt.workspace, shared=True, sink=self.sinks, out_scale=out_scale,
+                                        optional=True) is not None:
                 return
             ops.attn_keys_bf16(o_lat, q_att, cache.pages, g.block_tables, ctx.cu_seqlens, ctx.positions, ctx.num_seqs,
                                ops.attn_keys_tiles(q_lens, H, 1), H, 1, HD, g.page_size, self.scale, value_dim=R,

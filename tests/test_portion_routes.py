@@ -113,8 +113,10 @@ def both(monkeypatch, entry, kind, steps=MIXED, dtype=torch.bfloat16, longest=60
     calls, real = [], getattr(ops, entry)
 
     def counted(*a, **k):
-        calls.append(1)
-        return real(*a, **k)
+        r = real(*a, **k)
+        if r is not None:                # an answer of None: left to the other kernels
+            calls.append(1)
+        return r
     monkeypatch.setattr(ops, entry, counted)
     names = sorted({r for s in steps for r, _ in s})
     fast, plain = (Steps(layer(kind, dtype=dtype, plain=p, **over), names, longest) for p in (False, True))
@@ -160,3 +162,27 @@ def test_kept_first_tokens_with_a_distance_term(monkeypatch):
     """They are seen from beyond the chunk and the window: no table of distances is long enough, and the step stays with the other kernels."""
     diffs = both(monkeypatch, "attn_masked_bf16", "masked_attention", chunk=150, window=140, keep_first=20, distance_bias=True)
     assert max(diffs) < BF16, diffs
+
+
+def test_an_optional_call_leaves_what_the_rule_refuses():
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.parts.base import Workspace
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    i32 = lambda v: torch.as_tensor(v, dtype=torch.int32).to(dev)                                # noqa: E731
+
+    def ask(q=None, out=None, dim=128, q_lens=(8,), visible=500, heads=4, kv_heads=2, ws=None, **kw):
+        q = torch.zeros(8, heads * dim, dtype=bf, device=dev) if q is None else q
+        out = torch.zeros(8, heads * dim, dtype=bf, device=dev) if out is None else out
+        pages = torch.zeros(2, 1, kv_heads, PAGE, 2 * dim, dtype=bf, device=dev)
+        return ops.attn_entries_tcgen05(out, q, pages, i32([[0, 1]]), i32([0, 8]), i32(range(8)), list(q_lens), heads, kv_heads, dim, dim, PAGE, 0.1, visible,
+                                        ws, optional=True, **kw)
+    wide = torch.zeros(8, 4 * 128 + 4, dtype=bf, device=dev)
+    assert ask() is not None
+    for refused in (dict(visible=100), dict(dim=80), dict(q=wide[:, 4:]), dict(out=wide[:, 4:]), dict(gate=wide[:, 4:]), dict(q_lens=[131074], heads=128, kv_heads=1),
+                    dict(table_len=20000, r1=torch.ones(4, device=dev), r2=torch.ones(4, device=dev))):
+        before = ops.launches()
+        assert ask(**refused) is None and ops.launches() == before
+    ws = Workspace(dev, 64, 4)
+    assert ask(visible=100, ws=ws) is None and 128 in ws.entry_pieces       # a graph captured later, for the longest context, finds its scratch
+    torch.cuda.synchronize()
+    ops.check_device_errors(dev)
