@@ -1951,14 +1951,21 @@ def _attn_f32_lib():
 
 
 def attn_prefill_f32_supported(dtype: torch.dtype, num_heads: int, num_kv_heads: int, head_dim: int, q_lens) -> bool:
-    """Whether a step's tokens go through the tiled float32 kernel (csrc/attention_f32.cu): heads of 64 or 128, at most 64 query heads per kv head, and
-    a portion of F32_TILE_MIN_TOKENS or more (a block works through 64 rows whatever it has; single tokens stay with the general kernel)."""
-    return (dtype == torch.float32 and head_dim in (64, 128) and num_heads % num_kv_heads == 0 and num_heads // num_kv_heads <= 64
-            and max(q_lens) >= F32_TILE_MIN_TOKENS)
+    """Whether a step's tokens go through the tiled float32 kernel (csrc/attention_f32.cu): heads of 64 or 128, at most 64 query heads per kv head, a
+    portion of F32_TILE_MIN_TOKENS or more (a block works through 64 rows whatever it has), no more requests with fewer tokens than such portions
+    have tokens, and at most 65,535 blocks of rows."""
+    if not (dtype == torch.float32 and head_dim in (64, 128) and num_heads % num_kv_heads == 0 and num_heads // num_kv_heads <= 64
+            and max(q_lens) >= F32_TILE_MIN_TOKENS):
+        return False
+    long = [n for n in q_lens if n >= F32_TILE_MIN_TOKENS]
+    per = 64 // (num_heads // num_kv_heads)
+    return len(q_lens) - len(long) <= sum(long) and (sum(q_lens) <= 65535 or sum((n + per - 1) // per for n in q_lens) <= 65535)
 
 
 # Measured, a layer at 16/8 heads of 128, tiled against general, us: 64 tokens of a new prompt 78 / 88, 64 behind 400 145 / 300, 16 behind 1,000 206 /
 # 245; but 16 of a new prompt 57 / 52, 8 behind 1,000 205 / 178: a tile costs the same for one row as for 64.
+# Steps of both kinds: 64 tokens of a new prompt beside 8, 64 and 240 decoded tokens behind 300 others 127 / 173, 314 / 339, 897 / 816, behind 3,000 others
+# 564 / 903, 1,985 / 2,336, 6,319 / 6,387; 64 tokens behind 400 or 512 of a new prompt beside the 240: 970 / 1,062 and 1,063 / 1,950.
 F32_TILE_MIN_TOKENS = 32
 
 

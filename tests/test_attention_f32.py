@@ -80,3 +80,11 @@ def test_a_bad_token_reaches_no_token_that_does_not_see_it(window, plane, bad):
     assert torch.equal(got[~sees], clean[~sees])
     if plane == 1:
         assert not torch.isfinite(got[sees]).any()
+
+
+def test_steps_of_portions_and_single_tokens():
+    from cppvllm_b200.csrc import ops
+    ok = ops.attn_prefill_f32_supported
+    assert ok(torch.float32, 16, 8, 128, [64] + [1] * 64) and not ok(torch.float32, 16, 8, 128, [64] + [1] * 65)
+    assert ok(torch.float32, 16, 8, 128, [31] * 33 + [33]) and not ok(torch.float32, 16, 8, 128, [31] * 34 + [33])
+    assert ok(torch.float32, 64, 1, 64, [65535]) and not ok(torch.float32, 64, 1, 64, [65536])            # a block holds one token of 64 heads
