@@ -381,8 +381,22 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
 #pragma unroll
                 for (int c = 0; c < 4; ++c) tm_load32(my_s + lane_base + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[c * 32]));
                 tm_wait_ld();
+                const int hi = pooled ? row_nb - 1 : row_pos;
+                auto mask = [&](uint32_t with) {
+                    if (key0 + 127 > hi) {                                     // entries after the row's own
+                        const int n_see = hi - key0 + 1;
+#pragma unroll
+                        for (int c = 0; c < 128; ++c) v[c] = c < n_see ? v[c] : with;
+                    }
+                    if (!pooled && key0 < row_lo) {                            // entries before the row's window, but for the kept ones
+                        const int n_drop = row_lo - key0, n_keep = keep - key0;
+#pragma unroll
+                        for (int c = 0; c < 128; ++c) v[c] = (c < n_drop && c >= n_keep) ? with : v[c];
+                    }
+                };
                 if (TERMS) {
                     if (p.softcap > 0.f) {
+                        mask(0u);               // what a former holder left in a page must not choose between the two forms below
                         const float k = p.scale / p.softcap, back = p.softcap * kELog2e;
                         float top = 0.f;
 #pragma unroll
@@ -421,17 +435,7 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                         }
                     }
                 }
-                const int hi = pooled ? row_nb - 1 : row_pos;
-                if (key0 + 127 > hi) {                                         // entries after the row's own: -inf
-                    const int n_see = hi - key0 + 1;
-#pragma unroll
-                    for (int c = 0; c < 128; ++c) v[c] = c < n_see ? v[c] : 0xff800000u;
-                }
-                if (!pooled && key0 < row_lo) {                                // entries before the row's window, but for the kept ones
-                    const int n_drop = row_lo - key0, n_keep = keep - key0;
-#pragma unroll
-                    for (int c = 0; c < 128; ++c) v[c] = (c < n_drop && c >= n_keep) ? 0xff800000u : v[c];
-                }
+                mask(0xff800000u);                                             // -inf
                 float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};       // four chains of three-input maxima
 #pragma unroll
                 for (int c = 0; c < 128; c += 8) {

@@ -224,3 +224,14 @@ def test_a_nan_is_answered_with_nan(shared, pieces):
     want[:, 2:] = True
     want[5, 0] = True
     assert torch.equal(torch.isnan(out).all(-1), want) and not torch.isnan(out[~want]).any()
+
+
+@pytest.mark.gpu
+def test_a_cap_does_not_depend_on_what_unused_slots_hold():
+    H, G, dim, n, cached = 4, 2, 128, 300, 77
+    q, pages = one_request(H, G, dim, False, n, cached)
+    outs = []
+    for factor in (0.01, 3000.0):
+        pages[-1, :, :, (n + cached) % 32:] *= factor
+        outs.append(run_one(q, pages, H, G, dim, False, n, cached, softcap=30.0, chunk=200))
+    assert torch.equal(*outs)
