@@ -782,7 +782,23 @@ def _delta_lib():
 
 
 DELTA_CHUNK = 32              # tokens
-DELTA_CHUNKS_HELD = 96        # chunks whose images the scratch holds (170 MB at 32 heads of 128 x 128); longer steps go through it in turns
+DELTA_CHUNKS_HELD = 96        # chunks whose images the scratch holds at most (170 MB at 32 heads of 128 x 128); longer steps go through it in turns
+
+
+def delta_chunks_held(workspace) -> int:
+    """Chunks whose images the scratch holds: those of the largest step (its requests' last chunks are not full), within DELTA_CHUNKS_HELD."""
+    return min(DELTA_CHUNKS_HELD, workspace.max_tokens // DELTA_CHUNK + min(workspace.max_seqs, workspace.max_tokens))
+
+
+def delta_chunks_scratch(workspace, num_heads: int, num_kv_heads: int, vdim: int):
+    """Name and bytes of the scratch that delta_chunks takes from the workspace."""
+    return (f"delta_chunks_{num_heads}_{num_kv_heads}_{vdim}",
+            int(_delta_lib().cvb_delta_chunks_scratch(delta_chunks_held(workspace), num_heads, num_kv_heads, vdim)))
+
+
+def delta_chunks_shape(dtype: torch.dtype, taps: int, dim: int, vdim: int) -> bool:
+    """Whether the chunk kernels take a layer at all."""
+    return dtype == torch.bfloat16 and dim == 128 and vdim in (64, 128) and 1 <= taps <= 4
 
 
 def delta_chunks_supported(packed: torch.Tensor, qkv_off: int, taps: int, num_heads: int, num_kv_heads: int, dim: int, vdim: int, state: torch.Tensor,
@@ -793,7 +809,7 @@ def delta_chunks_supported(packed: torch.Tensor, qkv_off: int, taps: int, num_he
     further pair of them before the first token is done.  Measured, a layer, chunks against scan, us: 16/8 heads 64 tokens 46 / 47, 128 tokens 49 /
     69, 33 tokens 45 / 39; 32/8 heads 128 tokens 100 / 105, 64 tokens 94 / 79."""
     least = 24 + 40 * ((num_heads // num_kv_heads + 1) // 2)
-    return (packed.dtype == torch.bfloat16 and dim == 128 and vdim in (64, 128) and 1 <= taps <= 4 and state.shape[1] % 2 == 0
+    return (delta_chunks_shape(packed.dtype, taps, dim, vdim) and state.shape[1] % 2 == 0
             and packed.stride(0) % 2 == 0 and qkv_off % 2 == 0 and packed.data_ptr() % 4 == 0 and max(q_lens) >= least)
 
 
@@ -811,11 +827,12 @@ def delta_chunks(out, packed, qkv_off: int, conv_w, ba, dt_bias, a_log, state: t
         raise KernelError("delta_chunks: out [T, H * vdim], ba [T, 2 H], dt_bias, a_log [H], conv_w [channels, taps], state [slots, floats]")
     lib = _delta_lib()
     total = sum((n + DELTA_CHUNK - 1) // DELTA_CHUNK for n in q_lens)
-    scratch = workspace.flat(f"delta_chunks_{H}_{G}_{vdim}", lib.cvb_delta_chunks_scratch(DELTA_CHUNKS_HELD, H, G, vdim), torch.uint8)
+    held = delta_chunks_held(workspace)
+    scratch = workspace.flat(*delta_chunks_scratch(workspace, H, G, vdim), torch.uint8)
     _check(lib.cvb_delta_chunks(out.data_ptr(), packed.data_ptr(), packed.stride(0), qkv_off, conv_w.data_ptr(), conv_w.shape[1], ba.data_ptr(),
                                 dt_bias.data_ptr(), a_log.data_ptr(), state.data_ptr(), state.shape[1], conv_off, cu_seqlens.data_ptr(),
                                 state_slots.data_ptr(), state.shape[0], len(q_lens), total, H, G, dim, vdim, scratch.data_ptr(), scratch.numel(),
-                                error_flag(out.device).data_ptr(), _stream()), "delta_chunks", kernels=2 * -(-total // DELTA_CHUNKS_HELD))
+                                error_flag(out.device).data_ptr(), _stream()), "delta_chunks", kernels=2 * -(-total // held))
     return out
 
 

@@ -174,7 +174,10 @@ class ModelRunner:
         used = total_b - free_b
         cfg = self.model
         act_reserve = self.max_step_tokens * (16 * cfg.hidden_size) * 4 + self.max_seqs * cfg.vocab_size * 4 * 2 + (1 << 30)
-        budget = total_b * utilization - used - act_reserve - getattr(self, "_state_bytes", 0)
+        scratch: Dict[str, int] = {}
+        for b in cfg.blocks:
+            scratch.update(b.mixer.scratch_bytes())
+        budget = total_b * utilization - used - act_reserve - getattr(self, "_state_bytes", 0) - sum(scratch.values())
         per_page = sum(self.page_bytes) or 1
         n = int(budget // per_page)
         if n <= 0:

@@ -208,6 +208,11 @@ class Part:
         """Bytes of weights a decode step reads from this part (for the roofline)."""
         return 0
 
+    def scratch_bytes(self) -> Dict[str, int]:
+        """Large scratch buffers that the part takes from the workspace, beside rows of activations: bytes by name (layers of one shape share
+        them).  The cache's pages leave room for them."""
+        return {}
+
 
 class Norm(Part):
     category = "norm"

@@ -201,6 +201,11 @@ class HeadDeltaMixer(Mixer):
     def weight_bytes(self) -> int:
         return sum(w.numel() * w.element_size() for w in (self.w_in, self.w_b, self.w_a, self.w_o))
 
+    def scratch_bytes(self) -> Dict[str, int]:
+        if self.rt.plain_kernels or not ops.delta_chunks_shape(self.rt.dtype, self.taps, self.dim, self.vdim):
+            return {}
+        return dict([ops.delta_chunks_scratch(self.rt.workspace, self.num_heads, self.num_kv_heads, self.vdim)])
+
     def forward(self, x, ctx, cache, state):
         T, S = x.shape[0], ctx.num_seqs
         H, G, dk, dv = self.num_heads, self.num_kv_heads, self.dim, self.vdim

@@ -135,6 +135,26 @@ def both(monkeypatch, entry, kind, steps=MIXED, dtype=torch.bfloat16, longest=60
 BF16 = 2e-2
 
 
+ROUTES = [("attn_entries_tcgen05", "masked_attention", dict(chunk=150, element_gate=True, qkv_bias=True)),
+          ("attn_entries_tcgen05", "masked_attention", dict(chunk=200, softcap=5.0, distance_bias=True, sink=True, head_gate=True)),
+          ("attn_entries_tcgen05", "masked_attention", dict(window=140, distance_bias=True, dim=64)),
+          ("attn_entries_tcgen05", "masked_attention", dict(window=140, pool=16, heads=8)),
+          ("attn_entries_tcgen05", "masked_attention", dict(window=140, keep_first=5, softcap=3.0, qk_norm=False)),
+          ("attn_entries_tcgen05", "keys_attention", {}), ("attn_entries_tcgen05", "keys_attention", dict(window=140, keep_first=200, heads=6)),
+          ("attn_entries_tcgen05", "latent_attention", dict(gate="element", q_rank=48)),
+          ("attn_entries_tcgen05", "latent_attention", dict(gate="none", sink=True, heads=20)),
+          ("attn_entries_tcgen05", "biased_attention", {}), ("attn_entries_tcgen05", "biased_attention", dict(dim=64, kv_heads=1)),
+          ("delta_chunks", "head_delta", {}), ("delta_chunks", "head_delta", dict(dim=64, heads=3, kv_heads=1)),
+          ("attn_prefill_f32", "paged_attention", {}), ("attn_prefill_f32", "paged_attention", dict(window=50, dim=64))]
+
+
+@pytest.mark.parametrize("entry,kind,over", ROUTES)
+def test_prompts_in_portions_beside_decoded_tokens(monkeypatch, entry, kind, over):
+    exact = entry == "attn_prefill_f32"
+    diffs = both(monkeypatch, entry, kind, dtype=torch.float32 if exact else torch.bfloat16, **over)
+    assert max(diffs) < (1e-5 if exact else BF16), diffs
+
+
 @pytest.mark.parametrize("scale", [0.0, -0.08])
 @pytest.mark.parametrize("kind,over", [("keys_attention", {}), ("keys_attention", dict(window=100)), ("latent_attention", dict(sink=True)),
                                        ("masked_attention", dict(chunk=256)), ("masked_attention", dict(chunk=256, softcap=5.0)), ("biased_attention", {})])
@@ -186,3 +206,27 @@ def test_an_optional_call_leaves_what_the_rule_refuses():
     assert ask(visible=100, ws=ws) is None and 128 in ws.entry_pieces       # a graph captured later, for the longest context, finds its scratch
     torch.cuda.synchronize()
     ops.check_device_errors(dev)
+
+
+def test_scratch_of_the_delta_rule_follows_the_largest_step_and_is_left_free():
+    """What a step takes is what the part names, chunks for the largest step and no more; the pages' budget leaves it out."""
+    from types import SimpleNamespace
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.engine.runner import ModelRunner
+    part = layer("head_delta", max_tokens=128, max_seqs=4)
+    (name, size), = part.scratch_bytes().items()
+    assert ops.delta_chunks_held(part.rt.workspace) == 128 // 32 + 4 and size == ops._delta_lib().cvb_delta_chunks_scratch(8, 4, 2, 128)
+    run = Steps(part, ["a"], 128)
+    run(torch.zeros(128, WIDTH, dtype=torch.bfloat16, device="cuda:0"), [("a", 128)])
+    assert part.rt.workspace.flat(name, size, torch.uint8).numel() == size
+    big = layer("head_delta", max_tokens=8192, max_seqs=64)
+    assert ops.delta_chunks_held(big.rt.workspace) == ops.DELTA_CHUNKS_HELD
+    assert layer("head_delta", plain=True).scratch_bytes() == {} and layer("head_delta", dtype=torch.float32).scratch_bytes() == {}
+
+    def pages(*mixers):
+        model = SimpleNamespace(hidden_size=64, vocab_size=100, blocks=[SimpleNamespace(mixer=m) for m in mixers])
+        fake = SimpleNamespace(device=torch.device("cuda:0"), model=model, max_step_tokens=128, max_seqs=1 << 20, page_bytes=[1 << 16], table_width=1 << 20)
+        return ModelRunner._pages_from_free_memory(fake, 0.9)
+    other = layer("keys_attention")
+    per = sum(big.scratch_bytes().values()) / 65536
+    assert abs(pages(other) - pages(other, big, big) - per) < 0.02 * per + 64          # layers of one shape share it; other users' memory may move
