@@ -11,11 +11,14 @@
 // (request, head, slice of value columns) with S in registers, half of its warps on the chain and half on the outputs beside it.  Decays are
 // running products (never logarithms: g may be 0).
 //
-// Products run as `mma.sync.m16n8k16` with every float operand split into two bf16 (x = hi + lo, hi hi + hi lo + lo hi, float
-// accumulation): 2^-17 of an operand is lost, 1 / 64 of what the bf16 projection in front of the rule has rounded already.  W and U~ come
+// Products run as `mma.sync.m16n8k8` in tf32 with every float operand split in two when its fragment is loaded (x = hi + lo: hi the nearest tf32
+// number, lo the rest, of which the product reads 11 bits more; hi hi + hi lo + lo hi), float accumulation in several short chains that are added
+// up by the float units (the tensor core cuts a sum off instead of rounding it).  From the same projection, 64 to 2,048 tokens at 16/8 and 32/8
+// heads, the outputs are 2.7e-7 to 3.9e-7 from float64 and the states 2.4e-7 to 4.0e-7 (the float scan: 1.9e-7 to 3.7e-7, 2.2e-7 to 4.0e-7; with
+// bf16 pairs 5.3e-6 to 6.3e-6, 4.7e-6 to 4.9e-6); behind the layer's bf16 projections the two routes are equally far, 4.2e-3.  W and U~ come
 // from a float substitution, one thread per column.  Steps in float32 stay on the scan.
-// Chunk images in scratch are laid out as the chain kernel wants them in shared memory (rows padded against ldmatrix conflicts), so a
-// chunk arrives by a few bulk copies, two chunks ahead.
+// Chunk images in scratch are laid out as the chain kernel wants them in shared memory (every operand with its inner dimension running, rows
+// padded against ldmatrix conflicts), so a chunk arrives by a few bulk copies, two chunks ahead.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "mma_tiles.cuh"
@@ -24,11 +27,14 @@ namespace cvb {
 
 constexpr int kDC = 32;                                  // tokens per chunk
 constexpr int kDK = 128;                                 // key channels
-constexpr int kDLD = kDK + 8;                            // bf16 elements of a padded row of K, Q, W
-constexpr int kDLA = kDC + 8;                            // of A
-constexpr int kDRowsBytes = kDC * kDLD * 2;              // one image of K, Q or W
-constexpr int kDHeadBytes = 2 * kDRowsBytes + 2 * kDC * kDLA * 2 + 2 * kDC * 4;     // W hi, lo | A hi, lo | e | D_31
-constexpr int kDKvBytes = 4 * kDRowsBytes;               // K hi, lo | Q hi, lo
+constexpr int kDLF = kDK + 4;                            // floats of a padded row of K, Q, W, of convolved channels and of S transposed
+constexpr int kDLT = kDC + 4;                            // floats of a padded row of A and of K, U, D U transposed
+constexpr int kDRowsBytes = kDC * kDLF * 4;              // Q or W
+constexpr int kDTransBytes = kDK * kDLT * 4;             // K transposed
+constexpr int kDABytes = kDC * kDLT * 4;
+constexpr int kDVecBytes = 2 * kDC * 4;
+constexpr int kDHeadBytes = kDRowsBytes + kDABytes + kDVecBytes;                   // W | A | e | D_31
+constexpr int kDKvBytes = kDTransBytes + kDRowsBytes;    // K transposed | Q
 
 struct DeltaChunkParams {
     const __nv_bfloat16* packed;                         // rows of `stride` elements; from column qkv_off on q [G * 128], k [G * 128], v [H * dv]
@@ -63,34 +69,46 @@ __device__ __forceinline__ float* u_image(const DeltaChunkParams& p, int lc, int
     return reinterpret_cast<float*>(base) + ((static_cast<int64_t>(lc) * p.H + h) * (p.dv / NB) + cb) * (kDC * (NB + 8));
 }
 
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& lo) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    const float2 f = __bfloat1622float2(h);
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = pack2(x - f.x, y - f.y);
+// x = hi + lo: hi x rounded to tf32 (10 bits behind the first one), lo what is left, exact in float, of which the product reads its upper 11 bits.
+// (Rounding lo instead of leaving its tail to be cut off changed no error by 1 % and cost 3 % of the rule.)  A NaN stays one in lo.
+__device__ __forceinline__ void split_tf32(uint32_t x, uint32_t& hi, uint32_t& lo) {
+    hi = (x + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(__uint_as_float(x) - __uint_as_float(hi));
 }
+template <int N>
+__device__ __forceinline__ void split_tf32(const uint32_t (&x)[N], uint32_t (&hi)[N], uint32_t (&lo)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) split_tf32(x[i], hi[i], lo[i]);
+}
+// D += A B, 16 x 8 x 8.  With ldm_x4 over rows of floats a thread holds A's rows lane / 4 and + 8 at columns lane % 4 and + 4, and of B, whose
+// columns are rows in memory, column lane / 4 at inner indices lane % 4, + 4 (and + 8, + 12: the next product's).
+__device__ __forceinline__ void mma_1688(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// where a lane's rows lie for ldm_x4: of A 16 rows of 8 floats, of B 8 rows of 16
+__device__ __forceinline__ int a_lane(int lane, int ld) { return (lane & 15) * ld + (lane >> 4) * 4; }
+__device__ __forceinline__ int b_lane(int lane, int ld) { return (lane & 7) * ld + (lane >> 3) * 4; }
 
 __device__ __forceinline__ float delta_sigmoid(float z) { return 1.f / (1.f + expf(-z)); }
 
-constexpr int kDLF = kDK + 4;                            // floats of a padded row of convolved channels
 constexpr int kDPair = 2;                                // heads of a kv head worked on together
-constexpr size_t kDPrepBytes = static_cast<size_t>(kDKvBytes) + 3 * kDC * kDLF * sizeof(float) +
-                               kDPair * (kDC * 36 + kDC * 33 + 2 * kDC) * sizeof(float);
+constexpr size_t kDPrepBytes = static_cast<size_t>(4) * kDC * kDLF * sizeof(float) + kDPair * (kDC * 36 + kDC * 33 + 2 * kDC) * sizeof(float);
 
 // Grid (chunk, kv head).  From the packed projection: convolutions, silu, unit vectors, decays and input strengths as recurrent.cu's delta_prep
 // makes them, then the kv head's image and, two heads at a time, the heads' images; nothing between the projection and the images travels
 // through memory.  (With delta_prep in front, a block per (chunk, head) and the heads' float rows read back, it was 66 + 49 us for 2,048
-// tokens of 16/8 heads; now 58, bound by instruction issue: 0.41 a cycle and scheduler with two blocks an SM.)
+// tokens of 16/8 heads; now 59, bound by instruction issue with two blocks an SM.)
 template <int NB, int TAPS>
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const DeltaChunkParams p) {
     pdl_trigger();
     extern __shared__ __align__(128) unsigned char smem[];
-    __nv_bfloat16* sK = reinterpret_cast<__nv_bfloat16*>(smem);                    // hi, lo
-    __nv_bfloat16* sQ = sK + 2 * kDC * kDLD;                                       // hi, lo
-    float* sKf = reinterpret_cast<float*>(sQ + 2 * kDC * kDLD);                    // k, convolved, then of unit length
-    float* sV0 = sKf + kDC * kDLF;
-    float* sV1 = sV0 + kDC * kDLF;                                                 // the second head's v; before that, q
+    float* sK = reinterpret_cast<float*>(smem);                                    // k, convolved, then of unit length
+    float* sQ = sK + kDC * kDLF;                                                   // q, the same
+    float* sV0 = sQ + kDC * kDLF;
+    float* sV1 = sV0 + kDC * kDLF;                                                 // the second head's v
     float* sL = sV1 + kDC * kDLF;                                                  // [head of the pair] L transposed: [j][i], rows of 36
     float* sD = sL + kDPair * kDC * 36;                                            // [i][j], rows of 33
     float* sG = sD + kDPair * kDC * 33;                                            // [head][b | e][32]
@@ -177,50 +195,67 @@ delta_prepare_kernel(const DeltaChunkParams p) {
         fetch(raw_k, w_k, QK + kvh * kDK, kDK);
         fetch(raw_v, w_v, v_col, p.dv);
         if (share > 1) fetch(raw_v1, w_v1, v_col + p.dv, p.dv);
-        convolve(sV1, raw_q, w_q, kvh * kDK, kDK);
-        convolve(sKf, raw_k, w_k, QK + kvh * kDK, kDK);
+        convolve(sQ, raw_q, w_q, kvh * kDK, kDK);
+        convolve(sK, raw_k, w_k, QK + kvh * kDK, kDK);
         convolve(sV0, raw_v, w_v, v_col, p.dv);
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < kDC / 8; ++i) {                                            // unit vectors, split; a warp per row
+    for (int i = 0; i < kDC / 8; ++i) {                                            // unit vectors; a warp per row
         const int r = warp * (kDC / 8) + i;
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
-            float* row = (which ? sV1 : sKf) + r * kDLF + lane * 4;
-            float4 x = *reinterpret_cast<const float4*>(row);
+            float* row = (which ? sQ : sK) + r * kDLF + lane * 4;
+            const float4 x = *reinterpret_cast<const float4*>(row);
             const float ss = warp_sum(fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, x.w * x.w))));
             float inv = 1.f / sqrtf(ss + 1e-6f);
             if (which) inv *= 1.f / sqrtf(static_cast<float>(kDK));
-            x = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
-            if (!which) *reinterpret_cast<float4*>(row) = x;
-            uint2 hi, lo;
-            split_pair(x.x, x.y, hi.x, lo.x);
-            split_pair(x.z, x.w, hi.y, lo.y);
-            __nv_bfloat16* dst = (which ? sQ : sK) + r * kDLD + lane * 4;
-            *reinterpret_cast<uint2*>(dst) = hi;
-            *reinterpret_cast<uint2*>(dst + kDC * kDLD) = lo;
+            *reinterpret_cast<float4*>(row) = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
         }
     }
     __syncthreads();
     {                                                                              // the rows' pads are never read
-        const uint4* src = reinterpret_cast<const uint4*>(smem);
-        uint4* dst = reinterpret_cast<uint4*>(kv_image(p, lc, kvh));
-        for (int i = tid; i < kDKvBytes / 16; i += 256) dst[i] = src[i];
+        float* kt = reinterpret_cast<float*>(kv_image(p, lc, kvh));
+        const int c = tid & (kDK - 1);
+#pragma unroll
+        for (int t = (tid >> 7) * 4; t < kDC; t += 8)
+            *reinterpret_cast<float4*>(kt + c * kDLT + t) = make_float4(sK[t * kDLF + c], sK[(t + 1) * kDLF + c], sK[(t + 2) * kDLF + c], sK[(t + 3) * kDLF + c]);
+        const uint4* src = reinterpret_cast<const uint4*>(sQ);
+        uint4* dst = reinterpret_cast<uint4*>(kt + kDK * kDLT);
+        for (int i = tid; i < kDRowsBytes / 16; i += 256) dst[i] = src[i];
     }
     // K K^T and Q K^T, one tile of 16 x 8 of either per warp, the same for all heads of the group
     const int m = (warp & 1) * 16, nn = (warp >> 1) * 8;
-    float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
+    float kk[4], qk[4];
+    {
+        float ck[4][4], cq[4][4], xk[4] = {0.f, 0.f, 0.f, 0.f}, xq[4] = {0.f, 0.f, 0.f, 0.f};     // hi hi in four chains; the cross terms
 #pragma unroll
-    for (int k = 0; k < kDK / 16; ++k) {
-        const int ao = (m + (lane & 15)) * kDLD + k * 16 + (lane >> 4) * 8;
-        uint32_t kh[4], kl[4], qh[4], ql[4], b[4];
-        ldm_x4(kh, sK + ao); ldm_x4(kl, sK + kDC * kDLD + ao);
-        ldm_x4(qh, sQ + ao); ldm_x4(ql, sQ + kDC * kDLD + ao);
-        // b[0], b[1]: hi, columns k * 16 and k * 16 + 8 of the eight rows; b[2], b[3]: lo
-        ldm_x4(b, sK + (lane >> 4) * kDC * kDLD + (nn + (lane & 7)) * kDLD + k * 16 + ((lane >> 3) & 1) * 8);
-        mma_16816(kk, kh, b[0], b[1]); mma_16816(kk, kh, b[2], b[3]); mma_16816(kk, kl, b[0], b[1]);
-        mma_16816(qk, qh, b[0], b[1]); mma_16816(qk, qh, b[2], b[3]); mma_16816(qk, ql, b[0], b[1]);
+        for (int i = 0; i < 16; ++i) ck[i >> 2][i & 3] = cq[i >> 2][i & 3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < kDK / 16; ++k) {
+            uint32_t b[4], bh[4], bl[4];
+            ldm_x4(b, sK + nn * kDLF + k * 16 + b_lane(lane, kDLF));
+            split_tf32(b, bh, bl);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t a[4], ah[4], al[4];
+                ldm_x4(a, sK + m * kDLF + k * 16 + e * 8 + a_lane(lane, kDLF));
+                split_tf32(a, ah, al);
+                mma_1688(ck[k >> 1], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(xk, ah, bl[2 * e], bl[2 * e + 1]);
+                mma_1688(xk, al, bh[2 * e], bh[2 * e + 1]);
+                ldm_x4(a, sQ + m * kDLF + k * 16 + e * 8 + a_lane(lane, kDLF));
+                split_tf32(a, ah, al);
+                mma_1688(cq[k >> 1], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(xq, ah, bl[2 * e], bl[2 * e + 1]);
+                mma_1688(xq, al, bh[2 * e], bh[2 * e + 1]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            kk[i] = ((ck[0][i] + ck[1][i]) + (ck[2][i] + ck[3][i])) + xk[i];
+            qk[i] = ((cq[0][i] + cq[1][i]) + (cq[2][i] + cq[3][i])) + xq[i];
+        }
     }
     for (int h0 = 0; h0 < share; h0 += kDPair) {
         const int heads = min(kDPair, share - h0), hbase = kvh * share + h0;
@@ -232,7 +267,7 @@ delta_prepare_kernel(const DeltaChunkParams p) {
             if (heads > 1) fetch(raw_v1, w_v1, c0 + p.dv, p.dv);
             convolve(sV0, raw, w, c0, p.dv);
         }
-        if (heads > 1) convolve(sV1, raw_v1, w_v1, c0 + p.dv, p.dv);               // q has become its image
+        if (heads > 1) convolve(sV1, raw_v1, w_v1, c0 + p.dv, p.dv);
         if (warp < heads) {                                                        // a head per warp, a token per lane
             const int h = hbase + warp;
             float g = 1.f, be = 0.f;
@@ -258,7 +293,7 @@ delta_prepare_kernel(const DeltaChunkParams p) {
         __syncthreads();
         for (int x = 0; x < heads; ++x) {
             unsigned char* img = head_image(p, lc, hbase + x);
-            __nv_bfloat16* a_img = reinterpret_cast<__nv_bfloat16*>(img + 2 * kDRowsBytes);
+            float* a_img = reinterpret_cast<float*>(img + kDRowsBytes);
             const float* D = sD + x * kDC * 33;
             const float* G = sG + x * 2 * kDC;
             float* Lt = sL + x * kDC * 36;
@@ -267,13 +302,11 @@ delta_prepare_kernel(const DeltaChunkParams p) {
                 const int i = m + (lane >> 2) + half * 8, j = nn + (lane & 3) * 2;
                 Lt[j * 36 + i] = j < i ? G[i] * D[i * 33 + j] * kk[half * 2] : 0.f;
                 Lt[(j + 1) * 36 + i] = j + 1 < i ? G[i] * D[i * 33 + j + 1] * kk[half * 2 + 1] : 0.f;
-                uint32_t hi, lo;
-                split_pair(j <= i ? D[i * 33 + j] * qk[half * 2] : 0.f, j + 1 <= i ? D[i * 33 + j + 1] * qk[half * 2 + 1] : 0.f, hi, lo);
-                *reinterpret_cast<uint32_t*>(a_img + i * kDLA + j) = hi;
-                *reinterpret_cast<uint32_t*>(a_img + kDC * kDLA + i * kDLA + j) = lo;
+                *reinterpret_cast<float2*>(a_img + i * kDLT + j) = make_float2(j <= i ? D[i * 33 + j] * qk[half * 2] : 0.f,
+                                                                               j + 1 <= i ? D[i * 33 + j + 1] * qk[half * 2 + 1] : 0.f);
             }
             if (tid < kDC) {
-                float* v = reinterpret_cast<float*>(img + 2 * kDRowsBytes + 2 * kDC * kDLA * 2);
+                float* v = reinterpret_cast<float*>(img + kDRowsBytes + kDABytes);
                 v[tid] = G[kDC + tid];
                 v[kDC + tid] = D[(kDC - 1) * 33 + tid];
             }
@@ -286,7 +319,7 @@ delta_prepare_kernel(const DeltaChunkParams p) {
             if (!is_w && col >= p.dv) continue;
             const float* Lt = sL + x2 * kDC * 36;
             const float* G = sG + x2 * 2 * kDC;
-            const float* rhs = (is_w ? sKf : (x2 ? sV1 : sV0)) + col;
+            const float* rhs = (is_w ? sK : (x2 ? sV1 : sV0)) + col;
             float x[kDC];
 #pragma unroll
             for (int i = 0; i < kDC; ++i) x[i] = rhs[i * kDLF] * (is_w ? G[i] * G[kDC + i] : G[i]);
@@ -301,15 +334,10 @@ delta_prepare_kernel(const DeltaChunkParams p) {
                     x[i4 + 3] = fmaf(-l.w, x[j], x[i4 + 3]);
                 }
             }
-            if (is_w) {                                                            // of two neighbouring columns one thread stores hi, the other lo
-                __nv_bfloat16* w = reinterpret_cast<__nv_bfloat16*>(head_image(p, lc, hbase + x2)) + (col & 1) * kDC * kDLD + (col & ~1);
+            if (is_w) {
+                float* w = reinterpret_cast<float*>(head_image(p, lc, hbase + x2)) + col;
 #pragma unroll
-                for (int i = 0; i < kDC; ++i) {
-                    const float other = __shfl_xor_sync(0xffffffffu, x[i], 1);
-                    uint32_t hi, lo;
-                    split_pair((col & 1) ? other : x[i], (col & 1) ? x[i] : other, hi, lo);
-                    *reinterpret_cast<uint32_t*>(w + i * kDLD) = (col & 1) ? lo : hi;
-                }
+                for (int i = 0; i < kDC; ++i) w[i * kDLF] = x[i];
             } else {
                 float* u = u_image<NB>(p, lc, hbase + x2, col / NB) + col % NB;
 #pragma unroll
@@ -323,19 +351,18 @@ delta_prepare_kernel(const DeltaChunkParams p) {
 template <int NB>
 struct DeltaChainSmem {
     static constexpr int kU = kDC * (NB + 8) * 4;
-    static constexpr int kStageW = 2 * kDRowsBytes + 2 * kDRowsBytes + kU + 2 * kDC * 4;       // W hi, lo | K hi, lo | U~ | e, D_31
-    static constexpr int kStageQ = 2 * kDRowsBytes + 2 * kDC * kDLA * 2 + 2 * kDC * 4;         // Q hi, lo | A hi, lo | e, D_31
-    static constexpr int kS = 2 * kDK * (NB + 8) * 2;                              // S hi, lo
-    static constexpr int kUb = 2 * kDC * (NB + 8) * 2;                             // U hi, lo
+    static constexpr int kStageW = kDRowsBytes + kDTransBytes + kU + kDVecBytes;               // W | K transposed | U~ | e, D_31
+    static constexpr int kStageQ = kDRowsBytes + kDABytes + kDVecBytes;                        // Q | A | e, D_31
+    static constexpr int kS = NB * kDLF * 4;                                       // S transposed
+    static constexpr int kUb = NB * kDLT * 4;                                      // U transposed
     static constexpr size_t kBytes = static_cast<size_t>(2) * (kStageW + kStageQ + kS + kUb) + kUb + 4 * 8;
 };
 
 // Grid (request, head, NB value columns); NB / 2 warps in two halves.  The first half carries the chain: W S, U = U~ - W S, S = e_31 S + K^T (D_31 U),
 // with two barriers of its own a chunk.  The second half makes the outputs e Q S + A U beside it, up to a chunk behind: S and U have two
 // buffers, `ready` (U of the chunk is there, S was before) and `done` (the outputs have been made) hand them over.  Each half fetches for itself, two
-// chunks ahead.  What bounds it are the shared-memory reads of the split operands (528 ldmatrix of 512 bytes a chunk at 32 columns, 2,100
-// cycles); with all warps in step through both parts a chunk took 4,000 cycles, now
-// 3,400 (1,511 + 537 tokens, 16 heads: 96 -> 84 us); the rest is the chain's own latencies.
+// chunks ahead.  What bounds it is instruction issue: a fragment's split costs three instructions a register, six products stand where float ones would
+// be two (1,511 + 537 tokens, 16 heads: 150 us, 6,100 cycles a chunk; with bf16 pairs, split once in memory, 84).
 template <int NB>
 __global__ void __launch_bounds__(NB * 16, 1)
 delta_chain_kernel(const DeltaChunkParams p) {
@@ -345,10 +372,10 @@ delta_chain_kernel(const DeltaChunkParams p) {
     constexpr int LS = NB + 8, kHalf = NB / 4, kThreads = NB * 16;                 // warps of a half, threads of the block
     unsigned char* sStageW = smem;
     unsigned char* sStageQ = smem + 2 * L::kStageW;
-    __nv_bfloat16* sS = reinterpret_cast<__nv_bfloat16*>(sStageQ + 2 * L::kStageQ);             // two buffers of S hi, lo
-    __nv_bfloat16* sU = sS + 2 * 2 * kDK * LS;                                     // two buffers of U hi, lo
-    __nv_bfloat16* sDU = sU + 2 * 2 * kDC * LS;                                    // D_31 U hi, lo
-    uint64_t* full = reinterpret_cast<uint64_t*>(sDU + 2 * kDC * LS);              // [2] of the first half, [2] of the second
+    float* sS = reinterpret_cast<float*>(sStageQ + 2 * L::kStageQ);                // two buffers of S transposed
+    float* sU = sS + 2 * NB * kDLF;                                                // two buffers of U transposed
+    float* sDU = sU + 2 * NB * kDLT;                                               // D_31 U transposed
+    uint64_t* full = reinterpret_cast<uint64_t*>(sDU + NB * kDLT);                 // [2] of the first half, [2] of the second
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int s = blockIdx.x, h = blockIdx.y, cb = blockIdx.z, kvh = h / (p.H / p.G);
     const int slot = p.state_slots[s];
@@ -376,7 +403,6 @@ delta_chain_kernel(const DeltaChunkParams p) {
                      ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
         dst += bytes;
     };
-    constexpr int kABytes = 2 * kDC * kDLA * 2, kVecBytes = 2 * kDC * 4;
     auto fetch = [&](int c) {                                                      // one thread of a half: chunk c0 + c into the half's stage
         const int st = c & 1, lc = c0 + c - p.c_first;
         const unsigned char* head = head_image(p, lc, h);
@@ -385,45 +411,45 @@ delta_chain_kernel(const DeltaChunkParams p) {
         if (is_q) {
             unsigned char* dst = sStageQ + st * L::kStageQ;
             mbar_expect_tx(bar, L::kStageQ);
-            bulk(dst, kv + 2 * kDRowsBytes, 2 * kDRowsBytes, bar);
-            bulk(dst, head + 2 * kDRowsBytes, kABytes + kVecBytes, bar);
+            bulk(dst, kv + kDTransBytes, kDRowsBytes, bar);
+            bulk(dst, head + kDRowsBytes, kDABytes + kDVecBytes, bar);
         } else {
             unsigned char* dst = sStageW + st * L::kStageW;
             mbar_expect_tx(bar, L::kStageW);
-            bulk(dst, head, 2 * kDRowsBytes, bar);
-            bulk(dst, kv, 2 * kDRowsBytes, bar);
+            bulk(dst, head, kDRowsBytes, bar);
+            bulk(dst, kv, kDTransBytes, bar);
             bulk(dst, u_image<NB>(p, lc, h, cb), L::kU, bar);
-            bulk(dst, head + 2 * kDRowsBytes + kABytes, kVecBytes, bar);
+            bulk(dst, head + kDRowsBytes + kDABytes, kDVecBytes, bar);
         }
     };
     if (w == 0 && lane == 0) {
         fetch(0);
         if (n > 1) fetch(1);
     }
-    // lhs (32 rows of 128, hi and lo) times the chunk's S: the warp's tile, the three parts of the split in chains of their own
-    auto times_s = [&](float (&a0)[4], const __nv_bfloat16* lhs, const __nv_bfloat16* rhs) {
-        float a1[4] = {0.f, 0.f, 0.f, 0.f}, a2[4] = {0.f, 0.f, 0.f, 0.f};
+    // lhs (32 rows of 128) times the chunk's S: the warp's tile; hi hi in four chains, the cross terms in two
+    auto times_s = [&](float (&a0)[4], const float* lhs, const float* rhs) {
+        float c[4][4], x[2][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a0[i] = 0.f;
-        lhs += (m + (lane & 15)) * kDLD + (lane >> 4) * 8;
-        rhs += lane * LS + nn;
+        for (int i = 0; i < 16; ++i) { c[i >> 2][i & 3] = 0.f; x[(i >> 2) & 1][i & 3] = 0.f; }
+        lhs += m * kDLF + a_lane(lane, kDLF);
+        rhs += nn * kDLF + b_lane(lane, kDLF);
 #pragma unroll
-        for (int k = 0; k < kDK / 16; k += 2) {
-            uint32_t bh[4], bl[4];
-            ldm_x4_trans(bh, rhs + k * 16 * LS);
-            ldm_x4_trans(bl, rhs + (kDK + k * 16) * LS);
+        for (int k = 0; k < kDK / 16; ++k) {
+            uint32_t b[4], bh[4], bl[4];
+            ldm_x4(b, rhs + k * 16);
+            split_tf32(b, bh, bl);
 #pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-                uint32_t xh[4], xl[4];
-                ldm_x4(xh, lhs + (k + kk) * 16);
-                ldm_x4(xl, lhs + kDC * kDLD + (k + kk) * 16);
-                mma_16816(a0, xh, bh[2 * kk], bh[2 * kk + 1]);
-                mma_16816(a1, xh, bl[2 * kk], bl[2 * kk + 1]);
-                mma_16816(a2, xl, bh[2 * kk], bh[2 * kk + 1]);
+            for (int e = 0; e < 2; ++e) {
+                uint32_t a[4], ah[4], al[4];
+                ldm_x4(a, lhs + k * 16 + e * 8);
+                split_tf32(a, ah, al);
+                mma_1688(c[k & 3], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(x[0], ah, bl[2 * e], bl[2 * e + 1]);
+                mma_1688(x[1], al, bh[2 * e], bh[2 * e + 1]);
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a0[i] += a1[i] + a2[i];
+        for (int i = 0; i < 4; ++i) a0[i] = ((c[0][i] + c[1][i]) + (c[2][i] + c[3][i])) + (x[0][i] + x[1][i]);
     };
     // named barriers: 1 the first half; 2, 3 `ready` and 4, 5 `done` of even and odd chunks
     if (!is_q) {
@@ -432,17 +458,12 @@ delta_chain_kernel(const DeltaChunkParams p) {
         auto tile_n = [&](int t) { return (NB == 32 ? t : t & 1) * 8; };
         float* st_base = p.state + static_cast<int64_t>(slot) * p.state_floats + static_cast<int64_t>(h) * kDK * p.dv + cb * NB;
         float S[4][4];
-        auto write_s = [&](__nv_bfloat16* dst0) {
+        auto write_s = [&](float* dst0) {
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint32_t hi, lo;
-                    split_pair(S[t][half * 2], S[t][half * 2 + 1], hi, lo);
-                    __nv_bfloat16* dst = dst0 + (tile_m(t) + (lane >> 2) + half * 8) * LS + tile_n(t) + (lane & 3) * 2;
-                    *reinterpret_cast<uint32_t*>(dst) = hi;
-                    *reinterpret_cast<uint32_t*>(dst + kDK * LS) = lo;
-                }
+                for (int e = 0; e < 4; ++e)
+                    dst0[(tile_n(t) + (lane & 3) * 2 + (e & 1)) * kDLF + tile_m(t) + (lane >> 2) + (e >> 1) * 8] = S[t][e];
             }
         };
 #pragma unroll
@@ -459,26 +480,23 @@ delta_chain_kernel(const DeltaChunkParams p) {
         for (int c = 0; c < n; ++c) {
             const int st = c & 1;
             const unsigned char* base = sStageW + st * L::kStageW;
-            const __nv_bfloat16* sW = reinterpret_cast<const __nv_bfloat16*>(base);
-            const __nv_bfloat16* sK = sW + 2 * kDC * kDLD;
-            const float* sUt = reinterpret_cast<const float*>(base + 4 * kDRowsBytes);
+            const float* sW = reinterpret_cast<const float*>(base);
+            const float* sKt = reinterpret_cast<const float*>(base + kDRowsBytes);
+            const float* sUt = reinterpret_cast<const float*>(base + kDRowsBytes + kDTransBytes);
             const float* sE = sUt + kDC * LS;
-            __nv_bfloat16* u_buf = sU + st * 2 * kDC * LS;
+            float* u_buf = sU + st * NB * kDLT;
             mbar_wait(full + st, (c >> 1) & 1, p.err);
             float a[4];
-            times_s(a, sW, sS + st * 2 * kDK * LS);
+            times_s(a, sW, sS + st * NB * kDLF);
 #pragma unroll
             for (int half = 0; half < 2; ++half) {                                 // U = U~ - W S, and D_31 U
                 const int i = m + (lane >> 2) + half * 8, j = nn + (lane & 3) * 2;
                 const float2 ut = *reinterpret_cast<const float2*>(sUt + i * LS + j);
                 const float ux = ut.x - a[half * 2], uy = ut.y - a[half * 2 + 1], d = sE[kDC + i];
-                uint32_t hi, lo;
-                split_pair(d * ux, d * uy, hi, lo);
-                *reinterpret_cast<uint32_t*>(sDU + i * LS + j) = hi;
-                *reinterpret_cast<uint32_t*>(sDU + (kDC + i) * LS + j) = lo;
-                split_pair(ux, uy, hi, lo);
-                *reinterpret_cast<uint32_t*>(u_buf + i * LS + j) = hi;
-                *reinterpret_cast<uint32_t*>(u_buf + (kDC + i) * LS + j) = lo;
+                sDU[j * kDLT + i] = d * ux;
+                sDU[(j + 1) * kDLT + i] = d * uy;
+                u_buf[j * kDLT + i] = ux;
+                u_buf[(j + 1) * kDLT + i] = uy;
             }
             asm volatile("bar.arrive %0, %1;\n" ::"r"(2 + st), "n"(kThreads) : "memory");        // ready
             asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads / 2) : "memory");
@@ -490,26 +508,34 @@ delta_chain_kernel(const DeltaChunkParams p) {
                 for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
             }
             constexpr int kN = NB / 8, kM = 4 / kN;                                // the warp's column and row tiles
-            uint32_t bh[kN][4], bl[kN][4];
 #pragma unroll
-            for (int t = 0; t < kN; ++t) {
-                ldm_x4_trans(bh[t], sDU + lane * LS + t * 8);
-                ldm_x4_trans(bl[t], sDU + (kDC + lane) * LS + t * 8);
-            }
+            for (int k = 0; k < kDC / 16; ++k) {
+                uint32_t bh[kN][4], bl[kN][4];
 #pragma unroll
-            for (int mt = 0; mt < kM; ++mt) {
-                const __nv_bfloat16* kt = sK + ((lane & 7) + (lane >> 4) * 8) * kDLD + tile_m(mt * kN) + ((lane >> 3) & 1) * 8;
+                for (int t = 0; t < kN; ++t) {
+                    uint32_t b[4];
+                    ldm_x4(b, sDU + t * 8 * kDLT + k * 16 + b_lane(lane, kDLT));
+                    split_tf32(b, bh[t], bl[t]);
+                }
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
-                    uint32_t kh[4], kl[4];
-                    ldm_x4_trans(kh, kt + k * 16 * kDLD);
-                    ldm_x4_trans(kl, kt + (kDC + k * 16) * kDLD);
+                for (int mt = 0; mt < kM; ++mt) {
+                    float hh[kN][4], x[kN][4];                                     // a chain of two products, added up by the float units
 #pragma unroll
-                    for (int t = 0; t < kN; ++t) {
-                        mma_16816(acc[mt * kN + t], kh, bh[t][2 * k], bh[t][2 * k + 1]);
-                        mma_16816(acc[mt * kN + t], kh, bl[t][2 * k], bl[t][2 * k + 1]);
-                        mma_16816(acc[mt * kN + t], kl, bh[t][2 * k], bh[t][2 * k + 1]);
+                    for (int i = 0; i < kN * 4; ++i) hh[i >> 2][i & 3] = x[i >> 2][i & 3] = 0.f;
+#pragma unroll
+                    for (int ee = 0; ee < 2; ++ee) {
+                        uint32_t ka[4], kh[4], kl[4];
+                        ldm_x4(ka, sKt + tile_m(mt * kN) * kDLT + k * 16 + ee * 8 + a_lane(lane, kDLT));
+                        split_tf32(ka, kh, kl);
+#pragma unroll
+                        for (int t = 0; t < kN; ++t) {
+                            mma_1688(hh[t], kh, bh[t][2 * ee], bh[t][2 * ee + 1]);
+                            mma_1688(x[t], kh, bl[t][2 * ee], bl[t][2 * ee + 1]);
+                            mma_1688(x[t], kl, bh[t][2 * ee], bh[t][2 * ee + 1]);
+                        }
                     }
+#pragma unroll
+                    for (int i = 0; i < kN * 4; ++i) acc[mt * kN + (i >> 2)][i & 3] += hh[i >> 2][i & 3] + x[i >> 2][i & 3];
                 }
             }
 #pragma unroll
@@ -518,7 +544,7 @@ delta_chain_kernel(const DeltaChunkParams p) {
                 for (int i = 0; i < 4; ++i) S[t][i] = fmaf(e, S[t][i], acc[t][i]);
             }
             if (c > 0) asm volatile("bar.sync %0, %1;\n" ::"r"(4 + (st ^ 1)), "n"(kThreads) : "memory");     // done with the chunk before
-            if (c + 1 < n) write_s(sS + (st ^ 1) * 2 * kDK * LS);
+            if (c + 1 < n) write_s(sS + (st ^ 1) * NB * kDLF);
             asm volatile("bar.sync 1, %0;\n" ::"n"(kThreads / 2) : "memory");      // the new S is there; the stage may be filled again
             if (threadIdx.x == 0 && c + 2 < n) fetch(c + 2);
         }
@@ -532,29 +558,34 @@ delta_chain_kernel(const DeltaChunkParams p) {
     } else {
         for (int c = 0; c < n; ++c) {
             const int st = c & 1;
-            const __nv_bfloat16* sQ = reinterpret_cast<const __nv_bfloat16*>(sStageQ + st * L::kStageQ);
-            const __nv_bfloat16* sA = sQ + 2 * kDC * kDLD;
-            const float* sE = reinterpret_cast<const float*>(sA + 2 * kDC * kDLA);
-            const __nv_bfloat16* u_buf = sU + st * 2 * kDC * LS;
+            const float* sQ = reinterpret_cast<const float*>(sStageQ + st * L::kStageQ);
+            const float* sA = sQ + kDC * kDLF;
+            const float* sE = sA + kDC * kDLT;
+            const float* u_buf = sU + st * NB * kDLT;
             mbar_wait(full + 2 + st, (c >> 1) & 1, p.err);
             asm volatile("bar.sync %0, %1;\n" ::"r"(2 + st), "n"(kThreads) : "memory");          // ready
             float o[4];
-            times_s(o, sQ, sS + st * 2 * kDK * LS);
+            times_s(o, sQ, sS + st * NB * kDLF);
+            float au[2][4], x[2][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] *= sE[m + (lane >> 2) + (i >> 1) * 8];
-            uint32_t bh[4], bl[4];
-            ldm_x4_trans(bh, u_buf + lane * LS + nn);
-            ldm_x4_trans(bl, u_buf + (kDC + lane) * LS + nn);
-            const __nv_bfloat16* al = sA + (m + (lane & 15)) * kDLA + (lane >> 4) * 8;
+            for (int i = 0; i < 8; ++i) au[i >> 2][i & 3] = x[i >> 2][i & 3] = 0.f;
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                uint32_t xh[4], xl[4];
-                ldm_x4(xh, al + k * 16);
-                ldm_x4(xl, al + kDC * kDLA + k * 16);
-                mma_16816(o, xh, bh[2 * k], bh[2 * k + 1]);
-                mma_16816(o, xh, bl[2 * k], bl[2 * k + 1]);
-                mma_16816(o, xl, bh[2 * k], bh[2 * k + 1]);
+            for (int k = 0; k < kDC / 16; ++k) {
+                uint32_t b[4], bh[4], bl[4];
+                ldm_x4(b, u_buf + nn * kDLT + k * 16 + b_lane(lane, kDLT));
+                split_tf32(b, bh, bl);
+#pragma unroll
+                for (int ee = 0; ee < 2; ++ee) {
+                    uint32_t ra[4], ah[4], al[4];
+                    ldm_x4(ra, sA + m * kDLT + k * 16 + ee * 8 + a_lane(lane, kDLT));
+                    split_tf32(ra, ah, al);
+                    mma_1688(au[k], ah, bh[2 * ee], bh[2 * ee + 1]);
+                    mma_1688(x[0], ah, bl[2 * ee], bl[2 * ee + 1]);
+                    mma_1688(x[1], al, bh[2 * ee], bh[2 * ee + 1]);
+                }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = fmaf(o[i], sE[m + (lane >> 2) + (i >> 1) * 8], (au[0][i] + au[1][i]) + (x[0][i] + x[1][i]));
             if (c + 1 < n) asm volatile("bar.arrive %0, %1;\n" ::"r"(4 + st), "n"(kThreads) : "memory");     // done
             const int t0 = begin + (c0 + c - first) * kDC;
 #pragma unroll
