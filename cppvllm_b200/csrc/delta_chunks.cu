@@ -327,10 +327,10 @@ delta_prepare_kernel(const DeltaChunkParams p) {
             for (int j = 0; j < kDC - 1; ++j) {
 #pragma unroll
                 for (int i4 = (j + 1) / 4 * 4; i4 < kDC; i4 += 4) {
-                    const float4 l = *reinterpret_cast<const float4*>(Lt + j * 36 + i4);   // zero on and above the diagonal
-                    x[i4] = fmaf(-l.x, x[j], x[i4]);
-                    x[i4 + 1] = fmaf(-l.y, x[j], x[i4 + 1]);
-                    x[i4 + 2] = fmaf(-l.z, x[j], x[i4 + 2]);
+                    const float4 l = *reinterpret_cast<const float4*>(Lt + j * 36 + i4);
+                    if (i4 > j) x[i4] = fmaf(-l.x, x[j], x[i4]);                       // rows up to j stay out of it: 0 times a bad x_j is a NaN
+                    if (i4 + 1 > j) x[i4 + 1] = fmaf(-l.y, x[j], x[i4 + 1]);
+                    if (i4 + 2 > j) x[i4 + 2] = fmaf(-l.z, x[j], x[i4 + 2]);
                     x[i4 + 3] = fmaf(-l.w, x[j], x[i4 + 3]);
                 }
             }
@@ -585,7 +585,17 @@ delta_chain_kernel(const DeltaChunkParams p) {
                 }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o[i] = fmaf(o[i], sE[m + (lane >> 2) + (i >> 1) * 8], (au[0][i] + au[1][i]) + (x[0][i] + x[1][i]));
+            for (int i = 0; i < 4; ++i) {
+                const int row = m + (lane >> 2) + (i >> 1) * 8, col = nn + (lane & 3) * 2 + (i & 1);
+                const float qs = o[i] * sE[row];
+                o[i] = qs + ((au[0][i] + au[1][i]) + (x[0][i] + x[1][i]));
+                // A's zeros above the diagonal times an infinity or a NaN of a later token: the row's own tokens alone, one after the other
+                if (!(fabsf(o[i]) <= 3.402823466e38f)) {
+                    float own = 0.f;
+                    for (int j = 0; j <= row; ++j) own = fmaf(sA[row * kDLT + j], u_buf[col * kDLT + j], own);
+                    o[i] = qs + own;
+                }
+            }
             if (c + 1 < n) asm volatile("bar.arrive %0, %1;\n" ::"r"(4 + st), "n"(kThreads) : "memory");     // done
             const int t0 = begin + (c0 + c - first) * kDC;
 #pragma unroll

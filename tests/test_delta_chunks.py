@@ -85,3 +85,34 @@ def test_what_the_rule_leaves_to_the_scan():
     assert ok() and ok(dv=64) and ok(off=2)
     assert not ok(packed=row[:, :512].float()) and not ok(packed=row) and not ok(off=1) and not ok(taps=5)
     assert not ok(dk=64) and not ok(dv=96) and not ok(w=128 * 128 + 1) and not ok(n=63) and not ok(H=8)
+
+
+@pytest.mark.parametrize("channel", ["q", "k", "v"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_bad_token_reaches_no_token_before_it(channel, bad):
+    """As in the rule token by token: a bad query spoils the rows that its convolution reaches, a bad value its column from there on."""
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.parts.base import Workspace
+    gen, d = torch.Generator().manual_seed(6), torch.device("cuda:0")
+    H, G, dk, dv, T, taps, at = 2, 1, 128, 128, 90, 4, 50
+    mat, C = H * dk * dv, 2 * G * dk + H * dv
+    packed = torch.randn(T, C, generator=gen).to(torch.bfloat16)
+    conv, dt_bias, a_log = torch.randn(C, taps, generator=gen) * 0.6, torch.randn(H, generator=gen), torch.randn(H, generator=gen) - 1
+    ba = torch.randn(T, 2 * H, generator=gen)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=d)             # noqa: E731
+
+    def run():
+        state, out = torch.zeros(1, mat + (taps - 1) * C, device=d), torch.zeros(T, H * dv, device=d)
+        ops.delta_chunks(out, packed.to(d), 0, conv.to(d), ba.to(d), dt_bias.to(d), a_log.to(d), state, mat, i32([0, T]), i32([0]), [T], H, G, dk, dv,
+                         Workspace(d, 1024, 8))
+        return out.cpu()
+    clean = run()
+    packed[at, {"q": 3, "k": dk + 3, "v": 2 * dk + 3}[channel]] = bad
+    got = run()
+    assert torch.equal(got[:32], clean[:32])                         # the chunk in front; in its own a bad token's columns are summed another way
+    assert float((got[:at] - clean[:at]).abs().max()) < 1e-6 * float(clean.abs().max()) and not bool(torch.isfinite(got[at:at + taps]).all())
+    if channel == "q":
+        assert torch.equal(got[at + taps:], clean[at + taps:])
+    if channel == "v":
+        others = [i for i in range(H * dv) if i != 3]
+        assert torch.equal(got[:, others], clean[:, others]) and not bool(torch.isfinite(got[at:, 3]).any())
