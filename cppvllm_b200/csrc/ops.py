@@ -804,13 +804,16 @@ def delta_chunks_shape(dtype: torch.dtype, taps: int, dim: int, vdim: int) -> bo
 def delta_chunks_supported(packed: torch.Tensor, qkv_off: int, taps: int, num_heads: int, num_kv_heads: int, dim: int, vdim: int, state: torch.Tensor,
                            q_lens) -> bool:
     """Whether portions of the rule with one decay per head go through the tensor cores (csrc/delta_chunks.cu): activations in bf16 (float32 stays
-    on the token-by-token scan), keys of 128 and values of 64 or 128 elements, up to four taps, channels and states that start on whole pairs, and
-    a long portion.  The scan takes 0.41 us a token of the longest portion; the chunks cost 25 us at two heads a kv head and 17 us more for every
-    further pair of them before the first token is done.  Measured, a layer, chunks against scan, us: 16/8 heads 64 tokens 46 / 47, 128 tokens 49 /
-    69, 33 tokens 45 / 39; 32/8 heads 128 tokens 100 / 105, 64 tokens 94 / 79."""
-    least = 24 + 40 * ((num_heads // num_kv_heads + 1) // 2)
+    on the token-by-token scan), keys of 128 and values of 64 or 128 elements, up to four taps, channels and states that start on whole pairs, a
+    long portion and few other requests.  The scan takes 0.41 us a token of the longest portion, every request beside it at once; the chunks cost 25 us
+    at two heads a kv head and 17 us more for every further pair of them before the first token is done, and every other request, be it one token, a
+    chunk of 32 and blocks of its own on the SMs.  Measured, a layer, chunks against scan, us: 16/8 heads 33 tokens 56 / 60, 64 tokens 56 / 71, 256 tokens
+    68 / 143; 32/8 heads 64 tokens 103 / 105, 128 tokens 112 / 131; beside decoded tokens at 16/8 heads 64 + 8 of them 82 / 90, 64 + 64 282 / 164, 512 + 32
+    245 / 329, 512 + 64 364 / 366, 512 + 240 1,214 / 619; at 32/8 heads 512 + 32 445 / 491, 512 + 64 677 / 575."""
+    longest, least = max(q_lens), 24 + 40 * ((num_heads // num_kv_heads + 1) // 2)
     return (delta_chunks_shape(packed.dtype, taps, dim, vdim) and state.shape[1] % 2 == 0
-            and packed.stride(0) % 2 == 0 and qkv_off % 2 == 0 and packed.data_ptr() % 4 == 0 and max(q_lens) >= least)
+            and packed.stride(0) % 2 == 0 and qkv_off % 2 == 0 and packed.data_ptr() % 4 == 0
+            and longest >= least and (len(q_lens) - 1) * num_heads <= 2 * longest)
 
 
 def delta_chunks(out, packed, qkv_off: int, conv_w, ba, dt_bias, a_log, state: torch.Tensor, conv_off: int, cu_seqlens, state_slots, q_lens,

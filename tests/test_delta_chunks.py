@@ -116,3 +116,13 @@ def test_a_bad_token_reaches_no_token_before_it(channel, bad):
     if channel == "v":
         others = [i for i in range(H * dv) if i != 3]
         assert torch.equal(got[:, others], clean[:, others]) and not bool(torch.isfinite(got[at:, 3]).any())
+
+
+def test_steps_of_many_requests_stay_with_the_scan():
+    from cppvllm_b200.csrc import ops
+    state, row = torch.zeros(2, 128 * 128), torch.zeros(40, 512, dtype=torch.bfloat16)
+
+    def ok(q_lens, H=16):
+        return ops.delta_chunks_supported(row, 0, 4, H, H // 2, 128, 128, state, q_lens)
+    assert ok([64] + [1] * 8) and not ok([64] + [1] * 9) and ok([1] * 64 + [512]) and not ok([1] * 65 + [512])
+    assert ok([512] + [1] * 32, H=32) and not ok([512] + [1] * 33, H=32) and ok([200] * 8) and not ok([64] * 12)
