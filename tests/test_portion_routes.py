@@ -180,7 +180,7 @@ def test_the_kernel_refuses_a_scale_it_would_apply_behind_the_mask():
 
 def test_kept_first_tokens_with_a_distance_term(monkeypatch):
     """They are seen from beyond the chunk and the window: no table of distances is long enough, and the step stays with the other kernels."""
-    diffs = both(monkeypatch, "attn_masked_bf16", "masked_attention", chunk=150, window=140, keep_first=20, distance_bias=True)
+    diffs = both(monkeypatch, "attn_masked_bf16", "masked_attention", chunk=150, window=140, keep_first=100, distance_bias=True)
     assert max(diffs) < BF16, diffs
 
 
