@@ -7,15 +7,17 @@
 // What bounds the mma.sync kernels is the legacy tensor path and the shared-memory reads that feed it: 64 query rows per block and
 // 64 keys per tile, every operand fragment through ldmatrix.  Here a block owns 256 query rows of one kv head as two tiles of 128 (row r
 // of a tile = token r / g, head r % g of the group), walks tiles of 128 entries, and the tensor core alternates between the two query
-// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, before -> now): chunks of 1,024 179 -> 28; a latent of
-// 96 + 32 under 16 heads 171 -> 41; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 42; keys that are values at 32/8 heads
-// (1,917 tokens of three requests behind a window of 1,024) 196 -> 48.
+// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, before -> now): chunks of 1,024 179 -> 29; a latent of
+// 96 + 32 under 16 heads 171 -> 43; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 47; keys that are values at 32/8 heads
+// (1,917 tokens of three requests behind a window of 1,024) 196 -> 51.
 //   warp 0     producer: one lane per TMA box (page or 64 entries, times 64 columns, times key and value), 128-byte swizzle.  Key and
 //              value apart: two stages, each with the keys of tile i + 1 and the values of tile i (what one round reads).  Shared
 //              entries: four stages of one tile, read row-wise by S = Q K^T and transposed by O += P K;
 //   warp 1     allocates 512 columns of tensor memory and issues the products: P_i V_i, then S_{i+1}, for either query tile;
 //   warps 4-11 softmax, one thread per query row: S from tensor memory, scale, cap, term by distance, mask, exponentials, P back over
-//              S; O is rescaled in tensor memory only when a row's maximum has grown by 2^8.
+//              S; O is rescaled in tensor memory when some row of the warp has a new maximum.  The reference is the maximum itself, so that a row's
+//              largest probability is 1 and rounds to 1: with one that followed only after 2^8, layers were 1 to 5 % further from float64 (capped
+//              scores 4.00e-3 -> 4.22e-3, a bias per distance 4.82e-3 -> 4.90e-3) and 2 to 5 % faster (a bias per distance 79 us against 83).
 // The tiles a block walks are a list: pooled blocks any of its tokens sees (plane 1), kept first tokens that lie wholly before the
 // rest, then the tokens from the first one its first token sees to its last token; a query tile skips list entries it sees nothing of.
 //   distance terms: bias[h, min(p - j, L - 1)] or -r1_h ln(1 + r2_h (p - j)) come from a table in shared memory, one row per head of
@@ -36,7 +38,6 @@ constexpr int kEM = 128;                      // query rows per tile
 constexpr int kEN = 128;                      // entries per tile
 constexpr int kEThreads = 128 + 256;          // one warpgroup of helpers (two warps idle), one warpgroup per query tile
 constexpr float kELog2e = 1.4426950408889634f;
-constexpr float kERescaleStep = 8.f;          // log2 of the growth of a row's maximum that forces a rescale
 constexpr int kEMaxPieces = 8;
 constexpr int kEPadHigh = 160;                // entries behind a distance table's last one: 127 keys and 32 tokens of a warp
 
@@ -445,9 +446,7 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                 float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
                 if (!TERMS) m_tile *= scale_log2;
                 const float m_new = fmaxf(m_ref, m_tile);
-                // the reference maximum follows only when some row of the warp has outgrown it
-                const bool grow = m_new > m_ref + kERescaleStep;
-                if (__any_sync(0xffffffffu, grow)) {
+                if (__any_sync(0xffffffffu, m_new > m_ref)) {
                     const float m_use = m_new == -INFINITY ? 0.f : m_new;
                     const float factor = ex2(m_ref - m_use);             // 2^(-inf) = 0 before the first key
                     m_ref = m_new;

@@ -235,3 +235,18 @@ def test_a_cap_does_not_depend_on_what_unused_slots_hold():
         pages[-1, :, :, (n + cached) % 32:] *= factor
         outs.append(run_one(q, pages, H, G, dim, False, n, cached, softcap=30.0, chunk=200))
     assert torch.equal(*outs)
+
+
+@pytest.mark.gpu
+def test_the_largest_probability_of_a_row_is_not_rounded():
+    """Two keys that count, one in the first tile and one in the last with 7 to 200 times its weight, and values of 1: the weighted sum over the sum of the
+    weights is 1, where the larger weight is 1 and rounds to bf16 as 1 (the smaller one, at most 0.14, is off by 3e-4; outputs below 1 are 4e-3 apart)."""
+    H, G, dim, n, cached, heavy = 2, 2, 128, 32, 480, 480
+    for k in range(20, 56, 3):                               # times 0.1: the larger score; the smaller one is 0, the others -100
+        q, pages = one_request(H, G, dim, False, n, cached)
+        q[:], pages[..., :dim], pages[..., dim:] = 0, 0, 1
+        q[:, 0], q[:, dim] = 1, 1
+        pages[..., 0] = -1000
+        pages[0, 0, :, 0, 0], pages[heavy // 32, 0, :, heavy % 32, 0] = 0, k
+        out = run_one(q, pages, H, G, dim, False, n, cached)
+        assert bool((out == 1).all()), (k, float(out.min()), float(out.max()))
