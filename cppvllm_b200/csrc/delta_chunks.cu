@@ -12,11 +12,11 @@
 // running products (never logarithms: g may be 0).
 //
 // Products run as `mma.sync.m16n8k8` in tf32 with every float operand split in two when its fragment is loaded (x = hi + lo: hi the nearest tf32
-// number, lo the rest, of which the product reads 11 bits more; hi hi + hi lo + lo hi), float accumulation in several short chains that are added
-// up by the float units (the tensor core cuts a sum off instead of rounding it).  From the same projection, 64 to 2,048 tokens at 16/8 and 32/8
-// heads, the outputs are 2.7e-7 to 3.9e-7 from float64 and the states 2.4e-7 to 4.0e-7 (the float scan: 1.9e-7 to 3.7e-7, 2.2e-7 to 4.0e-7; with
-// bf16 pairs 5.3e-6 to 6.3e-6, 4.7e-6 to 4.9e-6); behind the layer's bf16 projections the two routes are equally far, 4.2e-3.  W and U~ come
-// from a float substitution, one thread per column.  Steps in float32 stay on the scan.
+// number, lo the rest, of which the product reads 11 bits more; hi hi + hi lo + lo hi), float accumulation, the leading terms in chains of two
+// products that are added up by the float units (the tensor core cuts a sum off instead of rounding it; chains of four cost the outputs 4 %).  From
+// the same projection, 64 to 2,048 tokens at 16/8 and 32/8 heads, the outputs are 2.5e-7 to 3.8e-7 from float64 and the states 2.4e-7 to 4.0e-7 (the
+// float scan: 1.9e-7 to 3.7e-7, 2.2e-7 to 4.0e-7; with bf16 pairs 5.3e-6 to 6.3e-6, 4.7e-6 to 4.9e-6); behind the layer's bf16 projections the two
+// routes are equally far, 4.2e-3.  W and U~ come from a float substitution, one thread per column.  Steps in float32 stay on the scan.
 // Chunk images in scratch are laid out as the chain kernel wants them in shared memory (every operand with its inner dimension running, rows
 // padded against ldmatrix conflicts), so a chunk arrives by a few bulk copies, two chunks ahead.
 #include "common.cuh"
@@ -228,34 +228,34 @@ delta_prepare_kernel(const DeltaChunkParams p) {
     const int m = (warp & 1) * 16, nn = (warp >> 1) * 8;
     float kk[4], qk[4];
     {
-        float ck[4][4], cq[4][4], xk[4] = {0.f, 0.f, 0.f, 0.f}, xq[4] = {0.f, 0.f, 0.f, 0.f};     // hi hi in four chains; the cross terms
+        float xk[4] = {0.f, 0.f, 0.f, 0.f}, xq[4] = {0.f, 0.f, 0.f, 0.f};          // the cross terms
 #pragma unroll
-        for (int i = 0; i < 16; ++i) ck[i >> 2][i & 3] = cq[i >> 2][i & 3] = 0.f;
+        for (int i = 0; i < 4; ++i) kk[i] = qk[i] = 0.f;
 #pragma unroll
         for (int k = 0; k < kDK / 16; ++k) {
             uint32_t b[4], bh[4], bl[4];
             ldm_x4(b, sK + nn * kDLF + k * 16 + b_lane(lane, kDLF));
             split_tf32(b, bh, bl);
+            float ck[4] = {0.f, 0.f, 0.f, 0.f}, cq[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 uint32_t a[4], ah[4], al[4];
                 ldm_x4(a, sK + m * kDLF + k * 16 + e * 8 + a_lane(lane, kDLF));
                 split_tf32(a, ah, al);
-                mma_1688(ck[k >> 1], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(ck, ah, bh[2 * e], bh[2 * e + 1]);
                 mma_1688(xk, ah, bl[2 * e], bl[2 * e + 1]);
                 mma_1688(xk, al, bh[2 * e], bh[2 * e + 1]);
                 ldm_x4(a, sQ + m * kDLF + k * 16 + e * 8 + a_lane(lane, kDLF));
                 split_tf32(a, ah, al);
-                mma_1688(cq[k >> 1], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(cq, ah, bh[2 * e], bh[2 * e + 1]);
                 mma_1688(xq, ah, bl[2 * e], bl[2 * e + 1]);
                 mma_1688(xq, al, bh[2 * e], bh[2 * e + 1]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { kk[i] += ck[i]; qk[i] += cq[i]; }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            kk[i] = ((ck[0][i] + ck[1][i]) + (ck[2][i] + ck[3][i])) + xk[i];
-            qk[i] = ((cq[0][i] + cq[1][i]) + (cq[2][i] + cq[3][i])) + xq[i];
-        }
+        for (int i = 0; i < 4; ++i) { kk[i] += xk[i]; qk[i] += xq[i]; }
     }
     for (int h0 = 0; h0 < share; h0 += kDPair) {
         const int heads = min(kDPair, share - h0), hbase = kvh * share + h0;
@@ -361,8 +361,8 @@ struct DeltaChainSmem {
 // Grid (request, head, NB value columns); NB / 2 warps in two halves.  The first half carries the chain: W S, U = U~ - W S, S = e_31 S + K^T (D_31 U),
 // with two barriers of its own a chunk.  The second half makes the outputs e Q S + A U beside it, up to a chunk behind: S and U have two
 // buffers, `ready` (U of the chunk is there, S was before) and `done` (the outputs have been made) hand them over.  Each half fetches for itself, two
-// chunks ahead.  What bounds it is instruction issue: a fragment's split costs three instructions a register, six products stand where float ones would
-// be two (1,511 + 537 tokens, 16 heads: 150 us, 6,100 cycles a chunk; with bf16 pairs, split once in memory, 84).
+// chunks ahead.  What bounds it is the tensor pipe at the rate of tf32 mma.sync (warps stall on it most) and, next to it, the fragments' splits of
+// three instructions a register: 1,511 + 537 tokens, 16 heads 145 us, 5,900 cycles a chunk; with bf16 pairs, split once in memory, 84.
 template <int NB>
 __global__ void __launch_bounds__(NB * 16, 1)
 delta_chain_kernel(const DeltaChunkParams p) {
@@ -426,11 +426,11 @@ delta_chain_kernel(const DeltaChunkParams p) {
         fetch(0);
         if (n > 1) fetch(1);
     }
-    // lhs (32 rows of 128) times the chunk's S: the warp's tile; hi hi in four chains, the cross terms in two
+    // lhs (32 rows of 128) times the chunk's S: the warp's tile
     auto times_s = [&](float (&a0)[4], const float* lhs, const float* rhs) {
-        float c[4][4], x[2][4];
+        float x[2][4];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { c[i >> 2][i & 3] = 0.f; x[(i >> 2) & 1][i & 3] = 0.f; }
+        for (int i = 0; i < 8; ++i) { x[i >> 2][i & 3] = 0.f; a0[i & 3] = 0.f; }
         lhs += m * kDLF + a_lane(lane, kDLF);
         rhs += nn * kDLF + b_lane(lane, kDLF);
 #pragma unroll
@@ -438,18 +438,21 @@ delta_chain_kernel(const DeltaChunkParams p) {
             uint32_t b[4], bh[4], bl[4];
             ldm_x4(b, rhs + k * 16);
             split_tf32(b, bh, bl);
+            float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 uint32_t a[4], ah[4], al[4];
                 ldm_x4(a, lhs + k * 16 + e * 8);
                 split_tf32(a, ah, al);
-                mma_1688(c[k & 3], ah, bh[2 * e], bh[2 * e + 1]);
+                mma_1688(c, ah, bh[2 * e], bh[2 * e + 1]);
                 mma_1688(x[0], ah, bl[2 * e], bl[2 * e + 1]);
                 mma_1688(x[1], al, bh[2 * e], bh[2 * e + 1]);
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a0[i] += c[i];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) a0[i] = ((c[0][i] + c[1][i]) + (c[2][i] + c[3][i])) + (x[0][i] + x[1][i]);
+        for (int i = 0; i < 4; ++i) a0[i] += x[0][i] + x[1][i];
     };
     // named barriers: 1 the first half; 2, 3 `ready` and 4, 5 `done` of even and odd chunks
     if (!is_q) {
