@@ -12,7 +12,7 @@ Every distance of `far` and more falls into the last bucket, so the bias is a ta
 load time; the kernels look up min(p - j, far).  The cache holds, per token and kv head, the normed key and behind it the
 value (pages [page, kv head, slot, dim + vdim]).  A mixer with ``reads_other_cache`` has no key and value projections and
 reads the entries another layer wrote, with its own queries, bias table and output projection.  bf16 with sizes the
-tensor-core kernel takes runs there (csrc/attention_bias.cu); float32 and other shapes take the general kernel
+tensor-core kernels take runs there (csrc/attention_bias.cu, portions at heads of 64 or 128 csrc/attention_entries_tcgen05.cu); float32 and other shapes take the general kernel
 (csrc/attention_general.cu).
 """
 from __future__ import annotations

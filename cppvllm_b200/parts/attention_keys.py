@@ -8,9 +8,10 @@
 
 No rotation: positions enter only through the mask.  The first ``keep_first`` positions stay visible after the window has
 passed them; the cache manager keeps their pages and gives the others back as the window passes.  All sizes and the
-scale are parameters.  Prompt portions and decoded tokens run through the same kernels: every token attends to its
+scale are parameters.  Prompt portions and decoded tokens read the same entries: every token attends to its
 request's pages, which already hold the step's own keys.  bf16 with head sizes that are multiples of 16 (up to 128) runs
-on the tensor cores (csrc/attention_keys.cu: one tile of keys in shared memory feeds both products); float32 and other
+on the tensor cores (csrc/attention_keys.cu, portions at heads of 64 or 128 csrc/attention_entries_tcgen05.cu: one tile of keys in
+shared memory feeds both products); float32 and other
 shapes take the general kernel (csrc/attention_general.cu).
 """
 from __future__ import annotations

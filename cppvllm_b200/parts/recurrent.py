@@ -13,7 +13,7 @@ type; only the projections around them are products in the activations' type.
   two low-rank projections are whatever the checkpoint holds.
 * ``head_delta``: the same rule with ONE decay per head and token, g = exp(-exp(A_h) * softplus(Wa x + dt_h)), S <- g S, full-rank
   projections for the decay (Wa [H, D]) and the output gate (Wg [H * vdim, D]), and the gate through silu instead of the
-  logistic function: y = Wo concat_h(RMSNorm(o_h) * w * silu(Wg x)_h).
+  logistic function: y = Wo concat_h(RMSNorm(o_h) * w * silu(Wg x)_h).  Long portions in bf16 run in chunks on the tensor cores (csrc/delta_chunks.cu).
 * ``gated_linear``: q = Wq x * dim^-1/2, k = Wk x, v = Wv x; g = sigmoid(Wa2 Wa1 x + b)^(1 / tau) per head and key channel;
   S <- diag(g) S + k v^T;  o = S^T q;  y = Wo concat_h(RMSNorm(o_h) * w * silu(Wg x)_h), w shared by the heads.  State per request:
   [H, dim, vdim].  A step of decoded tokens is one kernel between the projections.  The inner size of the low-rank projection is
