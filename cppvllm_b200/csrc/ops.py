@@ -1231,10 +1231,12 @@ def _attn_entries_shape(H, G, dk, dv, shared, page_size, planes, chunk, window, 
 
 
 # What a block costs outside its tiles (tensor memory, barriers, the query tiles, the output through shared memory) is more than an
-# mma.sync block's, so a step whose tokens all see less than one tile of entries stays there.  Measured, a layer of 64 tokens of a new
-# prompt / 4 tokens behind 124 / 128 tokens of a new prompt, us, mma.sync against tcgen05: chunks with cap, distance term and gate at
-# 32/8 heads 31 / 36 / 41 against 39 / 40 / 42, a bias per distance at 16/8 heads 22 / 24 / 27 against 26 / 24 / 27, keys that are values at
-# 32/8 heads 28 / 28 / 34.5 against 29.5 / 24 / 32, chunks with a gate at 16/8 heads 27 / 27 / 33 against 23 / 21 / 25.
+# mma.sync block's, so a step whose tokens all see less than one tile of entries stays there.  Measured, a layer's device time, us, mma.sync
+# against tcgen05, 64 tokens of a new prompt / 4 tokens behind 124 / 128 tokens of a new prompt: chunks with cap, distance term and gate at 32/8
+# heads 36.9 / 39.1 / 45.4 against 37.7 / 31.0 / 39.3, a window with kept tokens and a cap at 16/8 heads 25.6 / 26.0 / 33.1 against 26.6 / 20.4 /
+# 27.4, a bias per distance at 16/8 heads 22.7 / 22.7 / 30.9 against 24.8 / 19.8 / 25.0, keys that are values at 32/8 heads 33.1 / 30.9 / 41.2
+# against 33.0 / 24.9 / 33.1, a latent under 16 heads 43.3 / 38.3 / 47.5 against 43.3 / 34.2 / 43.6, under 32 heads 53.4 / 45.8 / 58.7 against
+# 55.4 / 42.9 / 57.2; the host's part of either call is the same.
 ENTRIES_MIN_VISIBLE = 128
 
 
