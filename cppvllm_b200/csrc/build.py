@@ -36,6 +36,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "attn_bf16": ["attention_bf16.cu"],
     "gemv_bf16": ["gemv_bf16.cu"],
     "gemm_bf16": ["gemm_tcgen05.cu"],
+    "gemm_experts": ["gemm_experts_tcgen05.cu"],
     "attn_tcgen05": ["attention_tcgen05.cu"],
     "attn_f32": ["attention_f32.cu"],
     "attn_entries": ["attention_entries_tcgen05.cu"],

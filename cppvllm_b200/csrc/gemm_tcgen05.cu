@@ -20,9 +20,6 @@
 //   warps 2-5 epilogue: each reads its 32 lanes of the accumulator with tcgen05.ld (32 columns at a time), applies the
 //            epilogue in float, rounds to bf16 once, stages boxes of 32 rows by 64 columns in shared memory for TMA
 //            stores (cp.async.bulk.tensor, whole lines, clipped at the edges) and hands the accumulator back.
-// Grouped form (a mixture of experts): the rows of A are sorted by expert into segments that start on multiples of 128
-// rows, a device table names the expert of every row tile, and the producer fetches the B tile from that expert's rows of
-// a weight that holds all experts' matrices one below the other; tiles without rows are skipped by all three roles.
 // Every wait on an mbarrier is bounded by a cycle count; a wait that runs out records error 5 and the block carries
 // on to its end (tensor memory is always given back).  No cluster launch, no multicast.
 #include "sm100.cuh"
@@ -35,10 +32,9 @@ constexpr int kBK = 64;                       // one 128-byte swizzle span of bf
 constexpr int kGemmThreads = 192;
 constexpr int kBoxBytes = 32 * 64 * 2;        // what a warp of the epilogue hands to one TMA store: 32 rows of 64 bf16
 
-// kRelu2: C = relu(T(A B^T))^2.  kSwiglu, kClamped and kGeglu share the gated tile: C = f(T(G), T(U)) with f = silu(g) u;
-// min(g, limit) sigmoid(alpha min(g, limit)) (clamp(u, -limit, limit) + 1);  gelu_tanh(g) u.
-enum GemmEpilogue { kPlain = 0, kSwiglu = 1, kAddResidual = 2, kRelu2 = 3, kClamped = 4, kGeglu = 5 };
-constexpr bool gated_epilogue(int e) { return e == kSwiglu || e == kClamped || e == kGeglu; }
+// kRelu2: C = relu(T(A B^T))^2.  kSwiglu and kGeglu share the gated tile: C = f(T(G), T(U)) with f = silu(g) u;  gelu_tanh(g) u.
+enum GemmEpilogue { kPlain = 0, kSwiglu = 1, kAddResidual = 2, kRelu2 = 3, kGeglu = 5 };
+constexpr bool gated_epilogue(int e) { return e == kSwiglu || e == kGeglu; }
 
 struct GemmParams {
     __nv_bfloat16* out;       // [M, n_out]
@@ -47,22 +43,12 @@ struct GemmParams {
     int n_out;                // output columns: N, or N / 2 with SwiGLU
     int tiles_m, tiles_n, num_tiles;
     int* err;
-    // grouped form (tile_expert != nullptr): W holds the matrices of several experts one below the other, `expert_rows`
-    // rows each; row tile i of A and of the output (128 rows) belongs to expert tile_expert[i] and is multiplied by that
-    // expert's matrix; a tile whose entry is negative holds no rows and is skipped by every role alike
-    const int* tile_expert;
-    int expert_rows;
-    float limit, alpha;       // kClamped
 };
 
 // One element of a gated epilogue, from the two products as T rounds them.
 template <int EPI>
-__device__ __forceinline__ float gated_value(float g, float u, float limit, float alpha) {
-    if constexpr (EPI == kClamped) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return __fdividef(g, 1.f + __expf(-alpha * g)) * (u + 1.f);
-    } else if constexpr (EPI == kGeglu) {
+__device__ __forceinline__ float gated_value(float g, float u) {
+    if constexpr (EPI == kGeglu) {
         // z / 2 (1 + tanh(s)) = z sigmoid(2 s)
         const float s = 0.7978845608028654f * (g + 0.044715f * g * g * g);
         return __fdividef(g, 1.f + __expf(-2.f * s)) * u;
@@ -138,12 +124,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
                 int m0, n0;
                 tile_origin(t, p, OUT_COLS, m0, n0);
-                int w0 = 0;                            // first row of this tile's expert in W
-                if (p.tile_expert != nullptr) {
-                    const int e = p.tile_expert[m0 / kBM];
-                    if (e < 0) continue;
-                    w0 = e * p.expert_rows;
-                }
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES) mbar_wait(empty + s, ((it / STAGES) - 1) & 1, p.err);
@@ -151,23 +131,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     unsigned char* b_dst = a_dst + L::kABytes;
                     mbar_expect_tx(full + s, L::kStageBytes);
                     tma_load_2d(a_dst, &map_a, full + s, kb * kBK, m0);
-                    tma_load_2d(b_dst, &map_w, full + s, kb * kBK, w0 + n0);
-                    if constexpr (SWIGLU) tma_load_2d(b_dst + 128 * kBK * 2, &map_w, full + s, kb * kBK, w0 + p.n_out + n0);
-                    else if constexpr (BN == 256) tma_load_2d(b_dst + 128 * kBK * 2, &map_w, full + s, kb * kBK, w0 + n0 + 128);
+                    tma_load_2d(b_dst, &map_w, full + s, kb * kBK, n0);
+                    if constexpr (SWIGLU) tma_load_2d(b_dst + 128 * kBK * 2, &map_w, full + s, kb * kBK, p.n_out + n0);
+                    else if constexpr (BN == 256) tma_load_2d(b_dst + 128 * kBK * 2, &map_w, full + s, kb * kBK, n0 + 128);
                 }
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {                               // ---- tensor-core issue ----
             constexpr uint32_t idesc = idesc_bf16(kBM, BN, false);
-            int it = 0, i = -1;
-            for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
-                if (p.tile_expert != nullptr) {
-                    int m0, n0;
-                    tile_origin(t, p, SWIGLU ? BN / 2 : BN, m0, n0);
-                    if (p.tile_expert[m0 / kBM] < 0) continue;
-                }
-                ++i;
+            int it = 0, i = 0;
+            for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++i) {
                 const int buf = i & 1, use = i >> 1;
                 if (use > 0) {                         // the epilogue of the tile before last has drained this accumulator
                     mbar_wait(acc_free + buf, (use - 1) & 1, p.err);
@@ -196,12 +170,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // at the matrix's edges.  Two boxes per warp, so that one is stored while the next is filled.
         const int quarter = warp & 3;
         unsigned char* boxes = staging + (warp - 2) * (2 * kBoxBytes);
-        int i = -1, n_box = 0;
-        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x) {
+        int i = 0, n_box = 0;
+        for (int t = blockIdx.x; t < p.num_tiles; t += gridDim.x, ++i) {
             int m0, n0;
             tile_origin(t, p, OUT_COLS, m0, n0);
-            if (p.tile_expert != nullptr && p.tile_expert[m0 / kBM] < 0) continue;
-            ++i;
             const int buf = i & 1, use = i >> 1;
             const int row = m0 + quarter * 32 + lane;
             const uint32_t tmem_d = tmem_base + buf * BN + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -235,8 +207,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 const float g0 = rnd<__nv_bfloat16>(y0), g1 = rnd<__nv_bfloat16>(y1);
                                 const float u0 = rnd<__nv_bfloat16>(__uint_as_float(u[j + 2 * k]));
                                 const float u1 = rnd<__nv_bfloat16>(__uint_as_float(u[j + 2 * k + 1]));
-                                y0 = gated_value<EPI>(g0, u0, p.limit, p.alpha);
-                                y1 = gated_value<EPI>(g1, u1, p.limit, p.alpha);
+                                y0 = gated_value<EPI>(g0, u0);
+                                y1 = gated_value<EPI>(g1, u1);
                             }
                             if constexpr (EPI == kRelu2) {
                                 y0 = fmaxf(rnd<__nv_bfloat16>(y0), 0.f); y0 *= y0;
@@ -344,38 +316,4 @@ extern "C" int cvb_gemm_bf16_tcgen05(void* out, const void* a, const void* w, co
     if (mode == 2) return tile_n == 256 ? launch_gemm<256, 4, kAddResidual>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kAddResidual>(ma, mw, mo, p, stream);
     if (mode == 3) return tile_n == 256 ? launch_gemm<256, 4, kRelu2>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kRelu2>(ma, mw, mo, p, stream);
     return CVB_E_SHAPE;
-}
-
-// The grouped form: A [M, K] holds the rows of E experts in segments that start on multiples of 128 rows; row tile i
-// belongs to expert tile_expert[i] (device memory, negative: no rows); W [E * N, K] holds the experts' matrices one below
-// the other.  mode 0: C[M, N] = A W_e^T per tile;  mode 1: C[M, N / 2] = silu(A Wg_e^T) * (A Wu_e^T), W_e = [Wg_e; Wu_e];
-// mode 3: C[M, N] = relu(A W_e^T)^2;  mode 4: like 1 with the clamped activation of `limit` and `alpha`.
-extern "C" int cvb_gemm_grouped_bf16_tcgen05(void* out, const void* a, const void* w, const int* tile_expert, int M, int N, int E,
-                                             int K, int mode, int tile_n, float limit, float alpha, int* err_flag, cudaStream_t stream) {
-    if (M == 0) return CVB_OK;
-    if (M < 0 || N <= 0 || K <= 0 || E <= 0 || tile_expert == nullptr) return CVB_E_SIZE;
-    if (K % 8 || M % kBM) return CVB_E_ALIGN;
-    auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-    if (!al(out) || !al(a) || !al(w)) return CVB_E_ALIGN;
-    if (mode != 0 && mode != 1 && mode != 3 && mode != 4) return CVB_E_SHAPE;
-    const bool gated = mode == 1 || mode == 4;
-    if (gated && (N % 2)) return CVB_E_SHAPE;
-    if (static_cast<int64_t>(E) * N > 2147483647LL) return CVB_E_SIZE;
-    GemmParams p{};
-    p.out = (__nv_bfloat16*)out; p.resid = nullptr; p.M = M; p.N = N; p.K = K;
-    p.n_out = gated ? N / 2 : N; p.err = err_flag;
-    p.limit = limit; p.alpha = alpha;
-    p.tile_expert = tile_expert; p.expert_rows = N;
-    if (p.n_out % 8) return CVB_E_ALIGN;
-    CUtensorMap ma, mw, mo;
-    int rc = matrix_map(&ma, a, M, K);
-    if (rc != CVB_OK) return rc;
-    rc = matrix_map(&mw, w, static_cast<int64_t>(E) * N, K);
-    if (rc != CVB_OK) return rc;
-    rc = cached_bf16_map(&mo, out, M, p.n_out, 64, 32);
-    if (rc != CVB_OK) return rc;
-    if (mode == 1) return launch_gemm<256, 4, kSwiglu>(ma, mw, mo, p, stream);
-    if (mode == 4) return launch_gemm<256, 4, kClamped>(ma, mw, mo, p, stream);
-    if (mode == 3) return tile_n == 256 ? launch_gemm<256, 4, kRelu2>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kRelu2>(ma, mw, mo, p, stream);
-    return tile_n == 256 ? launch_gemm<256, 4, kPlain>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kPlain>(ma, mw, mo, p, stream);
 }

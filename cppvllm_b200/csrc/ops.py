@@ -12,7 +12,7 @@ import math
 import os
 import sys
 from ctypes import c_int, c_int64, c_float, c_void_p
-from typing import Dict, Optional
+from typing import Dict, Optional, Tuple
 
 import torch
 
@@ -1427,7 +1427,7 @@ def _moe_lib():
     global _moe
     if _moe is None:
         lib = load_library("moe")
-        for name in ("cvb_route_topk", "cvb_expert_rows", "cvb_sort_pairs_padded", "cvb_combine_pairs_bf16"):
+        for name in ("cvb_route_topk", "cvb_expert_rows", "cvb_sort_pairs", "cvb_scatter_pairs_scaled_bf16", "cvb_combine_pairs_bf16"):
             getattr(lib, name).restype = c_int
         _moe = lib
     return _moe
@@ -1500,60 +1500,70 @@ def experts_grouped_supported(x_dtype: torch.dtype, D: int, F: int) -> bool:
 
 
 def grouped_rows_tcgen05(num_tokens: int, top: int, num_experts: int) -> int:
-    """Rows of scratch the tcgen05 grouped path needs: every expert's segment starts on a multiple of 128 rows."""
+    """Rows of scratch the tcgen05 grouped path asks for (a few more than the pairs; segments lie one behind the other)."""
     return ((num_tokens * top + 127) // 128 + num_experts) * 128
+
+
+GROUPED_TILE = 256          # pairs of a tile at most: an accumulator's columns.  Smaller tiles were slower at every size measured
+#                             (8 experts of 151 MB, 2,048 tokens: 256 pairs 557 us, 192 632, 128 775)
+
+
+def grouped_blocks(K: int) -> int:
+    """Blocks that share a tile of a grouped product with inner size K: a pair of SMs halves what comes in from the L2 and takes
+    twice the weight rows a tile, which pays where a tile lasts long enough.  Measured on a B200 (8 experts, 16 to 2,048 tokens, two
+    blocks against one): K 4,096 with 12,288 rows 199 / 207 us (16 tokens), 182 / 192 (600), 328 / 344 (2,048), K 6,144 with 4,096
+    rows 98 / 101, 107 / 110, 217 / 232;  K 1,024 with 3,072 rows 16.0 / 14.2, 20.2 / 18.7, 35.3 / 34.5, K 1,536 with 1,024 rows
+    19.1 / 17.0, 22.3 / 21.1, 31.8 / 32.3."""
+    return 2 if K >= 2048 else 1
+
+
+_gemm_experts = None
 
 
 def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, row_token, slot_of, xs, hid, rows,
                             activation: str = "silu", weight_on_input: bool = False, identity: int = 0, limit: float = 0.0,
-                            alpha: float = 1.702) -> torch.Tensor:
-    """More tokens on the tcgen05 tensor cores: the pairs are sorted by expert into segments that start on multiples of
-    128 rows (device side), the tokens' rows are gathered into that order, and two grouped products (the first with the
-    gated activation as its epilogue) run on csrc/gemm_tcgen05.cu's kernel; the last kernel adds a token's expert outputs
-    up with its weights.  Scratch: R = grouped_rows_tcgen05(T, top, E) rows: tile_expert int32 [R / 128], row_token int32 [R],
-    slot_of int32 [T * top], xs bf16 [R, D], hid bf16 [R, ff], rows bf16 [R, D]."""
-    global _gemm
+                            alpha: float = 1.702, tile: Optional[Tuple[int, int]] = None) -> torch.Tensor:
+    """More tokens on the tcgen05 tensor cores: the pairs are sorted by expert (device side), the tokens' rows are gathered into
+    that order, and two grouped products (the first with the gated activation as its epilogue) run on
+    csrc/gemm_experts_tcgen05.cu's kernel; the last kernel adds a token's expert outputs up with its weights.  Scratch:
+    R = grouped_rows_tcgen05(T, top, E) rows: tile_expert int32 [R / 128], row_token int32 [R] (the pairs' tokens, then the experts'
+    segments), slot_of int32 [T * top], xs bf16 [R, D], hid bf16 [R, ff], rows bf16 [R, D].  `tile` fixes (GROUPED_TILE, grouped_blocks)."""
+    global _gemm_experts
     _cuda(y, x, ids, weights, w_gate_up, w_down, tile_expert, row_token, slot_of, xs, hid, rows)
     _contig(y, x, ids, weights, w_gate_up, w_down, tile_expert, row_token, slot_of, xs, hid, rows)
     T, D = x.shape
     E, F2, _ = w_gate_up.shape
     gated = _expert_gated(activation, identity, weight_on_input)
     F, top = (F2 // 2 if gated else F2), ids.shape[1]
-    R = grouped_rows_tcgen05(T, top, E)
+    P, R = T * top, grouped_rows_tcgen05(T, top, E)
     bf = torch.bfloat16
     if (any(t.dtype != bf for t in (y, x, w_gate_up, w_down, xs, hid, rows)) or y.shape != x.shape or w_gate_up.shape != (E, F2, D)
             or w_down.shape != (E, D, F) or ids.dtype != torch.int32 or weights.dtype != torch.float32 or ids.shape != weights.shape
             or any(t.dtype != torch.int32 for t in (tile_expert, row_token, slot_of)) or tile_expert.numel() < R // 128
-            or row_token.numel() < R or slot_of.numel() < T * top or xs.numel() < R * D or hid.numel() < R * F or rows.numel() < R * D):
+            or row_token.numel() < R or slot_of.numel() < P or xs.numel() < R * D or hid.numel() < R * F or rows.numel() < R * D):
         raise KernelError("experts_grouped_tcgen05: bf16 x, y, weights and scratch of the documented sizes; int32 index scratch")
-    if _gemm is None:
-        lib = load_library("gemm_bf16")
-        lib.cvb_gemm_bf16_tcgen05.restype = c_int
-        _gemm = lib
-    _gemm.cvb_gemm_grouped_bf16_tcgen05.restype = c_int
+    if _gemm_experts is None:
+        lib = load_library("gemm_experts")
+        lib.cvb_gemm_experts_bf16.restype = c_int
+        _gemm_experts = lib
     err = _ptr(error_flag(x.device))
-    _check(_moe_lib().cvb_sort_pairs_padded(_ptr(tile_expert), _ptr(row_token), _ptr(slot_of), _ptr(ids), c_int(T), c_int(E), c_int(top),
-                                            c_int(R // 128), c_int(identity), err, _stream()), "sort_pairs_padded")
-    xs2, hid2, rows2 = xs.view(-1)[:R * D].view(R, D), hid.view(-1)[:R * F].view(R, F), rows.view(-1)[:R * D].view(R, D)
-    if weight_on_input:     # a pair's weight scales its row on the way in; the rows behind a segment keep what they held (finite)
-        _moe_lib().cvb_scatter_pairs_scaled_bf16.restype = c_int
+    tile_pairs = tile[0] if tile is not None else GROUPED_TILE
+    row_of = row_token.view(-1)[:P]
+    segments = row_token.view(-1)[P:P + 2 * (E + 1)]          # R is larger than P by 128 entries an expert or more
+    _check(_moe_lib().cvb_sort_pairs(_ptr(segments), _ptr(row_of), _ptr(slot_of), _ptr(ids), c_int(T), c_int(E), c_int(top), c_int(tile_pairs),
+                                     c_int(identity), err, _stream()), "sort_pairs")
+    xs2, hid2, rows2 = xs.view(-1)[:P * D].view(P, D), hid.view(-1)[:P * F].view(P, F), rows.view(-1)[:P * D].view(P, D)
+    if weight_on_input:     # a pair's weight scales its row on the way in
         _check(_moe_lib().cvb_scatter_pairs_scaled_bf16(_ptr(xs2), _ptr(x), _ptr(slot_of), _ptr(weights), c_int(T), c_int(D), c_int(top),
                                                         _stream()), "scatter_pairs_scaled")
     else:
-        gather_rows(xs2, x, row_token.view(-1)[:R])
-    if gated:
-        _check(_gemm.cvb_gemm_grouped_bf16_tcgen05(_ptr(hid2), _ptr(xs2), _ptr(w_gate_up), _ptr(tile_expert), c_int(R), c_int(2 * F), c_int(E),
-                                                   c_int(D), c_int(4 if activation == "clamped" else 1), c_int(256), c_float(limit), c_float(alpha),
-                                                   err, _stream()), "gemm_grouped_bf16_tcgen05")
-    else:           # the squared relu is the epilogue
-        up_256 = (T * top // 128 + 1) * ((F + 255) // 256)
-        _check(_gemm.cvb_gemm_grouped_bf16_tcgen05(_ptr(hid2), _ptr(xs2), _ptr(w_gate_up), _ptr(tile_expert), c_int(R), c_int(F), c_int(E),
-                                                   c_int(D), c_int(3), c_int(256 if up_256 >= 120 else 128), c_float(0.0), c_float(0.0), err, _stream()),
-               "gemm_grouped_bf16_tcgen05")
-    tiles_256 = (T * top // 128 + 1) * ((D + 255) // 256)
-    _check(_gemm.cvb_gemm_grouped_bf16_tcgen05(_ptr(rows2), _ptr(hid2), _ptr(w_down), _ptr(tile_expert), c_int(R), c_int(D), c_int(E),
-                                               c_int(F), c_int(0), c_int(256 if tiles_256 >= 120 else 128), c_float(0.0), c_float(0.0), err, _stream()),
-           "gemm_grouped_bf16_tcgen05")
+        gather_rows(xs2, x, row_of)
+
+    def product(out, a, w, n, k, mode):
+        _check(_gemm_experts.cvb_gemm_experts_bf16(_ptr(out), _ptr(a), _ptr(w), _ptr(segments), c_int(P), c_int(n), c_int(E), c_int(k), c_int(mode),
+                                                   c_int(tile_pairs), c_int(tile[1] if tile is not None else grouped_blocks(k)), c_float(limit), c_float(alpha), err, _stream()), "gemm_experts_bf16")
+    product(hid2, xs2, w_gate_up, F2, D, (4 if activation == "clamped" else 1) if gated else 3)
+    product(rows2, hid2, w_down, D, F, 0)
     _check(_moe_lib().cvb_combine_pairs_bf16(_ptr(y), _ptr(rows2), _ptr(x), _ptr(slot_of), _ptr(None if weight_on_input else weights), c_int(T),
                                              c_int(D), c_int(top), _stream()),
            "combine_pairs")

@@ -1,0 +1,62 @@
+"""The grouped products of the experts at the edges of their tiles, against the same layer in float64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# rows per expert: none, one, around multiples of 16, 32 and the largest tile
+COUNTS = {"edges": [0, 1, 15, 16, 17, 31, 32, 33, 0, 63, 64, 65], "tiles": [255, 256, 257, 0, 513, 5], "one": [0, 0, 3, 0]}
+BF = torch.bfloat16
+
+
+def _layer(x, ids, wts, wgu, wd, act, limit, alpha):
+    """Rounded where the kernels round: both products, the activation and the sum."""
+    T, D = x.shape
+    y = torch.zeros(T, D, dtype=torch.float64, device=x.device)
+    for k in range(ids.shape[1]):
+        for e in range(wgu.shape[0]):
+            t = (ids[:, k] == e).nonzero()[:, 0]
+            if not len(t):
+                continue
+            h = (x[t].double() @ wgu[e].double().T).to(BF).double()
+            if act == "relu2":
+                h = torch.relu(h) ** 2
+            else:
+                g, u = h.chunk(2, -1)
+                if act == "clamped":
+                    g, u = g.clamp(max=limit), u.clamp(-limit, limit)
+                    h = g * torch.sigmoid(alpha * g) * (u + 1)
+                else:
+                    h = (g * torch.sigmoid(g)).to(BF).double() * u
+            y[t] += wts[t, k].double()[:, None] * (h.to(BF).double() @ wd[e].double().T).to(BF).double()
+    return y
+
+
+@pytest.mark.parametrize("counts", sorted(COUNTS))
+@pytest.mark.parametrize("act,D,F", [("silu", 136, 200), ("silu", 512, 256), ("relu2", 72, 264), ("clamped", 128, 72)])
+@pytest.mark.parametrize("tile", [(256, 2), (256, 1), (64, 2), (32, 1)])
+def test_expert_products_at_tile_edges(counts, act, D, F, tile):
+    from cppvllm_b200.csrc import ops
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(hash((D, F)) % 1000)
+    sizes = COUNTS[counts]
+    E, T = len(sizes), sum(sizes)
+    one = torch.cat([torch.full((n,), e) for e, n in enumerate(sizes)])[torch.randperm(T, generator=g)]
+    ids = torch.stack([one, (one + 1) % E], 1).to(torch.int32)               # the second choice shifts every count by one expert
+    wts = torch.rand(T, 2, generator=g)
+    x = torch.randn(T, D, generator=g).to(BF)
+    wgu = (torch.randn(E, F if act == "relu2" else 2 * F, D, generator=g) * D ** -0.5).to(BF)
+    wd = (torch.randn(E, D, F, generator=g) * F ** -0.5).to(BF)
+    x, ids, wts, wgu, wd = (t.to(dev) for t in (x, ids, wts, wgu, wd))
+    R = ops.grouped_rows_tcgen05(T, 2, E)
+    ints = dict(dtype=torch.int32, device=dev)
+    scratch = [torch.full((n, m), float("nan"), dtype=BF, device=dev) for n, m in ((R, D), (R, F), (R, D))]
+    y = torch.empty(T, D, dtype=BF, device=dev)
+    ops.experts_grouped_tcgen05(y, x, ids, wts, wgu, wd, torch.empty(R // 128, **ints), torch.empty(R, **ints), torch.empty(T * 2, **ints), *scratch,
+                                activation=act, limit=2.0, alpha=1.702, tile=tile)
+    ops.check_device_errors(dev)
+    ref = _layer(x, ids, wts, wgu, wd, act, 2.0, 1.702)
+    # an intermediate may round the other way (float sums of up to 512 products against float64): one unit of bf16, 2^-8, on some of a row's
+    # terms, and the last rounding; 2^-6 of the row's largest value covers both
+    err = (y.double() - ref).abs().amax(1) / ref.abs().amax(1).clamp(min=1e-3)
+    assert float(err.max()) < 2.0 ** -6, float(err.max())
