@@ -37,6 +37,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "gemv_bf16": ["gemv_bf16.cu"],
     "gemm_bf16": ["gemm_tcgen05.cu"],
     "gemm_experts": ["gemm_experts_tcgen05.cu"],
+    "gemm_f32": ["gemm_f32_tcgen05.cu"],
     "attn_tcgen05": ["attention_tcgen05.cu"],
     "attn_f32": ["attention_f32.cu"],
     "attn_entries": ["attention_entries_tcgen05.cu"],

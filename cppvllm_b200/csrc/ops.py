@@ -2406,7 +2406,7 @@ def project_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows:
     if gemv_stream_supported(x.dtype, weight, rows):
         return gemv_stream_bf16(out, x, weight, rows, dependent=dependent)
     if rows > GEMV_MAX_ROWS or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
-        return linear(x, weight, out=out)
+        return gemm_f32_split(out, x, weight) if gemm_f32_split_supported(x, weight, out) else linear(x, weight, out=out)
     key = (weight.shape[0], weight.shape[1], rows if rows <= 2 else (8 if rows <= 8 else 16))
     choice = _project_choice.get(key)
     if choice is None:
@@ -2525,6 +2525,63 @@ def feed_tokens(tokens: torch.Tensor, src: torch.Tensor, sampled: torch.Tensor, 
     _check(core().cvb_feed_tokens(_ptr(tokens), _ptr(src), _ptr(sampled), c_int(n), c_int(sampled.numel()), _stream()),
            "feed_tokens")
     return tokens
+
+
+# ---- float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) --------------------------------------------
+
+_gemm_f32 = None
+# From 17 rows and 128 of K on the error is smaller than the library's at every size measured (128 to 4,096 outputs, 17 to 512 rows, K 128 to
+# 3,072: 1.1e-7 to 1.9e-7 where the library's is 2.0e-7 to 9.9e-7); for 16 rows and fewer, and a short K, the library adds in shorter chains
+# (16 x 128 x 256: 1.0e-7, here 1.2e-7;  K 64: 8.6e-8, here 1.1e-7).
+SPLIT_MIN_ROWS, SPLIT_MIN_K = 17, 128
+SPLIT_STAGE = {32: 1.1, 64: 1.25, 96: 1.5, 128: 1.75}       # us per 64 of K for a block of so many rows of x (measured, 40 to 148 blocks)
+SPLIT_FIXED = 6.0                                           # us a block otherwise
+SPLIT_BLOCKS = {1: 148, 2: 148, 4: 136, 8: 112}             # blocks at once in clusters of 1, 2, 4, 8 (a cluster lies in one group of SMs)
+
+
+def split_tile(rows: int, n_out: int, k: int) -> Tuple[int, int]:
+    """(rows of x a block of the split product takes, blocks that share a tile's K): the choice whose waves of blocks take the
+    shortest time by the figures above.  Measured on a B200, us with (rows, blocks): 449 x 1,024 x 2,048 (128, 1) 57, (128, 4) 21,
+    (64, 2) 29, (64, 8) 53;  64 x 1,024 x 2,048 (64, 1) 47, (64, 8) 11;  200 x 4,096 x 1,024 (128, 1) 33, (128, 2) 22, (64, 1) 28;
+    449 x 4,096 x 1,024 (128, 1) 34, (128, 2) 43, (64, 1) 55."""
+    stages, best = -(-k // 64), None
+    for tile, us in SPLIT_STAGE.items():
+        tiles = -(-n_out // 128) * -(-rows // tile)
+        for parts, blocks in SPLIT_BLOCKS.items():
+            if parts > stages:
+                break
+            cost = -(-tiles * parts // blocks) * (SPLIT_FIXED + -(-stages // parts) * us)
+            if best is None or cost < best[0]:
+                best = (cost, tile, parts)
+    return best[1], best[2]
+
+
+def gemm_f32_split_supported(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether a float32 product goes through the tensor cores.  Against the library's float32 product on a B200 (us): 32 rows by
+    4,096 x 1,024 10 / 21, by 1,024 x 2,048 10 / 22;  64: 10 / 24 and 10 / 37;  200: 22 / 47 and 15 / 42;  449: 33 / 87 and 21 / 57;
+    600: 59 / 124 and 31 / 88;  2,048 by 4,096 x 1,024 128 / 330."""
+    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32 and x.shape[0] >= SPLIT_MIN_ROWS
+            and x.shape[1] >= SPLIT_MIN_K and x.shape[1] % 4 == 0 and max(x.numel(), weight.numel()) < 1 << 30 and x.is_contiguous() and weight.is_contiguous() and out.is_contiguous()
+            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
+
+
+def gemm_f32_split(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, tile: Optional[Tuple[int, int]] = None) -> torch.Tensor:
+    """out = x @ weight^T, all float32, with products of bf16 parts and float sums that are no further from float64 than a float32
+    product's.  `tile` fixes split_tile's choice."""
+    global _gemm_f32
+    if _gemm_f32 is None:
+        lib = load_library("gemm_f32")
+        lib.cvb_gemm_f32_split.restype = c_int
+        _gemm_f32 = lib
+    _cuda(out, x, weight); _contig(out, x, weight)
+    M, K = x.shape
+    N = weight.shape[0]
+    if any(t.dtype != torch.float32 for t in (out, x, weight)) or weight.shape[1] != K or out.shape != (M, N):
+        raise KernelError("gemm_f32_split: x [M, K], weight [N, K], out [M, N], all float32")
+    rows, parts = tile if tile is not None else split_tile(M, N, K)
+    _check(_gemm_f32.cvb_gemm_f32_split(_ptr(out), _ptr(x), _ptr(weight), c_int(M), c_int(N), c_int(K), c_int(rows), c_int(parts),
+                                        _ptr(error_flag(x.device)), _stream()), "gemm_f32_split")
+    return out
 
 
 # ---- library matrix products ---------------------------------------------------------------------------------

@@ -1,0 +1,59 @@
+"""The float32 product on the tensor cores: edges of its tiles and stages, its error beside the library's, values without parts."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# around the rows of a block, the columns of a block and the 64 of K of a stage
+SHAPES = [(1, 4, 4), (16, 128, 64), (31, 100, 60), (33, 130, 68), (65, 1, 128), (96, 257, 132), (127, 300, 516), (129, 96, 1024), (200, 640, 196)]
+
+
+def _run(ops, x, w, tile=None):
+    out = torch.full((x.shape[0], w.shape[0]), float("nan"), device=x.device)
+    ops.gemm_f32_split(out, x, w, tile=tile)
+    ops.check_device_errors(x.device)
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", SHAPES)
+@pytest.mark.parametrize("rows", [32, 64, 96, 128])
+@pytest.mark.parametrize("parts", [1, 2, 4, 8])
+def test_edges(M, N, K, rows, parts):
+    from cppvllm_b200.csrc import ops
+    if parts > -(-K // 64):
+        pytest.skip("fewer stages than parts")
+    g = torch.Generator().manual_seed(M * 1000 + N)
+    x, w = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    out = _run(ops, x, w, (rows, parts))
+    ref, mag = x.double() @ w.double().T, x.abs().double() @ w.abs().double().T
+    # 2^-23 of every product for the parts left out; at most 9 truncated additions in tensor memory (128 of K by 16), 2^-23 each; as many
+    # rounded additions as there are groups of 128 of K and parts, 2^-24 each
+    bound = (1 + 9 + (K // 128 + 1 + parts) / 2) * 2.0 ** -23 * mag + 1e-37
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 1024, 128), (33, 512, 320), (100, 256, 256), (17, 4096, 1024), (449, 1024, 2048), (300, 4096, 1024)])
+def test_error_no_larger_than_the_library(M, N, K):
+    from cppvllm_b200.csrc import ops
+    ops.configure_library_matmul()
+    g = torch.Generator().manual_seed(5)
+    x, w = torch.randn(M, K, generator=g).cuda(), (torch.randn(N, K, generator=g) * 0.02).cuda()
+    ref = x.double() @ w.double().T
+    ours, lib = ((y.double() - ref).norm() / ref.norm() for y in (_run(ops, x, w), torch.mm(x, w.T)))
+    assert float(ours) <= float(lib), (float(ours), float(lib))
+
+
+@pytest.mark.parametrize("tile", [(32, 1), (64, 2), (128, 1)])
+def test_infinities_and_nan(tile):
+    """A row with a value that has no parts gives what float sums give; the other rows do not see it."""
+    from cppvllm_b200.csrc import ops
+    g = torch.Generator().manual_seed(7)
+    x, w = torch.randn(40, 192, generator=g).cuda(), torch.randn(70, 192, generator=g).cuda()
+    clean = _run(ops, x, w, tile)
+    x[3, 5], x[17, 191], x[30, 64], x[39, 0] = float("inf"), float("-inf"), float("nan"), 3.4e38
+    out, ref = _run(ops, x, w, tile), x.double() @ w.double().T
+    assert bool(torch.isnan(out[30]).all()) and torch.equal(torch.isinf(out[3]), torch.isinf(ref[3])) and torch.equal(out[17].double(), ref[17])
+    big = ref[39].abs() < 3.4e38
+    assert bool(torch.isfinite(out[39][big]).all())
+    rest = [i for i in range(40) if i not in (3, 17, 30, 39)]
+    assert torch.equal(out[rest], clean[rest])
