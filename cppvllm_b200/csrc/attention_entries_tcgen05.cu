@@ -7,17 +7,21 @@
 // What bounds the mma.sync kernels is the legacy tensor path and the shared-memory reads that feed it: 64 query rows per block and
 // 64 keys per tile, every operand fragment through ldmatrix.  Here a block owns 256 query rows of one kv head as two tiles of 128 (row r
 // of a tile = token r / g, head r % g of the group), walks tiles of 128 entries, and the tensor core alternates between the two query
-// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, before -> now): chunks of 1,024 179 -> 29; a latent of
-// 96 + 32 under 16 heads 171 -> 43; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 47; keys that are values at 32/8 heads
-// (1,917 tokens of three requests behind a window of 1,024) 196 -> 51.
+// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, mma.sync -> now): chunks of 1,024 179 -> 26; a latent of
+// 96 + 32 under 16 heads 171 -> 37; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 45; keys that are values at 32/8 heads
+// (1,917 tokens of three requests behind a window of 1,024) 196 -> 44.
 //   warp 0     producer: one lane per TMA box (page or 64 entries, times 64 columns, times key and value), 128-byte swizzle.  Key and
 //              value apart: two stages, each with the keys of tile i + 1 and the values of tile i (what one round reads).  Shared
 //              entries: four stages of one tile, read row-wise by S = Q K^T and transposed by O += P K;
-//   warp 1     allocates 512 columns of tensor memory and issues the products: P_i V_i, then S_{i+1}, for either query tile;
+//   warp 1     allocates 512 columns of tensor memory and issues the products: P_i V_i in two halves as P is handed over, then S_{i+1},
+//              for either query tile; the whole warp walks the list with values that are the same in all lanes and one lane issues (the
+//              four cases above: 29.5, 44.6, 48.1, 50.8 from one thread's branch, 28.7, 42.3, 44.6, 47.5 so);
 //   warps 4-11 softmax, one thread per query row: S from tensor memory, scale, cap, term by distance, mask, exponentials, P back over
 //              S; O is rescaled in tensor memory when some row of the warp has a new maximum.  The reference is the maximum itself, so that a row's
 //              largest probability is 1 and rounds to 1: with one that followed only after 2^8, layers were 1 to 5 % further from float64 (capped
 //              scores 4.00e-3 -> 4.22e-3, a bias per distance 4.82e-3 -> 4.90e-3) and 2 to 5 % faster (a bias per distance 79 us against 83).
+//              Without a cap or a distance term one exponential in three is made on the multiply-add units (27.7, 41.2, -, 46.3); with
+//              them those units have no room.
 // The tiles a block walks are a list: pooled blocks any of its tokens sees (plane 1), kept first tokens that lie wholly before the
 // rest, then the tokens from the first one its first token sees to its last token; a query tile skips list entries it sees nothing of.
 //   distance terms: bias[h, min(p - j, L - 1)] or -r1_h ln(1 + r2_h (p - j)) come from a table in shared memory, one row per head of
@@ -110,7 +114,7 @@ __device__ __forceinline__ int entry_find_block(const EntryAttnParams& p, int bl
 template <int HD>
 struct EntrySmem {
     static constexpr int kTile = 128 * HD * 2;
-    static constexpr int kNumBars = 4 + 4 + 2 + 2 + 2;
+    static constexpr int kNumBars = 4 + 4 + 2 + 4 + 2;
     static constexpr size_t kBytes = static_cast<size_t>(kTile) * 6 + kNumBars * 8 + 16;      // and the distance table behind it
 };
 
@@ -147,12 +151,12 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
     uint64_t* kv_full = bars;                      // TMA: what the stage holds has landed
     uint64_t* kv_empty = kv_full + 4;              // tensor core: the products that read the stage are done
     uint64_t* s_ready = kv_empty + 4;              // [2 query tiles]  tensor core: S(X) and everything issued before it is done
-    uint64_t* p_ready = s_ready + 2;               // [2 query tiles]  128 softmax threads: P(X) is in tensor memory
-    uint64_t* o_done = p_ready + 2;                // [2 query tiles]  tensor core: the last PV(X) is done
+    uint64_t* p_ready = s_ready + 2;               // [2 query tiles][2 halves of the tile's entries]  128 softmax threads: P(X) is in tensor memory
+    uint64_t* o_done = p_ready + 4;                // [2 query tiles]  tensor core: the last PV(X) is done
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
     float* sT = reinterpret_cast<float*>(tmem_slot + 4);            // distance table [g][table_stride]
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = same_in_warp(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int g = p.H / p.G;
     const int tok_per_tile = kEM / g;
     const int tok_per_block = 2 * tok_per_tile;
@@ -218,7 +222,8 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
     if (warp == 0) {
         if (lane == 0) {
             for (int i = 0; i < 4; ++i) { mbar_init(kv_full + i, 1); mbar_init(kv_empty + i, 1); }
-            for (int i = 0; i < 2; ++i) { mbar_init(s_ready + i, 1); mbar_init(p_ready + i, 128); mbar_init(o_done + i, 1); }
+            for (int i = 0; i < 2; ++i) { mbar_init(s_ready + i, 1); mbar_init(o_done + i, 1); }
+            for (int i = 0; i < 4; ++i) mbar_init(p_ready + i, 128);
             mbar_fence_init();
         }
         __syncwarp();
@@ -311,45 +316,63 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {                             // ---- tensor-core issue ----
-            constexpr uint32_t idesc_s = idesc_bf16(kEM, kEN, false);
-            constexpr uint32_t idesc_pv = idesc_bf16(kEM, HD, true);
-            auto issue_s = [&](int x, int i) {       // S(X) of list entry it_lo + i; its stage has been waited for
-                const uint32_t q_addr = smem_u32(sQ + x * L::kTile), k_addr = smem_u32(entry_tile(i, false));
+        // ---- tensor-core issue: the whole warp walks the list with values that are the same in all lanes, one lane issues ----
+        constexpr uint32_t idesc_s = idesc_bf16(kEM, kEN, false);
+        constexpr uint32_t idesc_pv = idesc_bf16(kEM, HD, true);
+        constexpr uint32_t kTileStep = L::kTile >> 4;                         // in units of a descriptor's address
+        const uint64_t q_desc = desc_sw128(smem_u32(sQ), 16, 1024), v_desc = desc_sw128(smem_u32(sKV), 16384, 1024);
+        const uint32_t q_lo = static_cast<uint32_t>(q_desc), k_lo = static_cast<uint32_t>(desc_sw128(smem_u32(sKV), 16, 1024));
+        const uint32_t v_lo = static_cast<uint32_t>(v_desc), k_hi = static_cast<uint32_t>(q_desc >> 32), v_hi = static_cast<uint32_t>(v_desc >> 32);
+        const uint32_t t0 = same_in_warp(tmem);
+        const int n = same_in_warp(n_here), end[2] = {same_in_warp(last_it[0] - it_lo), same_in_warp(last_it[1] - it_lo)};
+        auto sees = [&](int x, int i) { return __any_sync(0xffffffffu, active(x, it_lo + i)) != 0; };
+        auto issue_s = [&](int x, int i) {           // S(X) of list entry it_lo + i; its stage has been waited for
+            const uint32_t ql = q_lo + x * kTileStep, kl = k_lo + (SHARED ? i % kStages : 2 * (i % kStages)) * kTileStep;
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-                    umma(tS[x], desc_sw128(q_addr + off, 16, 1024), desc_sw128(k_addr + off, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+                    const uint32_t off = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
+                    umma(t0 + x * 128, desc_words(ql + off, k_hi), desc_words(kl + off, k_hi), idesc_s, k > 0 ? 1u : 0u);
                 }
                 tc_commit(s_ready + x);
-            };
-            int done[2] = {0, 0};                    // list entries of either query tile behind us
-            mbar_wait(kv_full + 0, 0, p.err);
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-                if (active(x, it_lo)) issue_s(x, 0);
-            if (!SHARED) tc_commit(kv_empty + 0);
-            for (int i = 0; i < n_here; ++i) {
-                const int next = i + 1, st = next % kStages;        // apart: load i + 1 brings these values and the next keys
-                if (!SHARED || next < n_here) mbar_wait(kv_full + st, (next / kStages) & 1, p.err);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const bool more = next < n_here && active(x, it_lo + next);
-                    if (active(x, it_lo + i)) {
-                        mbar_wait(p_ready + x, done[x] & 1, p.err);
-                        tc_after();
-                        const uint32_t v_addr = smem_u32(entry_tile(i, true));
-#pragma unroll
-                        for (int k = 0; k < kEN / 16; ++k)   // P: 16 entries = 8 columns of packed pairs; V: 16 entries further down
-                            umma_ts(tO[x], tS[x] + k * 8, desc_sw128(v_addr + k * 16 * 128, 16384, 1024), idesc_pv,
-                                    (done[x] > 0 || k > 0) ? 1u : 0u);
-                        ++done[x];
-                        if (it_lo + i == last_it[x]) tc_commit(o_done + x);
-                    }
-                    if (more) issue_s(x, next);
-                }
-                tc_commit(kv_empty + (SHARED ? i % kStages : st));
             }
+            __syncwarp();
+        };
+        int done[2] = {0, 0};                        // list entries of either query tile behind us
+        bool now[2] = {sees(0, 0), sees(1, 0)};
+        mbar_wait(kv_full + 0, 0, p.err);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (now[x]) issue_s(x, 0);
+        if (!SHARED && elect_one()) tc_commit(kv_empty + 0);
+        __syncwarp();
+        for (int i = 0; i < n; ++i) {
+            const int next = i + 1, st = next % kStages;        // apart: load i + 1 brings these values and the next keys
+            const bool soon[2] = {next < n && sees(0, next), next < n && sees(1, next)};
+            if (!SHARED || next < n) mbar_wait(kv_full + st, (next / kStages) & 1, p.err);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (now[x]) {
+                    const uint32_t vl = v_lo + (SHARED ? i % kStages : 2 * st + 1) * kTileStep, more = done[x] > 0 ? 1u : 0u;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {             // a half's product runs while the exponentials of the other are made
+                        mbar_wait(p_ready + 2 * x + h, done[x] & 1, p.err);
+                        tc_after();
+                        if (elect_one()) {
+#pragma unroll
+                            for (int k = h * (kEN / 32); k < (h + 1) * (kEN / 32); ++k)   // P: 16 entries = 8 columns of packed pairs; V: 16 entries further down
+                                umma_ts(t0 + 256 + x * HD, t0 + x * 128 + k * 8, desc_words(vl + k * (16 * 128 >> 4), v_hi), idesc_pv, k > 0 ? 1u : more);
+                            if (h == 1 && i == end[x]) tc_commit(o_done + x);
+                        }
+                        __syncwarp();
+                    }
+                    ++done[x];
+                }
+                if (soon[x]) issue_s(x, next);
+                now[x] = soon[x];
+            }
+            if (elect_one()) tc_commit(kv_empty + (SHARED ? i % kStages : st));
+            __syncwarp();
         }
     }
     } else {                                         // ---- softmax: one thread per query row ----
@@ -463,25 +486,6 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                         }
                     }
                 }
-                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-                const float2 scale2 = make_float2(scale_log2, scale_log2), neg_m2 = make_float2(-m_use, -m_use);
-                float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t packed[32];
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const int c = h * 64 + 2 * k;
-                        const float2 s = make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1]));
-                        const float2 arg = TERMS ? __fadd2_rn(s, neg_m2) : __ffma2_rn(s, scale2, neg_m2);
-                        const float2 pr = make_float2(ex2(arg.x), ex2(arg.y));
-                        sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
-                        __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
-                        packed[k] = *reinterpret_cast<uint32_t*>(&hh);
-                    }
-                    tm_store32(my_s + lane_base + h * 32, packed);     // P over the first 64 columns of S
-                }
-                l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
                 // Entries that no token of the block sees have probability 0, but what the page holds there (a former holder's
                 // Inf, a NaN) times 0 would be NaN: thread r clears row r of the tile the product P V reads.  (The threads of the
                 // other query tile may do the same; they write the same zeros.)
@@ -497,9 +501,28 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                     }
                     fence_async_smem();                                       // the tensor core reads through the async proxy
                 }
-                tm_wait_st();
-                tc_before();
-                mbar_arrive(p_ready + x);
+                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+                const float2 scale2 = make_float2(scale_log2, scale_log2), neg_m2 = make_float2(-m_use, -m_use);
+                float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t packed[32];
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) {
+                        const int c = h * 64 + 2 * k;
+                        const float2 s = make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1]));
+                        const float2 arg = TERMS ? __fadd2_rn(s, neg_m2) : __ffma2_rn(s, scale2, neg_m2);
+                        const float2 pr = !TERMS && k % 3 == 2 ? ex2_fma2(arg) : make_float2(ex2(arg.x), ex2(arg.y));
+                        sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
+                        __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
+                        packed[k] = *reinterpret_cast<uint32_t*>(&hh);
+                    }
+                    tm_store32(my_s + lane_base + h * 32, packed);     // P over the first 64 columns of S
+                    tm_wait_st();
+                    tc_before();
+                    mbar_arrive(p_ready + 2 * x + h);
+                }
+                l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
                 ++done;
             }
         }

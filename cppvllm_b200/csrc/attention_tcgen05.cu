@@ -10,18 +10,27 @@
 //              two stages, each with the keys of tile j + 1 and the values of tile j (what one round of the tensor core
 //              reads), so a round costs the issuing thread one wait and one commit for its operands; the block-table
 //              reads of a load are in flight together;
-//   warp 1     allocates 512 columns of tensor memory; one thread issues, per key tile j and query tile X,
+//   warp 1     allocates 512 columns of tensor memory and issues, per key tile j and query tile X,
 //                  PV_j(X)    = P_j(X) V_j        (M 128, N = head size, K 128; P from tensor memory, V MN-major)
 //                  S_{j+1}(X) = Q(X) K_{j+1}^T    (M 128, N 128, K = head size; both operands K-major)
 //              PV_j(X) accumulates into O(X) in tensor memory; P_j(X) lies over the first half of S_j(X), where the
-//              softmax threads put it, so S_{j+1}(X) follows PV_j(X) in the tensor core's queue;
+//              softmax threads put it, so S_{j+1}(X) follows PV_j(X) in the tensor core's queue.  The whole warp walks the
+//              rounds with values that are the same in all lanes and one lane issues: from one thread's branch, with
+//              descriptors built for every product, a product of 64 cycles took about 115 to issue.  P_j(X) is handed over
+//              in two halves, so that half of PV_j(X) runs beside the exponentials of the other half;
 //   warps 2-3  idle (they fill the first warpgroup, which hands its registers to the other two with setmaxnreg);
 //   warps 4-7  softmax of tile A, warps 8-11 of tile B: one thread per query row.  A thread reads its row of S (128
 //              floats) with tcgen05.ld, exponentiates against a reference maximum and writes the row of P as bf16 back
 //              into tensor memory with tcgen05.st.  The output accumulator stays in tensor memory; it is rescaled (read,
 //              multiplied, written back by the row's thread) only when the running maximum of some row of the warp has
 //              grown by more than 2^8 since the reference was set, which happens in the first tiles and then hardly
-//              ever.  The result is exact: the same reference scales P and the row sum.
+//              ever.  The result is exact: the same reference scales P and the row sum.  One exponential in three is made on the
+//              multiply-add units (ex2_fma2): all on the special-function unit, two tiles take its whole 2,048 cycles a round.
+// A tile's chain (scores, exponentials, products) sets the pace: 512 tokens behind 7,680 at 32/8 heads / a prompt of 2,048 at 16/8 heads
+// 73.4 / 39.2 us; issue by the whole warp 66.9 / 35.4; a third of the exponentials on the multiply-add units 63.9 / 33.3 (an eighth 66.1 /
+// 34.8, a quarter 64.6 / 34.0, half 68.3 / 35.4); two halves 62.2 / 32.3.  Scores by 64 keys in two buffers a tile, so that a tile's products
+// and exponentials need not wait for one another, were slower (75.6 / 38.7: products of 128 x 64 read shared memory for 48 cycles and
+// compute for 32), and so was a ring of five tiles given back one by one (the loads are not what a round waits for).
 // A grid of few query blocks with many key tiles each (a portion behind a long context) leaves SMs idle, so the launcher
 // may allow a query block's key tiles to be shared out among up to eight blocks ("pieces"); each leaves its unnormalised
 // rows, reference maxima and sums in global memory, and attn_prefill_merge_kernel adds them up in the order of the pieces.
@@ -63,7 +72,7 @@ constexpr int kTcThreads = 128 + 256;         // one warpgroup of helpers (two w
 template <int HD>
 struct TcSmem {
     static constexpr int kTile = 128 * HD * 2;
-    static constexpr int kNumBars = 2 * kStages + 2 + 2 + 2;
+    static constexpr int kNumBars = 2 * kStages + 2 + 4 + 2;
     static constexpr size_t kBytes = static_cast<size_t>(kTile) * (2 + 2 * kStages) + kNumBars * 8 + 16;
 };
 
@@ -85,11 +94,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
     uint64_t* kv_full = bars;                      // [2]  TMA: the stage's keys and values have landed
     uint64_t* kv_empty = kv_full + kStages;        // [2]  tensor core: the products that read the stage are done
     uint64_t* s_ready = kv_empty + kStages;        // [2 tiles]  tensor core: S_j(X) and everything issued before it is done
-    uint64_t* p_ready = s_ready + 2;               // [2 tiles]  128 softmax threads: P_j(X) is in tensor memory
-    uint64_t* o_done = p_ready + 2;                // [2 tiles]  tensor core: the last PV(X) is done
+    uint64_t* p_ready = s_ready + 2;               // [2 tiles][2 halves of the tile's keys]  128 softmax threads: P_j(X) is in tensor memory
+    uint64_t* o_done = p_ready + 4;                // [2 tiles]  tensor core: the last PV(X) is done
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = same_in_warp(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int g = p.H / p.KV;
     const int tok_per_tile = kTM / g;
     const int tok_per_block = 2 * tok_per_tile;
@@ -223,7 +232,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
     if (warp == 0) {
         if (lane == 0) {
             for (int i = 0; i < kStages; ++i) { mbar_init(kv_full + i, 1); mbar_init(kv_empty + i, 1); }
-            for (int i = 0; i < 2; ++i) { mbar_init(s_ready + i, 1); mbar_init(p_ready + i, 128); mbar_init(o_done + i, 1); }
+            for (int i = 0; i < 2; ++i) { mbar_init(s_ready + i, 1); mbar_init(o_done + i, 1); }
+            for (int i = 0; i < 4; ++i) mbar_init(p_ready + i, 128);
             mbar_fence_init();
         }
         __syncwarp();
@@ -273,47 +283,62 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
             if (has) tma_load_2d(sKV + (2 * st + which) * L::kTile + half * 16384 + box * p.box_rows * 128, &kv_map, kv_full + st, half * 64, row);
         }
     } else if (warp == 1) {
-        if (lane == 0) {                             // ---- tensor-core issue ----
-            constexpr uint32_t idesc_s = idesc_bf16(kTM, kTN, false);
-            constexpr uint32_t idesc_pv = idesc_bf16(kTM, HD, true);
-            auto active = [&](int x, int j) { return j >= t_lo[x] && j < t_hi[x]; };
-            auto issue_s = [&](int x, int j) {       // S_j(X); the stage with K_j has been waited for
-                const int st = (j - j_lo) % kStages;
-                const uint32_t q_addr = smem_u32(sQ + x * L::kTile), k_addr = smem_u32(sKV + 2 * st * L::kTile);
+        // ---- tensor-core issue: the whole warp walks the rounds with values that are the same in all lanes, one lane issues ----
+        constexpr uint32_t idesc_s = idesc_bf16(kTM, kTN, false);
+        constexpr uint32_t idesc_pv = idesc_bf16(kTM, HD, true);
+        constexpr uint32_t kTileStep = L::kTile >> 4;                         // in units of a descriptor's address
+        const uint64_t q_desc = desc_sw128(smem_u32(sQ), 16, 1024), v_desc = desc_sw128(smem_u32(sKV) + L::kTile, 16384, 1024);
+        const uint32_t q_lo = static_cast<uint32_t>(q_desc), k_lo = static_cast<uint32_t>(desc_sw128(smem_u32(sKV), 16, 1024));
+        const uint32_t v_lo = static_cast<uint32_t>(v_desc), k_hi = static_cast<uint32_t>(q_desc >> 32), v_hi = static_cast<uint32_t>(v_desc >> 32);
+        const uint32_t t0 = same_in_warp(tmem);
+        const int n = same_in_warp(j_hi - j_lo);
+        int first[2], last[2];                       // rounds in which a query tile has products
+#pragma unroll
+        for (int x = 0; x < 2; ++x) { first[x] = same_in_warp(t_lo[x] - j_lo); last[x] = same_in_warp(t_hi[x] - j_lo); }
+        auto active = [&](int x, int i) { return i >= first[x] && i < last[x]; };
+        auto issue_s = [&](int x, int st) {          // S(X) from the keys of stage st, which has been waited for
+            const uint32_t ql = q_lo + x * kTileStep, kl = k_lo + st * (2 * kTileStep);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < HD / 16; ++k) {
-                    const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-                    umma(tS[x], desc_sw128(q_addr + off, 16, 1024), desc_sw128(k_addr + off, 16, 1024), idesc_s, k > 0 ? 1u : 0u);
+                    const uint32_t off = (k >> 2) * (16384 >> 4) + (k & 3) * 2;
+                    umma(t0 + x * 128, desc_words(ql + off, k_hi), desc_words(kl + off, k_hi), idesc_s, k > 0 ? 1u : 0u);
                 }
                 tc_commit(s_ready + x);
-            };
-            mbar_wait(kv_full + 0, 0, p.err);        // the bytes came through the async proxy: the wait itself orders them
-#pragma unroll
-            for (int x = 0; x < 2; ++x)
-                if (active(x, j_lo)) issue_s(x, j_lo);
-            tc_commit(kv_empty + 0);
-            for (int j = j_lo; j < j_hi; ++j) {
-                const int i = j - j_lo + 1, st = i % kStages;                  // load i: V_j and K_{j+1}
-                mbar_wait(kv_full + st, (i / kStages) & 1, p.err);
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (!active(x, j)) {
-                        // a tile that starts later (window): its first S belongs to the round before its first PV
-                        if (j + 1 < j_hi && active(x, j + 1)) issue_s(x, j + 1);
-                        continue;
-                    }
-                    mbar_wait(p_ready + x, (j - t_lo[x]) & 1, p.err);
-                    tc_after();
-                    const uint32_t v_addr = smem_u32(sKV + (2 * st + 1) * L::kTile);
-#pragma unroll
-                    for (int k = 0; k < kTN / 16; ++k)   // P: 16 keys = 8 columns of packed pairs; V: 16 keys further down
-                        umma_ts(tO[x], tS[x] + k * 8, desc_sw128(v_addr + k * 16 * 128, 16384, 1024), idesc_pv,
-                                (j > t_lo[x] || k > 0) ? 1u : 0u);
-                    if (active(x, j + 1)) issue_s(x, j + 1);
-                    else tc_commit(o_done + x);
-                }
-                tc_commit(kv_empty + st);
             }
+            __syncwarp();
+        };
+        mbar_wait(kv_full + 0, 0, p.err);            // the bytes came through the async proxy: the wait itself orders them
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+            if (active(x, 0)) issue_s(x, 0);
+        if (elect_one()) tc_commit(kv_empty + 0);
+        __syncwarp();
+        for (int i = 0; i < n; ++i) {
+            const int st = (i + 1) % kStages;        // load i + 1: the values of round i and the keys of the next
+            mbar_wait(kv_full + st, ((i + 1) / kStages) & 1, p.err);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (active(x, i)) {
+                    const uint32_t vl = v_lo + st * (2 * kTileStep), more = i > first[x] ? 1u : 0u;
+                    const bool ends = !active(x, i + 1);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {             // a half's product runs while the exponentials of the other are made
+                        mbar_wait(p_ready + 2 * x + h, (i - first[x]) & 1, p.err);
+                        tc_after();
+                        if (elect_one()) {
+#pragma unroll
+                            for (int k = h * (kTN / 32); k < (h + 1) * (kTN / 32); ++k)   // P: 16 keys = 8 columns of packed pairs; V: 16 keys further down
+                                umma_ts(t0 + 256 + x * HD, t0 + x * 128 + k * 8, desc_words(vl + k * (16 * 128 >> 4), v_hi), idesc_pv, k > 0 ? 1u : more);
+                            if (h == 1 && ends) tc_commit(o_done + x);
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (active(x, i + 1)) issue_s(x, st);        // also the first scores of a tile that starts later (window)
+            }
+            if (elect_one()) tc_commit(kv_empty + st);
+            __syncwarp();
         }
     }
     } else {                                         // ---- softmax: one thread per query row ----
@@ -375,24 +400,6 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
                         }
                     }
                 }
-                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
-                const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
-                float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint32_t packed[32];
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const int c = h * 64 + 2 * k;
-                        const float2 arg = __ffma2_rn(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), scale2, neg_m2);
-                        const float2 pr = make_float2(ex2(arg.x), ex2(arg.y));
-                        sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
-                        __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
-                        packed[k] = *reinterpret_cast<uint32_t*>(&hh);
-                    }
-                    tm_store32(tS[x] + lane_base + h * 32, packed);     // P over the first 64 columns of S
-                }
-                l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
                 if (key0 + kTN - 1 > seq_last) {
                     // Keys behind the request's last one came along with its last page.  Their probability is 0, but
                     // what a former holder of the page left there (an Inf, a NaN) times 0 would be NaN: thread r clears
@@ -407,9 +414,27 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
                     }
                     fence_async_smem();                                       // the tensor core reads through the async proxy
                 }
-                tm_wait_st();
-                tc_before();
-                mbar_arrive(p_ready + x);
+                const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+                const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), neg_m2 = make_float2(-m_use, -m_use);
+                float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t packed[32];
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) {
+                        const int c = h * 64 + 2 * k;
+                        const float2 arg = __ffma2_rn(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), scale2, neg_m2);
+                        const float2 pr = k % 3 == 2 ? ex2_fma2(arg) : make_float2(ex2(arg.x), ex2(arg.y));
+                        sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
+                        __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
+                        packed[k] = *reinterpret_cast<uint32_t*>(&hh);
+                    }
+                    tm_store32(tS[x] + lane_base + h * 32, packed);     // P over the first 64 columns of S
+                    tm_wait_st();
+                    tc_before();
+                    mbar_arrive(p_ready + 2 * x + h);
+                }
+                l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
             }
             mbar_wait(o_done + x, 0, p.err);
             tc_after();

@@ -94,7 +94,7 @@ gemm_f32_split_kernel(const SplitParams p) {
     uint64_t* acc_free = acc_ready + 2;                // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 2);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = same_in_warp(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int w0 = blockIdx.x * kSplitRows, m0 = blockIdx.y * NT;
     // the block's share of K, in stages from kb0; a cluster's blocks share a tile of C (grid.z), none without a stage
     const int all_kb = (p.K + kSplitBK - 1) / kSplitBK;
@@ -158,9 +158,10 @@ gemm_f32_split_kernel(const SplitParams p) {
     } else {                                           // ---- sums: two warps per 32 lanes, half of the columns each ----
         const int quarter = warp & 3, half = (warp - 8) >> 2;
         constexpr int COLS = NT / 2;
-        // the products of stage kb, by one thread of warp 8; descriptors are those of the first stage and an offset
+        // the products of stage kb: warp 8 walks them with values that are the same in all lanes, one lane issues
         constexpr uint32_t id1 = idesc_bf16(128, NT, false), id2 = idesc_bf16(128, 2 * NT, false), id3 = idesc_bf16(128, 3 * NT, false);
-        const uint64_t w_desc = desc_sw128(smem_u32(stage0), 16, 1024), a_desc = desc_sw128(smem_u32(stage0) + 3 * kSplitABytes, 16, 1024);
+        const uint64_t desc = desc_sw128(smem_u32(stage0), 16, 1024);
+        const uint32_t w_lo = static_cast<uint32_t>(desc), hi = static_cast<uint32_t>(desc >> 32), t0 = same_in_warp(tmem_base);
         int s = 0, round = 0;
         auto issue = [&](int kb) {
             const int group = kb / kSplitFlush, buf = group & 1;
@@ -168,39 +169,39 @@ gemm_f32_split_kernel(const SplitParams p) {
             if (first && group >= 2) { mbar_wait(acc_free + buf, ((group >> 1) - 1) & 1, p.err); tc_after(); }
             mbar_wait(full + s, round & 1, p.err);
             tc_after();
-            const uint64_t wd = w_desc + s * (stage_bytes >> 4), ad = a_desc + s * (stage_bytes >> 4);
-            const uint32_t d = tmem_base + buf * 256;
-            constexpr uint64_t W1 = kSplitABytes >> 4, W2 = 2 * W1, A1 = b_plane >> 4, A2 = 2 * A1;
+            const uint32_t wl = w_lo + s * (stage_bytes >> 4), al = wl + (3 * kSplitABytes >> 4), d = t0 + buf * 256, more0 = first ? 0u : 1u;
+            constexpr uint32_t W1 = kSplitABytes >> 4, W2 = 2 * W1, A1 = b_plane >> 4, A2 = 2 * A1;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kSplitBK / 16; ++k) {
-                const uint32_t more = k > 0 || !first ? 1u : 0u;
-                const uint64_t wk = wd + k * 2, ak = ad + k * 2;
-                if (stacked) {                         // columns [0, NT): w0 a0;  [NT, 2 NT): w0 a1 + w1 a0;  [2 NT, 3 NT): w0 a2 + w1 a1 + w2 a0
-                    umma(d, wk, ak, id3, more);
-                    umma(d + NT, wk + W1, ak, id2, 1u);
-                    umma(d + 2 * NT, wk + W2, ak, id1, 1u);
-                } else {
-                    umma(d, wk, ak, id1, more);
-                    umma(d + NT, wk + W2, ak, id1, more);
-                    umma(d + NT, wk + W1, ak + A1, id1, 1u);
-                    umma(d + NT, wk, ak + A2, id1, 1u);
-                    umma(d + NT, wk + W1, ak, id1, 1u);
-                    umma(d + NT, wk, ak + A1, id1, 1u);
+                for (int k = 0; k < kSplitBK / 16; ++k) {
+                    const uint32_t more = k > 0 ? 1u : more0;
+                    auto at = [&](uint32_t lo) { return desc_words(lo + k * 2, hi); };
+                    if (stacked) {                     // columns [0, NT): w0 a0;  [NT, 2 NT): w0 a1 + w1 a0;  [2 NT, 3 NT): w0 a2 + w1 a1 + w2 a0
+                        umma(d, at(wl), at(al), id3, more);
+                        umma(d + NT, at(wl + W1), at(al), id2, 1u);
+                        umma(d + 2 * NT, at(wl + W2), at(al), id1, 1u);
+                    } else {
+                        umma(d, at(wl), at(al), id1, more);
+                        umma(d + NT, at(wl + W2), at(al), id1, more);
+                        umma(d + NT, at(wl + W1), at(al + A1), id1, 1u);
+                        umma(d + NT, at(wl), at(al + A2), id1, 1u);
+                        umma(d + NT, at(wl + W1), at(al), id1, 1u);
+                        umma(d + NT, at(wl), at(al + A1), id1, 1u);
+                    }
                 }
+                tc_commit(empty + s);
+                if (kb % kSplitFlush == kSplitFlush - 1 || kb == num_kb - 1) tc_commit(acc_ready + buf);
             }
-            tc_commit(empty + s);
-            if (kb % kSplitFlush == kSplitFlush - 1 || kb == num_kb - 1) tc_commit(acc_ready + buf);
+            __syncwarp();
             if (++s == STAGES) { s = 0; ++round; }
         };
-        const bool issuer = warp == 8 && lane == 0;
-        if (issuer) issue(0);
-        __syncwarp();
+        if (warp == 8) issue(0);
         uint64_t acc[COLS / 2];
 #pragma unroll
         for (int j = 0; j < COLS / 2; ++j) acc[j] = 0;
         const uint32_t mine = tmem_base + half * COLS + (static_cast<uint32_t>(quarter * 32) << 16);
         for (int kb = 0; kb < num_kb; ++kb) {
-            if (issuer && kb + 1 < num_kb) issue(kb + 1);
+            if (warp == 8 && kb + 1 < num_kb) issue(kb + 1);
             if (kb % kSplitFlush != kSplitFlush - 1 && kb != num_kb - 1) continue;
             __syncwarp();
             const int group = kb / kSplitFlush, buf = group & 1;
