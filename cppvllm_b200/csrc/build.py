@@ -51,6 +51,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "lru": ["lru.cu"],
     "linear": ["linear.cu"],
     "ssd": ["ssd.cu"],
+    "ssd_tc": ["ssd_tcgen05.cu"],
     "sandwich": ["sandwich.cu"],
     "hyper": ["hyper.cu"],
     "attn_masked": ["attention_masked.cu"],

@@ -859,7 +859,9 @@ def skip_scan(out, q, k, v, log_decay, step, skip, state: torch.Tensor, cu_seqle
 # ---- state-space recurrence (csrc/ssd.cu) -----------------------------------------------------------------------------------------
 
 _ssd = None
+_ssd_tc = None
 SSD_CHUNK = 64              # tokens per chunk of the tensor-core form
+SSD_TC_CHUNK = 128          # and of its tcgen05 form
 
 
 def _ssd_lib():
@@ -923,11 +925,18 @@ def ssd_held_chunks(max_tokens: int) -> int:
     return 2 * max_tokens // SSD_CHUNK + 2
 
 
+def ssd_tcgen05_supported(dim: int, vdim: int) -> bool:
+    """The tcgen05 kernels take states of 128 x 64, at every length of the portions: the three passes against the `mma.sync` form's on a
+    B200 (us, 32 heads): 8 tokens 9.2 / 10.3, 65 9.5 / 21, 300 18 / 28, 2,048 36 / 80, eight portions of 20 tokens 14.8 / 15.5;  128 heads: 8
+    tokens 9.3 / 11, 2,048 118 / 282."""
+    return dim == 128 and vdim == 64
+
+
 def ssd_chunks(y: torch.Tensor, u: torch.Tensor, dt: torch.Tensor, log_decay: torch.Tensor, skip: torch.Tensor, state: torch.Tensor, cu_seqlens,
                state_slots, q_lens, num_heads: int, groups: int, dim: int, vdim: int, ends: Optional[torch.Tensor] = None,
-               decays: Optional[torch.Tensor] = None) -> torch.Tensor:
+               decays: Optional[torch.Tensor] = None, kernel: str = "") -> torch.Tensor:
     """Per request and head: S <- exp(log_decay) S + dt B x^T, y = S^T C + skip_h x over the request's tokens of this step, in chunks of 64 tokens on
-    the tensor cores; u bf16 [T, H vdim + 2 G dim] rows [x | B | C]; y float32 [T, H * vdim].  Portions of more than 64 tokens go through `ends`
+    the tensor cores (128 on csrc/ssd_tcgen05.cu's kernels, see ssd_tcgen05_supported; `kernel` = "mma" | "tcgen05" fixes the choice); u bf16 [T, H vdim + 2 G dim] rows [x | B | C]; y float32 [T, H * vdim].  Portions of more than 64 tokens go through `ends`
     (float32, H dim vdim per chunk of such a portion) and `decays` (float32, H per chunk)."""
     _cuda(y, u, dt, log_decay, skip, state, cu_seqlens, state_slots, ends, decays); _contig(y, u, dt, log_decay, skip, cu_seqlens, state_slots, ends, decays)
     sp, sf, n_slots = _state_args(state)
@@ -936,9 +945,16 @@ def ssd_chunks(y: torch.Tensor, u: torch.Tensor, dt: torch.Tensor, log_decay: to
             or log_decay.shape != dt.shape or skip.numel() != num_heads or cu_seqlens.dtype != torch.int32 or state_slots.dtype != torch.int32
             or any(t is not None and t.dtype != torch.float32 for t in (y, dt, log_decay, skip, ends, decays))):
         raise KernelError("ssd_chunks: u bf16 [T, channels]; y float32 [T, H * vdim]; dt, log_decay float32 [T, H]; skip float32 [H]")
-    per = [-(-n // SSD_CHUNK) for n in q_lens]
+    tcgen05 = kernel == "tcgen05" or (kernel == "" and ssd_tcgen05_supported(dim, vdim))
+    size = SSD_TC_CHUNK if tcgen05 else SSD_CHUNK
+    per = [-(-n // size) for n in q_lens]
     held = sum(c for c in per if c > 1)
-    _check(_ssd_lib().cvb_ssd_chunks(
+    global _ssd_tc
+    if tcgen05 and _ssd_tc is None:
+        lib = load_library("ssd_tc")
+        lib.cvb_ssd_chunks_tcgen05.restype = c_int
+        _ssd_tc = lib
+    _check((_ssd_tc.cvb_ssd_chunks_tcgen05 if tcgen05 else _ssd_lib().cvb_ssd_chunks)(
         _ptr(y), _ptr(u), _ptr(dt), _ptr(log_decay), _ptr(skip), _ptr(ends), c_int64(ends.numel() if ends is not None else 0), _ptr(decays),
         c_int64(decays.numel() if decays is not None else 0), sp, sf, c_int(n_slots), _ptr(cu_seqlens), _ptr(state_slots), c_int(len(per)),
         c_int(sum(per)), c_int(held), c_int(num_heads), c_int(groups), c_int(dim), c_int(vdim), _ptr(error_flag(u.device)), _stream()),
