@@ -214,7 +214,11 @@ qk_norm_rope_kv_vec_kernel(T* __restrict__ q_out, const T* __restrict__ qkv, con
     }
     if (q_w != nullptr) {
 #pragma unroll
-        for (int i = 0; i < N; ++i) { wq[i] = q_w[c * N + i]; wk[i] = k_w[c * N + i]; }
+        for (int i = 0; i < N; i += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(q_w + c * N + i), b = *reinterpret_cast<const float4*>(k_w + c * N + i);
+            wq[i] = a.x; wq[i + 1] = a.y; wq[i + 2] = a.z; wq[i + 3] = a.w;
+            wk[i] = b.x; wk[i + 1] = b.y; wk[i + 2] = b.z; wk[i + 3] = b.w;
+        }
     }
     // what does not change from head to head is computed once: the row of this token in q_out, and the row of its slot
     // in the K block of its page (the V block lies KV * page_size rows further, head kvh page_size rows further)
@@ -318,7 +322,7 @@ extern "C" int cvb_qk_norm_rope_kv(void* q_out, const void* qkv, const float* q_
         auto al = [](const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
         const bool full_rot = cos_t == nullptr || (rot == hd && !interleaved);
         if (CH >= 2 && CH <= 32 && (CH & (CH - 1)) == 0 && full_rot && al(q_out) && al(qkv) && al(cache) && al(cos_t) &&
-            al(sin_t) && (dtype == CVB_DTYPE_BF16 || dtype == CVB_DTYPE_F32)) {
+            al(sin_t) && al(q_w) && al(k_w) && (dtype == CVB_DTYPE_BF16 || dtype == CVB_DTYPE_F32)) {
             dim3 vgrid(static_cast<unsigned>(T));
 #define VCALL_CH(TY, C)                                                                                        \
     launch_kernel(qk_norm_rope_kv_vec_kernel<TY, C>, dim3(vgrid), dim3(kVecThreads), 0, stream,                                      \
