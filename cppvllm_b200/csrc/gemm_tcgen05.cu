@@ -32,8 +32,8 @@ constexpr int kBK = 64;                       // one 128-byte swizzle span of bf
 constexpr int kGemmThreads = 192;
 constexpr int kBoxBytes = 32 * 64 * 2;        // what a warp of the epilogue hands to one TMA store: 32 rows of 64 bf16
 
-// kRelu2: C = relu(T(A B^T))^2.  kSwiglu and kGeglu share the gated tile: C = f(T(G), T(U)) with f = silu(g) u;  gelu_tanh(g) u.
-enum GemmEpilogue { kPlain = 0, kSwiglu = 1, kAddResidual = 2, kRelu2 = 3, kGeglu = 5 };
+// kSwiglu and kGeglu share the gated tile: C = f(T(G), T(U)) with f = silu(g) u;  gelu_tanh(g) u.
+enum GemmEpilogue { kPlain = 0, kSwiglu = 1, kAddResidual = 2, kGeglu = 5 };
 constexpr bool gated_epilogue(int e) { return e == kSwiglu || e == kGeglu; }
 
 struct GemmParams {
@@ -210,10 +210,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 y0 = gated_value<EPI>(g0, u0);
                                 y1 = gated_value<EPI>(g1, u1);
                             }
-                            if constexpr (EPI == kRelu2) {
-                                y0 = fmaxf(rnd<__nv_bfloat16>(y0), 0.f); y0 *= y0;
-                                y1 = fmaxf(rnd<__nv_bfloat16>(y1), 0.f); y1 *= y1;
-                            }
                             if constexpr (EPI == kAddResidual) {
                                 const float2 r = __bfloat1622float2(r2[k]);
                                 y0 = rnd<__nv_bfloat16>(y0) + r.x;
@@ -314,6 +310,5 @@ extern "C" int cvb_gemm_bf16_tcgen05(void* out, const void* a, const void* w, co
     if (mode == 5) return launch_gemm<256, 4, kGeglu>(ma, mw, mo, p, stream);
     if (mode == 0) return tile_n == 256 ? launch_gemm<256, 4, kPlain>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kPlain>(ma, mw, mo, p, stream);
     if (mode == 2) return tile_n == 256 ? launch_gemm<256, 4, kAddResidual>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kAddResidual>(ma, mw, mo, p, stream);
-    if (mode == 3) return tile_n == 256 ? launch_gemm<256, 4, kRelu2>(ma, mw, mo, p, stream) : launch_gemm<128, 6, kRelu2>(ma, mw, mo, p, stream);
     return CVB_E_SHAPE;
 }

@@ -21,7 +21,7 @@
 //                   pass 1: per (chunk but the last, head, 64 columns): what the chunk adds to a state from zero; e^(l_last)
 //                   pass 2: the states in front of the chunks, element by element
 //                   pass 3: per (chunk, head, 64 columns): the outputs from the true state; a request's last chunk leaves the new state
-//                 Where no request has more than one chunk only pass 3 runs.
+//                 Where no request has more than one chunk only pass 3 runs.  States of 128 x 64 take ssd_tcgen05.cu instead.
 //   ssd_step    : a step of decoded tokens (one per request) in one kernel, a block per (request, head): convolutions, ring, dt, the
 //                 rule on S, y.
 //   ssd_norm    : out = T( u / sqrt(mean(u^2) + eps) * w ), u = y silu(z), over equal parts of the row; a weight per element of the row.

@@ -22,7 +22,8 @@ type; only the projections around them are products in the activations' type.
   S <- exp(-exp(A_h) dt) S + dt B x^T  ([state, vdim], B and C of group h / (heads / groups));  y = S^T C + D_h x;
   out = Wo (RMSNorm_parts(y * silu(z)) * w), the norm over ``norm_parts`` equal parts of the row, the gate in front of it.  State per
   request: S of every head and behind it a ring of the last ``taps`` inputs of the convolution.  Portions in bf16 run in chunks on the tensor
-  cores, decoded tokens in one kernel and the norm; float32 and other sizes take the token-by-token scan (csrc/ssd.cu, csrc/recurrent.cu).
+  cores (csrc/ssd_tcgen05.cu for states of 128 x 64, csrc/ssd.cu), decoded tokens in one kernel and the norm; float32 and other sizes take
+  the token-by-token scan (csrc/recurrent.cu).
 """
 from __future__ import annotations
 
