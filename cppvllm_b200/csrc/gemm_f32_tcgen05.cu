@@ -20,7 +20,9 @@
 // What bounds it: shared memory (a product of parts of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, and the parts have to
 // be written) and, close behind, the cuts (about six instructions an element).  449 rows by 4,096 x 1,024: 87 us as a float32
 // library product, now 33 (113 TFLOP/s of float32 work); by 1,024 x 2,048: 57, now 21.
-// Every wait is bounded by a cycle count; one that runs out records error 5 and the block carries on to its end.
+// Every wait is bounded by a cycle count; one that runs out records error 5 and the block carries on to its end.  The kernel may start while
+// the ones before it run, for as long as those take, so the threads ask for W alone and pass griddepcontrol.wait before they wait
+// for anything else.
 #include "sm100.cuh"
 
 namespace cvb {
@@ -149,6 +151,7 @@ gemm_f32_split_kernel(const SplitParams p) {
             if (++s == STAGES) { s = 0; ++round; }
         }
     } else {                                           // ---- sums: two warps per 32 lanes, half of the columns each ----
+        pdl_wait();                                    // before the first bounded wait: its limit is not for the time of the kernels before this one
         const int quarter = warp & 3, half = (warp - 8) >> 2;
         constexpr int COLS = NT / 2;
         // the products of stage kb: warp 8 walks them with values that are the same in all lanes, one lane issues
@@ -220,7 +223,6 @@ gemm_f32_split_kernel(const SplitParams p) {
             if (lane == 0) mbar_arrive(acc_free + buf);
         }
         if (gridDim.z == 1) {
-            pdl_wait();                                // nothing is written before the kernels before this one are done
             const int n = w0 + quarter * 32 + lane, first = m0 + half * COLS;
             if (n < p.N) {
 #pragma unroll
@@ -236,7 +238,6 @@ gemm_f32_split_kernel(const SplitParams p) {
     if (gridDim.z > 1) {                               // each block adds up and stores its rows of the tile, the parts of K in order
         __syncwarp();
         cluster_sync();
-        pdl_wait();
         const int n = threadIdx.x % kSplitRows;
         for (int j = blockIdx.z * 4 + threadIdx.x / kSplitRows; j < NT; j += gridDim.z * 4) {
             if (m0 + j >= p.M || w0 + n >= p.N) continue;

@@ -57,3 +57,30 @@ def test_infinities_and_nan(tile):
     assert bool(torch.isfinite(out[39][big]).all())
     rest = [i for i in range(40) if i not in (3, 17, 30, 39)]
     assert torch.equal(out[rest], clean[rest])
+
+
+def test_a_long_kernel_in_front_does_not_run_out_the_waits():
+    """The product may start beside the kernel before it, whose time is no part of its waits' limit (40 million cycles)."""
+    from cppvllm_b200.csrc import ops
+    dev, T, dim, vdim = torch.device("cuda:0"), 300000, 16, 64
+    g = torch.Generator().manual_seed(9)
+    q, k, v = (torch.randn(T, n, generator=g).to(dev) for n in (vdim, vdim, vdim))
+    la, dt, skip = torch.full((T, 1), -0.5, device=dev), torch.full((T, 1), 0.1, device=dev), torch.ones(1, device=dev)
+    out, state = torch.empty(T, vdim, device=dev), torch.zeros(1, dim * vdim, device=dev)
+    cu, slots = (torch.tensor(x, dtype=torch.int32, device=dev) for x in ([0, T], [0]))
+    x, w, y = out.view(-1)[-40 * 128:].view(40, 128), torch.randn(70, 128, generator=g).to(dev), torch.empty(40, 70, device=dev)
+
+    def scan():                                # token by token in a block or two: the other SMs are free for the product
+        ops.skip_scan(out, q[:, :dim], k[:, :dim], v, la, dt, skip, state, cu, slots, 1, 1, 1, dim, vdim)
+    scan()
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()
+    scan()
+    e1.record()
+    torch.cuda.synchronize()
+    assert e0.elapsed_time(e1) > 40.0          # more than the limit at any clock the GPU runs at under load
+    out.zero_()
+    scan()
+    ops.gemm_f32_split(y, x, w)
+    ops.check_device_errors(dev)
+    torch.testing.assert_close(y.double(), x.double() @ w.double().T, rtol=1e-5, atol=1e-5 * float(x.abs().max()))
