@@ -258,7 +258,7 @@ gemm_f32_split_kernel(const SplitParams p) {
 }
 
 template <int NT>
-static int launch_split(const SplitParams& p, int parts, cudaStream_t stream) {
+static int launch_split(const SplitParams& p, int parts, bool dependent, cudaStream_t stream) {
     constexpr int stages = NT <= kSplitStack ? 3 : 2;
     constexpr size_t smem = 1024 + static_cast<size_t>(stages) * 3 * (kSplitABytes + NT * 128) + 10 * 8 + 16;
     static bool set = false;
@@ -282,7 +282,7 @@ static int launch_split(const SplitParams& p, int parts, cudaStream_t stream) {
         ++n;
     }
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (pdl_enabled() && cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+    if (dependent && pdl_enabled() && cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -298,7 +298,9 @@ static int launch_split(const SplitParams& p, int parts, cudaStream_t stream) {
 using namespace cvb;
 
 // tile: rows of A a block (32, 64, 96 or 128); parts: blocks that share a tile's K (1, 2, 4 or 8, each with 64 of K or more).
-extern "C" int cvb_gemm_f32_split(float* out, const float* a, const float* w, int M, int N, int K, int tile, int parts, int* err_flag, cudaStream_t stream) {
+// dependent: launch with the programmatic-dependent-launch attribute (outside captures).
+extern "C" int cvb_gemm_f32_split(float* out, const float* a, const float* w, int M, int N, int K, int tile, int parts, int dependent, int* err_flag,
+                                  cudaStream_t stream) {
     if (M == 0) return CVB_OK;
     if (M < 0 || N <= 0 || K <= 0) return CVB_E_SIZE;
     if (tile < 32 || tile > 128 || tile % 32 || parts < 1 || parts > 8 || (parts & (parts - 1)) || parts > (K + kSplitBK - 1) / kSplitBK) return CVB_E_SHAPE;
@@ -307,8 +309,8 @@ extern "C" int cvb_gemm_f32_split(float* out, const float* a, const float* w, in
     if (rows > 65535) return CVB_E_SIZE;
     if ((static_cast<int64_t>(M) > N ? M : N) * static_cast<int64_t>(K) > (1LL << 30) - 1) return CVB_E_SIZE;     // byte offsets in 32 bits
     const SplitParams p{out, a, w, M, N, K, err_flag};
-    if (tile == 32) return launch_split<32>(p, parts, stream);
-    if (tile == 64) return launch_split<64>(p, parts, stream);
-    if (tile == 96) return launch_split<96>(p, parts, stream);
-    return launch_split<128>(p, parts, stream);
+    if (tile == 32) return launch_split<32>(p, parts, dependent != 0, stream);
+    if (tile == 64) return launch_split<64>(p, parts, dependent != 0, stream);
+    if (tile == 96) return launch_split<96>(p, parts, dependent != 0, stream);
+    return launch_split<128>(p, parts, dependent != 0, stream);
 }

@@ -2413,7 +2413,7 @@ def _measure_projection(name: str, x, weight, out, rows) -> float:
 
 def project_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows: int, dependent: bool = True) -> torch.Tensor:
     """out = x @ weight^T by the kernel that suits the step.  A weight whose share per SM fits into shared memory goes
-    through the product made for chains of dependent launches (`dependent=False` keeps that kernel behind its
+    through the product made for chains of dependent launches (`dependent=False` keeps that kernel, or the float32 one, behind its
     predecessor's end instead of letting it start early and fetch its weights meanwhile).  Otherwise the candidates for a
     few bf16 rows (the weight-streaming product, its split-K form, the ring-buffered product, the library's product) are timed once per shape, with
     the weight out of the L2, the first time the shape is seen outside a graph capture, and the fastest is kept; during
@@ -2422,7 +2422,9 @@ def project_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows:
     if gemv_stream_supported(x.dtype, weight, rows):
         return gemv_stream_bf16(out, x, weight, rows, dependent=dependent)
     if rows > GEMV_MAX_ROWS or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
-        return gemm_f32_split(out, x, weight) if gemm_f32_split_supported(x, weight, out) else linear(x, weight, out=out)
+        if gemm_f32_split_supported(x, weight, out):
+            return gemm_f32_split(out, x, weight, dependent=dependent)
+        return linear(x, weight, out=out)
     key = (weight.shape[0], weight.shape[1], rows if rows <= 2 else (8 if rows <= 8 else 16))
     choice = _project_choice.get(key)
     if choice is None:
@@ -2581,9 +2583,10 @@ def gemm_f32_split_supported(x: torch.Tensor, weight: torch.Tensor, out: torch.T
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
-def gemm_f32_split(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, tile: Optional[Tuple[int, int]] = None) -> torch.Tensor:
+def gemm_f32_split(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, tile: Optional[Tuple[int, int]] = None,
+                   dependent: bool = True) -> torch.Tensor:
     """out = x @ weight^T, all float32, with products of bf16 parts and float sums that are no further from float64 than a float32
-    product's.  `tile` fixes split_tile's choice."""
+    product's.  `tile` fixes split_tile's choice; `dependent=False` launches without the programmatic-dependent-launch attribute."""
     global _gemm_f32
     if _gemm_f32 is None:
         lib = load_library("gemm_f32")
@@ -2596,7 +2599,7 @@ def gemm_f32_split(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, til
         raise KernelError("gemm_f32_split: x [M, K], weight [N, K], out [M, N], all float32")
     rows, parts = tile if tile is not None else split_tile(M, N, K)
     _check(_gemm_f32.cvb_gemm_f32_split(_ptr(out), _ptr(x), _ptr(weight), c_int(M), c_int(N), c_int(K), c_int(rows), c_int(parts),
-                                        _ptr(error_flag(x.device)), _stream()), "gemm_f32_split")
+                                        c_int(1 if dependent else 0), _ptr(error_flag(x.device)), _stream()), "gemm_f32_split")
     return out
 
 
