@@ -1,12 +1,16 @@
 // Matrix product of the 32-bit path on the fifth-generation tensor cores (tcgen05):
-//   C[M, N] = A[M, K] * W[N, K]^T,  all float32, with the error of a float32 product or less.
+//   C[M, N] = A[M, K] * W[N, K]^T,  all float32, with the error of a product in float32.
 //
 // The tensor cores multiply 16-bit operands far faster than the float units add up 32-bit ones, so every element is cut into
-// three bf16 parts of eight significant bits each, a = a0 + a1 + a2.  The cuts truncate, so they are exact: nothing of the 24 bits
-// is lost.  Of the nine products of parts, the six of weight 2^0, 2^-8 and 2^-16 are taken; what is left out is at most 2^-23 of
-// |a w|, and products of parts are exact in the float accumulators' inputs.  The tensor core's accumulation truncates where a
-// float add rounds, so a chain in tensor memory is kept short: after every 128 of K the partial sums (those of weight 2^0 apart
-// from the smaller ones) are read back and added, rounded to nearest, to sums in registers.
+// three bf16 parts, a = a0 + a1 + a2: a0 is a rounded to nearest, a1 what is left rounded to nearest, a2 the rest, which has at most
+// eight bits left.  The cuts are exact: |a1| <= 2^-8 |a|, |a2| <= 2^-17 |a|, and nothing of the 24 bits is lost.  Of the nine products of parts,
+// the six of weight 2^0, 2^-8 and 2^-16 are taken; what is left out (a1 w2, a2 w1, a2 w2) is at most 2^-24 (1 + 2^-9) of |a w|, of either sign, no
+// more than the rounding of a float32 product.  (Parts cut off instead of rounded leave up to 2^-21 out, always towards zero:
+// operands just above a bf16 came out 4.7e-7 too small.)  Products of parts are exact in the float accumulators' inputs.  The tensor
+// core's accumulation truncates where a float add rounds, so a chain in tensor memory is kept short: after every 128 of K the partial sums
+// (those of weight 2^0 apart from the smaller ones) are read back and added, rounded to nearest, to sums in registers.  Error against
+// float64, 17 to 449 rows, K 128 to 8,192: 0.7e-7 to 1.5e-7 for operands of both signs (the library's float32 product 2.0e-7 to 8.1e-7), 0.8e-7 to
+// 1.5e-7 for operands of one sign (1.4e-7 to 6.0e-7), where truncation makes nearly all of it.
 //
 // A block makes 128 columns of C (rows of W: the M operand) for up to 128 rows of A (the N operand, rounded up to 32):
 //   warps 0-7   fetch the next 64 of K of both operands (16 bytes a thread), cut them and lay the parts into shared memory as
@@ -18,8 +22,9 @@
 // With few tiles the blocks of a cluster share a tile's K and add their sums up through distributed shared memory.
 //
 // What bounds it: shared memory (a product of parts of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, and the parts have to
-// be written) and, close behind, the cuts (about six instructions an element).  449 rows by 4,096 x 1,024: 87 us as a float32
-// library product, now 33 (113 TFLOP/s of float32 work); by 1,024 x 2,048: 57, now 21.
+// be written) and, close behind, the cuts (about six instructions an element).  us between events, with the weights out of the L2: 449
+// rows by 4,096 x 1,024 91 as a float32 library product, 40 with parts cut off, now 36; by 1,024 x 2,048 62, 28, now 25; 2,048 rows by
+// 4,096 x 2,048 651, 243, now 224 (153 TFLOP/s of float32 work).
 // Every wait is bounded by a cycle count; one that runs out records error 5 and the block carries on to its end.  The kernel may start while
 // the ones before it run, for as long as those take, so the threads ask for W alone and pass griddepcontrol.wait before they wait
 // for anything else.
@@ -46,21 +51,30 @@ struct SplitParams {
 __device__ __forceinline__ uint64_t pack2(float a, float b) { return static_cast<uint64_t>(__float_as_uint(a)) | (static_cast<uint64_t>(__float_as_uint(b)) << 32); }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) { uint64_t d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) { uint64_t d; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-// Their upper halves side by side: the leading eight bits, truncated, as two bf16
+// Two bf16 side by side: rounded to nearest, or the upper halves, which are all of a number of up to eight bits
+__device__ __forceinline__ uint32_t nearest2(uint64_t v) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float(static_cast<uint32_t>(v >> 32))), "f"(__uint_as_float(static_cast<uint32_t>(v))));
+    return d;
+}
 __device__ __forceinline__ uint32_t upper_halves(uint64_t v) { return __byte_perm(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32), 0x7632); }
-__device__ __forceinline__ uint64_t cut2(uint64_t v) { return sub2(v, v & 0xFFFF0000FFFF0000ull); }
+// What two bf16 leave of two floats, exactly
+__device__ __forceinline__ uint64_t rest2(uint64_t v, uint32_t h) { return sub2(v, static_cast<uint64_t>(h << 16) | (static_cast<uint64_t>(h & 0xFFFF0000u) << 32)); }
 
 // Four consecutive elements into the three tiles of parts: 8 bytes each, `plane` bytes apart.
 __device__ __forceinline__ void store_parts(unsigned char* at, uint32_t plane, float4 f) {
     uint64_t x = pack2(f.x, f.y), y = pack2(f.z, f.w);
 #pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        *reinterpret_cast<uint2*>(at + p * plane) = make_uint2(upper_halves(x), upper_halves(y));
-        if (p < 2) { x = cut2(x); y = cut2(y); }
+    for (int p = 0; p < 2; ++p) {
+        const uint32_t hx = nearest2(x), hy = nearest2(y);
+        *reinterpret_cast<uint2*>(at + p * plane) = make_uint2(hx, hy);
+        x = rest2(x, hx);
+        y = rest2(y, hy);
     }
+    *reinterpret_cast<uint2*>(at + 2 * plane) = make_uint2(upper_halves(x), upper_halves(y));
 }
 
-// A result that is not finite is computed again: an infinity has no finite parts.
+// A result that is not finite is computed again: an infinity, or a number that rounds to one, has no finite parts.
 __device__ __forceinline__ void split_store(const SplitParams& p, int m, int n, float v) {
     if (!isfinite(v)) {
         const float* x = p.a + static_cast<int64_t>(m) * p.K;

@@ -43,6 +43,36 @@ def test_error_no_larger_than_the_library(M, N, K):
     assert float(ours) <= float(lib), (float(ours), float(lib))
 
 
+def _one_sign(kind, shape, g):
+    """Numbers from 1 up to 2 whose first part is a multiple of 2^-7, at the edges of the cuts."""
+    a = 1 + torch.randint(0, 127, shape, generator=g) / 128.0
+    if kind == "below a bf16":                   # cut off instead of rounded, all of the other two parts is there
+        return a + 2.0 ** -7 - 2.0 ** -23 * torch.randint(1, 4, shape, generator=g)
+    if kind == "below half a step":              # the second part is as large as it gets, the third of either sign
+        return a + 2.0 ** -8 - 2.0 ** -17 + 2.0 ** -23 * torch.randint(-1, 2, shape, generator=g)
+    return a + 2.0 ** -8 + 2.0 ** -17 * (1 - 2.0 ** -6)
+
+
+@pytest.mark.parametrize("kind", ["below a bf16", "below half a step", "above half a step"])
+@pytest.mark.parametrize("M,N,K", [(17, 200, 128), (40, 96, 384), (130, 300, 1024)])
+def test_operands_of_one_sign_at_the_edges_of_the_cuts(kind, M, N, K):
+    """Nothing cancels here, so what the cuts leave out adds up over K."""
+    from cppvllm_b200.csrc import ops
+    g = torch.Generator().manual_seed(K)
+    x, w = _one_sign(kind, (M, K), g).cuda(), _one_sign(kind, (N, K), g).cuda()
+    ref = x.double() @ w.double().T
+    for tile in (None, (64, 1), (128, 2)):
+        err = (_run(ops, x, w, tile).double() - ref) / ref
+        # Sums of leading parts are exact in tensor memory (multiples of 2^-14 below 2^9), the others are below 2^-6 of them: 40 truncations of
+        # 2^-23 of that at most.  2^-24 (1 + 2^-9) of every product is left out, a group of 128 of K is added with two roundings, each
+        # of at most 2^-24 of what is there, and up to 8 parts of K with one.
+        bound = (1 + 2.0 ** -9 + 40 * 2.0 ** -5 + 2 * -(-K // 128) + (0 if tile is None or tile[1] == 1 else 2)) * 2.0 ** -24
+        if tile is None:
+            bound += 8 * 2.0 ** -24
+        assert float(err.abs().max()) <= bound
+        assert abs(float(err.mean())) <= (1.5 + 40 * 2.0 ** -5) * 2.0 ** -24       # roundings to nearest leave no mean
+
+
 @pytest.mark.parametrize("tile", [(32, 1), (64, 2), (128, 1)])
 def test_infinities_and_nan(tile):
     """A row with a value that has no parts gives what float sums give; the other rows do not see it."""
