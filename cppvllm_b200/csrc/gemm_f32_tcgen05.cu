@@ -22,9 +22,9 @@
 // With few tiles the blocks of a cluster share a tile's K and add their sums up through distributed shared memory.
 //
 // What bounds it: shared memory (a product of parts of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, and the parts have to
-// be written) and, close behind, the cuts (about six instructions an element).  us between events, with the weights out of the L2: 449
-// rows by 4,096 x 1,024 91 as a float32 library product, 40 with parts cut off, now 36; by 1,024 x 2,048 62, 28, now 25; 2,048 rows by
-// 4,096 x 2,048 651, 243, now 224 (153 TFLOP/s of float32 work).
+// be written) and, close behind, the cuts (about six instructions an element).  449 rows by 4,096 x 1,024: 86 us as a float32
+// library product, 33 with parts cut off, now 28 (134 TFLOP/s of float32 work); by 1,024 x 2,048 57, 21, now 18; 2,048 rows by 4,096 x 1,024 330,
+// 128, now 108 (159 TFLOP/s).
 // Every wait is bounded by a cycle count; one that runs out records error 5 and the block carries on to its end.  The kernel may start while
 // the ones before it run, for as long as those take, so the threads ask for W alone and pass griddepcontrol.wait before they wait
 // for anything else.

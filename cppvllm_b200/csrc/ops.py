@@ -2548,20 +2548,20 @@ def feed_tokens(tokens: torch.Tensor, src: torch.Tensor, sampled: torch.Tensor, 
 # ---- float32 products on the tensor cores (csrc/gemm_f32_tcgen05.cu) --------------------------------------------
 
 _gemm_f32 = None
-# From 17 rows and 128 of K on the error is smaller than the library's at every size measured (128 to 4,096 outputs, 17 to 512 rows, K 128 to
-# 3,072: 1.1e-7 to 1.9e-7 where the library's is 2.0e-7 to 9.9e-7); for 16 rows and fewer, and a short K, the library adds in shorter chains
-# (16 x 128 x 256: 1.0e-7, here 1.2e-7;  K 64: 8.6e-8, here 1.1e-7).
+# For 16 rows and fewer the library adds in shorter chains, and with K below 128 too.  Error against float64 of 17 to 512 rows by 128 to 4,096
+# outputs, K 128 to 3,072: 0.7e-7 to 1.5e-7 where the library's is 2.0e-7 to 9.9e-7.
 SPLIT_MIN_ROWS, SPLIT_MIN_K = 17, 128
-SPLIT_STAGE = {32: 1.1, 64: 1.25, 96: 1.5, 128: 1.75}       # us per 64 of K for a block of so many rows of x (measured, 40 to 148 blocks)
+# us per 64 of K for a block of so many rows of x (measured: 0.8, 1.0, 1.2, 1.4 with 40 blocks; 1.2, 1.6, 1.5, 1.7 with 140)
+SPLIT_STAGE = {32: 1.1, 64: 1.25, 96: 1.5, 128: 1.75}
 SPLIT_FIXED = 6.0                                           # us a block otherwise
 SPLIT_BLOCKS = {1: 148, 2: 148, 4: 136, 8: 112}             # blocks at once in clusters of 1, 2, 4, 8 (a cluster lies in one group of SMs)
 
 
 def split_tile(rows: int, n_out: int, k: int) -> Tuple[int, int]:
     """(rows of x a block of the split product takes, blocks that share a tile's K): the choice whose waves of blocks take the
-    shortest time by the figures above.  Measured on a B200, us with (rows, blocks): 449 x 1,024 x 2,048 (128, 1) 57, (128, 4) 21,
-    (64, 2) 29, (64, 8) 53;  64 x 1,024 x 2,048 (64, 1) 47, (64, 8) 11;  200 x 4,096 x 1,024 (128, 1) 33, (128, 2) 22, (64, 1) 28;
-    449 x 4,096 x 1,024 (128, 1) 34, (128, 2) 43, (64, 1) 55."""
+    shortest time by the figures above.  Measured on a B200, us with (rows, blocks): 449 x 1,024 x 2,048 (128, 1) 47, (128, 4) 18,
+    (64, 2) 23, (64, 8) 44;  64 x 1,024 x 2,048 (64, 1) 36, (64, 8) 10;  200 x 4,096 x 1,024 (128, 1) 27, (128, 2) 19, (64, 1) 21;
+    449 x 4,096 x 1,024 (128, 1) 28, (128, 2) 37, (64, 1) 41."""
     stages, best = -(-k // 64), None
     for tile, us in SPLIT_STAGE.items():
         tiles = -(-n_out // 128) * -(-rows // tile)
@@ -2574,13 +2574,31 @@ def split_tile(rows: int, n_out: int, k: int) -> Tuple[int, int]:
     return best[1], best[2]
 
 
+def gemm_f32_split_preferred(rows: int, n_out: int, k: int) -> bool:
+    """Where the product on the tensor cores is the faster one.  Against the library's float32 product on a B200 (us, launches back to back): 32
+    rows by 4,096 x 1,024 12 / 21, by 1,024 x 2,048 10 / 21;  64: 10 / 23 and 10 / 37;  200: 20 / 47 and 14 / 41;  449: 28 / 86 and 18 / 57;  600:
+    46 / 123 and 26 / 87;  2,048 108 / 331 and 49 / 160.
+    It multiplies tiles of 128 outputs, so few outputs cost as much as 128, and a block's start is 6 us: one output (between events, 500 rows,
+    K 4,096 20 / 15; 8,192 rows 73 / 39) and a short K for few outputs (8,192 rows by 16, K 256 18.4 / 15.2, K 384 20.5 / 18.4, K 512 equal;
+    2,048 rows by 16, K 256 12.3 / 13.3) or for few of them in all (K 128: 4,096 by 256 16.4 / 14.3, 8,192 by 128 16.4 / 15.2, 8,192 by 256 16.4 /
+    20.4, 2,048 by 1,024 16.3 / 20.5; K 192: 512 by 1,024 14.3 / 13.2) are the library's."""
+    if n_out < 2:
+        return False
+    if k >= 512:
+        return True
+    if k >= 256:
+        return n_out >= 128 or rows <= 2048
+    return n_out >= 128 and rows * n_out >= 1 << 21
+
+
 def gemm_f32_split_supported(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> bool:
-    """Whether a float32 product goes through the tensor cores.  Against the library's float32 product on a B200 (us): 32 rows by
-    4,096 x 1,024 10 / 21, by 1,024 x 2,048 10 / 22;  64: 10 / 24 and 10 / 37;  200: 22 / 47 and 15 / 42;  449: 33 / 87 and 21 / 57;
-    600: 59 / 124 and 31 / 88;  2,048 by 4,096 x 1,024 128 / 330."""
-    return (x.dtype == torch.float32 and weight.dtype == torch.float32 and out.dtype == torch.float32 and x.shape[0] >= SPLIT_MIN_ROWS
-            and x.shape[1] >= SPLIT_MIN_K and x.shape[1] % 4 == 0 and max(x.numel(), weight.numel()) < 1 << 30 and x.is_contiguous() and weight.is_contiguous() and out.is_contiguous()
-            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
+    """Whether a float32 product goes through the tensor cores: what the kernel takes (whole 16-byte pieces, byte offsets in 32 bits, 65,535
+    tiles of 32 rows) where it is the faster one.  Everything else is the library's to compute or to refuse."""
+    return (all(t.dtype == torch.float32 and t.dim() == 2 and t.is_contiguous() for t in (x, weight, out))
+            and out.shape == (x.shape[0], weight.shape[0]) and x.shape[1] == weight.shape[1]
+            and SPLIT_MIN_ROWS <= x.shape[0] <= 65535 * 32 and x.shape[1] >= SPLIT_MIN_K and x.shape[1] % 4 == 0
+            and max(x.numel(), weight.numel()) < 1 << 30 and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+            and gemm_f32_split_preferred(x.shape[0], weight.shape[0], x.shape[1]))
 
 
 def gemm_f32_split(out: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, tile: Optional[Tuple[int, int]] = None,
