@@ -347,7 +347,8 @@ constexpr int kSortThreads = 1024;
 // Counts per expert, the experts' segments of sorted rows one behind the other, and the tiles of at most `tile_pairs` rows that
 // the grouped product cuts them into: segments[0 .. E] the first row of every expert (and the number of rows), then the tiles before
 // every expert (and their number).  One block.  The order of an expert's rows among themselves is not fixed; no result depends on
-// it.  row_token[slot]: the token whose row goes to sorted row `slot`.  slot_of[pair]: where the pair's row lies; -1 for a pair
+// it.  row_token[slot]: the token whose row goes to sorted row `slot`; 0 behind the last of them, for as many entries as there are pairs
+// whose expert is the input itself (those rows are gathered and never read).  slot_of[pair]: where the pair's row lies; -1 for a pair
 // whose expert is the input itself.
 // A pair's place in its segment comes out of the counting (kept in slot_of until the segments are known), and the lanes of a
 // warp that share an expert make one atomic of it: with an atomic per pair, twice, 4,096 pairs of 8 experts took 12.5 us, nearly
@@ -401,7 +402,7 @@ sort_pairs_kernel(int* __restrict__ segments, int* __restrict__ row_token, int* 
             rows += __shfl_sync(0xffffffffu, rs, 31);
             tiles += __shfl_sync(0xffffffffu, ts, 31);
         }
-        if (lane == 0) { segments[E] = rows; segments[2 * E + 1] = tiles; }
+        if (lane == 0) { start[E] = segments[E] = rows; segments[2 * E + 1] = tiles; }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n_pairs; i += kSortThreads) {        // a thread reads back the places that it wrote itself
@@ -413,6 +414,7 @@ sort_pairs_kernel(int* __restrict__ segments, int* __restrict__ row_token, int* 
         row_token[slot] = i / top;
         slot_of[i] = slot;
     }
+    for (int i = start[E] + threadIdx.x; i < n_pairs; i += kSortThreads) row_token[i] = 0;
 }
 
 // xs[slot_of[pair], :] = T(weights[pair] * x[pair / top, :]): the rows of the grouped product when a pair's weight multiplies

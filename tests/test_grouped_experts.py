@@ -60,3 +60,30 @@ def test_expert_products_at_tile_edges(counts, act, D, F, tile):
     # terms, and the last rounding; 2^-6 of the row's largest value covers both
     err = (y.double() - ref).abs().amax(1) / ref.abs().amax(1).clamp(min=1e-3)
     assert float(err.max()) < 2.0 ** -6, float(err.max())
+
+
+@pytest.mark.parametrize("counts,beside", [([5, 0, 33, 2], 7), ([0, 0, 3, 0], 40), ([0, 0, 0, 0], 9), ([16, 17, 64, 1], 0)])
+def test_pairs_whose_expert_is_the_input(counts, beside):
+    """`beside` pairs have no row among the sorted ones; what the index scratch held before is no row of theirs either."""
+    from cppvllm_b200.csrc import ops
+    dev, D, F, E = torch.device("cuda:0"), 136, 72, len(counts)
+    g = torch.Generator().manual_seed(beside)
+    ids = torch.cat([torch.full((n,), e) for e, n in enumerate(counts)] + [E + torch.randint(0, 3, (beside,), generator=g)])
+    P = len(ids)
+    ids = ids[torch.randperm(P, generator=g)].to(torch.int32).view(P, 1).to(dev)
+    wts = torch.rand(P, 1, generator=g).to(dev)
+    x = torch.randn(P, D, generator=g).to(BF).to(dev)
+    wgu, wd = ((torch.randn(E, n, m, generator=g) * m ** -0.5).to(BF).to(dev) for n, m in ((2 * F, D), (D, F)))
+    R = ops.grouped_rows_tcgen05(P, 1, E)
+    ints = dict(dtype=torch.int32, device=dev)
+    row_token = torch.full((R,), 1 << 30, **ints)
+    scratch = [torch.full((R, m), float("nan"), dtype=BF, device=dev) for m in (D, F, D)]
+    y = torch.empty(P, D, dtype=BF, device=dev)
+    ops.experts_grouped_tcgen05(y, x, ids, wts, wgu, wd, torch.empty(R // 128, **ints), row_token, torch.empty(P, **ints), *scratch, identity=3)
+    ops.check_device_errors(dev)
+    own = (ids >= E).double()
+    ref = _layer(x, ids, wts, wgu, wd, "silu", 0.0, 0.0) + own * wts.double() * x.double()
+    err = (y.double() - ref).abs().amax(1) / ref.abs().amax(1).clamp(min=1e-3)
+    assert float(err.max()) < 2.0 ** -6                        # as above
+    assert row_token[P - beside:P].tolist() == [0] * beside
+    assert int(row_token[:P].min()) >= 0 and int(row_token[:P].max()) < P
