@@ -418,7 +418,7 @@ sort_pairs_kernel(int* __restrict__ segments, int* __restrict__ row_token, int* 
 }
 
 // xs[slot_of[pair], :] = T(weights[pair] * x[pair / top, :]): the rows of the grouped product when a pair's weight multiplies
-// the expert's input.  Padding rows keep what they held; they are computed and never read.
+// the expert's input.
 __global__ void scatter_pairs_scaled_kernel(__nv_bfloat16* __restrict__ xs, const __nv_bfloat16* __restrict__ x,
                                             const int* __restrict__ slot_of, const float* __restrict__ weights, int D, int top) {
     pdl_trigger();

@@ -1516,8 +1516,9 @@ def experts_grouped_supported(x_dtype: torch.dtype, D: int, F: int) -> bool:
 
 
 def grouped_rows_tcgen05(num_tokens: int, top: int, num_experts: int) -> int:
-    """Rows of scratch the tcgen05 grouped path asks for (a few more than the pairs; segments lie one behind the other)."""
-    return ((num_tokens * top + 127) // 128 + num_experts) * 128
+    """Entries of the index scratch `row_token` of the tcgen05 grouped path: the pairs' tokens and, behind them, the experts' segments.  (The
+    rows themselves lie one behind the other: as many as there are pairs.)"""
+    return num_tokens * top + 2 * (num_experts + 1)
 
 
 GROUPED_TILE = 256          # pairs of a tile at most: an accumulator's columns.  Smaller tiles were slower at every size measured
@@ -1542,11 +1543,12 @@ def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, 
     """More tokens on the tcgen05 tensor cores: the pairs are sorted by expert (device side), the tokens' rows are gathered into
     that order, and two grouped products (the first with the gated activation as its epilogue) run on
     csrc/gemm_experts_tcgen05.cu's kernel; the last kernel adds a token's expert outputs up with its weights.  Scratch:
-    R = grouped_rows_tcgen05(T, top, E) rows: tile_expert int32 [R / 128], row_token int32 [R] (the pairs' tokens, then the experts'
-    segments), slot_of int32 [T * top], xs bf16 [R, D], hid bf16 [R, ff], rows bf16 [R, D].  `tile` fixes (GROUPED_TILE, grouped_blocks)."""
+    row_token int32 [grouped_rows_tcgen05(T, top, E)] (the pairs' tokens, then the experts' segments), slot_of int32 [T * top], xs bf16
+    [T * top, D], hid bf16 [T * top, ff], rows bf16 [T * top, D]; `tile_expert` is not read and may be None (the segments are the table of
+    tiles).  `tile` fixes (GROUPED_TILE, grouped_blocks)."""
     global _gemm_experts
-    _cuda(y, x, ids, weights, w_gate_up, w_down, tile_expert, row_token, slot_of, xs, hid, rows)
-    _contig(y, x, ids, weights, w_gate_up, w_down, tile_expert, row_token, slot_of, xs, hid, rows)
+    _cuda(y, x, ids, weights, w_gate_up, w_down, row_token, slot_of, xs, hid, rows)
+    _contig(y, x, ids, weights, w_gate_up, w_down, row_token, slot_of, xs, hid, rows)
     T, D = x.shape
     E, F2, _ = w_gate_up.shape
     gated = _expert_gated(activation, identity, weight_on_input)
@@ -1555,8 +1557,8 @@ def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, 
     bf = torch.bfloat16
     if (any(t.dtype != bf for t in (y, x, w_gate_up, w_down, xs, hid, rows)) or y.shape != x.shape or w_gate_up.shape != (E, F2, D)
             or w_down.shape != (E, D, F) or ids.dtype != torch.int32 or weights.dtype != torch.float32 or ids.shape != weights.shape
-            or any(t.dtype != torch.int32 for t in (tile_expert, row_token, slot_of)) or tile_expert.numel() < R // 128
-            or row_token.numel() < R or slot_of.numel() < P or xs.numel() < R * D or hid.numel() < R * F or rows.numel() < R * D):
+            or any(t.dtype != torch.int32 for t in (row_token, slot_of)) or row_token.numel() < R or slot_of.numel() < P
+            or xs.numel() < P * D or hid.numel() < P * F or rows.numel() < P * D):
         raise KernelError("experts_grouped_tcgen05: bf16 x, y, weights and scratch of the documented sizes; int32 index scratch")
     if _gemm_experts is None:
         lib = load_library("gemm_experts")
@@ -1565,7 +1567,7 @@ def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, 
     err = _ptr(error_flag(x.device))
     tile_pairs = tile[0] if tile is not None else GROUPED_TILE
     row_of = row_token.view(-1)[:P]
-    segments = row_token.view(-1)[P:P + 2 * (E + 1)]          # R is larger than P by 128 entries an expert or more
+    segments = row_token.view(-1)[P:R]
     _check(_moe_lib().cvb_sort_pairs(_ptr(segments), _ptr(row_of), _ptr(slot_of), _ptr(ids), c_int(T), c_int(E), c_int(top), c_int(tile_pairs),
                                      c_int(identity), err, _stream()), "sort_pairs")
     xs2, hid2, rows2 = xs.view(-1)[:P * D].view(P, D), hid.view(-1)[:P * F].view(P, F), rows.view(-1)[:P * D].view(P, D)
@@ -1576,8 +1578,9 @@ def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, 
         gather_rows(xs2, x, row_of)
 
     def product(out, a, w, n, k, mode):
+        blocks = tile[1] if tile is not None else grouped_blocks(k)
         _check(_gemm_experts.cvb_gemm_experts_bf16(_ptr(out), _ptr(a), _ptr(w), _ptr(segments), c_int(P), c_int(n), c_int(E), c_int(k), c_int(mode),
-                                                   c_int(tile_pairs), c_int(tile[1] if tile is not None else grouped_blocks(k)), c_float(limit), c_float(alpha), err, _stream()), "gemm_experts_bf16")
+                                                   c_int(tile_pairs), c_int(blocks), c_float(limit), c_float(alpha), err, _stream()), "gemm_experts_bf16")
     product(hid2, xs2, w_gate_up, F2, D, (4 if activation == "clamped" else 1) if gated else 3)
     product(rows2, hid2, w_down, D, F, 0)
     _check(_moe_lib().cvb_combine_pairs_bf16(_ptr(y), _ptr(rows2), _ptr(x), _ptr(slot_of), _ptr(None if weight_on_input else weights), c_int(T),
@@ -1609,18 +1612,19 @@ def routed_experts(y, x, ids, weights, w_gate_up, w_down, workspace=None, kernel
     expert_bytes = (3 if gated else 2) * D * F * x.element_size()
     grouped = kernel == "tcgen05" or (kernel == "" and grouped_experts_preferred(T * top, E, expert_bytes))
     if grouped and experts_grouped_supported(x.dtype, D, F):
-        R = grouped_rows_tcgen05(T, top, E)
+        # sized once for the largest step (the address must not move: captured graphs hold it)
+        most = workspace.max_tokens if workspace is not None else T
 
         def buf(name, n, dtype):
             if workspace is not None:
-                # sized once for the largest step (the address must not move: captured graphs hold it)
-                return workspace.flat(f"{name}_{E}_{top}", grouped_rows_tcgen05(workspace.max_tokens, top, E) * (n // R), dtype, zero=True)
+                return workspace.flat(f"{name}_{E}_{top}", n, dtype, zero=True)
             return torch.zeros(n, dtype=dtype, device=x.device)
         slot_of = workspace.rows("moe_slot_of", T, top, torch.int32) if workspace is not None else torch.empty(T * top, dtype=torch.int32, device=x.device)
-        return experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, buf("moe_tile_expert", R, torch.int32),
-                                       buf("moe_row_token", R, torch.int32), slot_of, buf(f"moe_xs{D}", R * D, x.dtype),
-                                       buf(f"moe_hid{F}", R * F, x.dtype), buf(f"moe_rows{D}", R * D, x.dtype), activation=activation,
-                                       weight_on_input=weight_on_input, identity=identity, limit=limit, alpha=alpha)
+        return experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, None,
+                                       buf("moe_row_token", grouped_rows_tcgen05(most, top, E), torch.int32), slot_of,
+                                       buf(f"moe_xs{D}", most * top * D, x.dtype), buf(f"moe_hid{F}", most * top * F, x.dtype),
+                                       buf(f"moe_rows{D}", most * top * D, x.dtype), activation=activation, weight_on_input=weight_on_input,
+                                       identity=identity, limit=limit, alpha=alpha)
     if workspace is not None:
         hid = workspace.rows("moe_hidden", T, top * F, x.dtype)
     else:

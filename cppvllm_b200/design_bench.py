@@ -354,9 +354,9 @@ def kernel_pairs(s, pk):
     wgu, wd = rnd(EXPERTS, 2 * F, D, scale=0.02), rnd(EXPERTS, D, F, scale=0.02)
     y = torch.empty(T, D, dtype=bf, device=d)
     R = ops.grouped_rows_tcgen05(T, TOP, EXPERTS)
-    scr2 = dict(tile_expert=torch.empty(R, dtype=torch.int32, device=d), row_token=torch.empty(R, dtype=torch.int32, device=d),
-                slot_of=torch.empty(T * TOP, dtype=torch.int32, device=d), xs=torch.empty(R, D, dtype=bf, device=d), hid=torch.empty(R, F, dtype=bf, device=d),
-                rows=torch.empty(R, D, dtype=bf, device=d))
+    scr2 = dict(tile_expert=None, row_token=torch.empty(R, dtype=torch.int32, device=d), slot_of=torch.empty(T * TOP, dtype=torch.int32, device=d),
+                xs=torch.empty(T * TOP, D, dtype=bf, device=d), hid=torch.empty(T * TOP, F, dtype=bf, device=d),
+                rows=torch.empty(T * TOP, D, dtype=bf, device=d))
     new = _us(lambda i: ops.experts_grouped_tcgen05(y, x, ids, wts, wgu, wd, **scr2))
     w_gate_up, w_down = rnd(2 * I, D, scale=0.02), rnd(D, I, scale=0.02)
     act = torch.empty(T, I, dtype=bf, device=d)

@@ -87,3 +87,21 @@ def test_pairs_whose_expert_is_the_input(counts, beside):
     assert float(err.max()) < 2.0 ** -6                        # as above
     assert row_token[P - beside:P].tolist() == [0] * beside
     assert int(row_token[:P].min()) >= 0 and int(row_token[:P].max()) < P
+
+
+def test_scratch_is_as_large_as_the_pairs():
+    """No room for padding: many experts with few pairs each ask for no more than the pairs and the experts' segments."""
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.parts.base import Workspace
+    dev, T, top, E, D, F = torch.device("cuda:0"), 40, 2, 64, 72, 40
+    g = torch.Generator().manual_seed(1)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32).to(dev)
+    wts, x = torch.rand(T, top, generator=g).to(dev), torch.randn(T, D, generator=g).to(BF).to(dev)
+    wgu, wd = ((torch.randn(E, n, m, generator=g) * m ** -0.5).to(BF).to(dev) for n, m in ((2 * F, D), (D, F)))
+    ws, y = Workspace(dev, T), torch.empty(T, D, dtype=BF, device=dev)
+    ops.routed_experts(y, x, ids, wts, wgu, wd, workspace=ws, kernel="tcgen05")
+    ops.check_device_errors(dev)
+    assert sum(b.numel() * b.element_size() for b in ws._buffers.values()) <= T * top * (2 * (2 * D + F) + 2 * 4) + 2 * (E + 1) * 4
+    ref = _layer(x, ids, wts, wgu, wd, "silu", 0.0, 0.0)
+    err = (y.double() - ref).abs().amax(1) / ref.abs().amax(1).clamp(min=1e-3)
+    assert float(err.max()) < 2.0 ** -6                        # as above
