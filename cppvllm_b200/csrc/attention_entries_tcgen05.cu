@@ -7,9 +7,9 @@
 // What bounds the mma.sync kernels is the legacy tensor path and the shared-memory reads that feed it: 64 query rows per block and
 // 64 keys per tile, every operand fragment through ldmatrix.  Here a block owns 256 query rows of one kv head as two tiles of 128 (row r
 // of a tile = token r / g, head r % g of the group), walks tiles of 128 entries, and the tensor core alternates between the two query
-// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, mma.sync -> now): chunks of 1,024 179 -> 26; a latent of
-// 96 + 32 under 16 heads 171 -> 37; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 45; keys that are values at 32/8 heads
-// (1,917 tokens of three requests behind a window of 1,024) 196 -> 44.
+// tiles, as in attention_tcgen05.cu.  Measured, 2,048 tokens at 16/8 heads of 128 (us, mma.sync -> now): chunks of 1,024 179 -> 27; a latent of
+// 96 + 32 under 16 heads 171 -> 39; a bias per distance (1,500 tokens and 548 behind 700) 211 -> 40; keys that are values at 32/8 heads
+// (1,917 tokens of three requests behind a window of 1,024) 196 -> 43.
 //   warp 0     producer: one lane per TMA box (page or 64 entries, times 64 columns, times key and value), 128-byte swizzle.  Key and
 //              value apart: two stages, each with the keys of tile i + 1 and the values of tile i (what one round reads).  Shared
 //              entries: four stages of one tile, read row-wise by S = Q K^T and transposed by O += P K;
@@ -20,8 +20,8 @@
 //              S; O is rescaled in tensor memory when some row of the warp has a new maximum.  The reference is the maximum itself, so that a row's
 //              largest probability is 1 and rounds to 1: with one that followed only after 2^8, layers were 1 to 5 % further from float64 (capped
 //              scores 4.00e-3 -> 4.22e-3, a bias per distance 4.82e-3 -> 4.90e-3) and 2 to 5 % faster (a bias per distance 79 us against 83).
-//              Without a cap or a distance term one exponential in three is made on the multiply-add units (27.7, 41.2, -, 46.3); with
-//              them those units have no room.
+//              All exponentials are the special-function unit's (a third of them as a polynomial on the multiply-add units: 25.5, 36.0,
+//              -, 40.8 us where 26.8, 39.1, 39.9, 42.7, and coarser: attention_tcgen05.cu).
 // The tiles a block walks are a list: pooled blocks any of its tokens sees (plane 1), kept first tokens that lie wholly before the
 // rest, then the tokens from the first one its first token sees to its last token; a query tile skips list entries it sees nothing of.
 //   distance terms: bias[h, min(p - j, L - 1)] or -r1_h ln(1 + r2_h (p - j)) come from a table in shared memory, one row per head of
@@ -512,7 +512,7 @@ attn_entries_tcgen05_kernel(const __grid_constant__ CUtensorMap map, const Entry
                         const int c = h * 64 + 2 * k;
                         const float2 s = make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1]));
                         const float2 arg = TERMS ? __fadd2_rn(s, neg_m2) : __ffma2_rn(s, scale2, neg_m2);
-                        const float2 pr = !TERMS && k % 3 == 2 ? ex2_fma2(arg) : make_float2(ex2(arg.x), ex2(arg.y));
+                        const float2 pr = make_float2(ex2(arg.x), ex2(arg.y));
                         sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
                         __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
                         packed[k] = *reinterpret_cast<uint32_t*>(&hh);

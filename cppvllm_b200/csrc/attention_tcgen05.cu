@@ -24,11 +24,12 @@
 //              into tensor memory with tcgen05.st.  The output accumulator stays in tensor memory; it is rescaled (read,
 //              multiplied, written back by the row's thread) only when the running maximum of some row of the warp has
 //              grown by more than 2^8 since the reference was set, which happens in the first tiles and then hardly
-//              ever.  The result is exact: the same reference scales P and the row sum.  One exponential in three is made on the
-//              multiply-add units (ex2_fma2): all on the special-function unit, two tiles take its whole 2,048 cycles a round.
-// A tile's chain (scores, exponentials, products) sets the pace: 512 tokens behind 7,680 at 32/8 heads / a prompt of 2,048 at 16/8 heads
-// 73.4 / 39.2 us; issue by the whole warp 66.9 / 35.4; a third of the exponentials on the multiply-add units 63.9 / 33.3 (an eighth 66.1 /
-// 34.8, a quarter 64.6 / 34.0, half 68.3 / 35.4); two halves 62.2 / 32.3.  Scores by 64 keys in two buffers a tile, so that a tile's products
+//              ever.  The result is exact: the same reference scales P and the row sum.
+// A tile's chain (scores, exponentials, products) sets the pace, and the exponentials of two tiles take the special-function unit's whole
+// 2,048 cycles a round: 512 tokens behind 7,680 at 32/8 heads / a prompt of 2,048 at 16/8 heads 72.4 / 37.2 us; issue by the whole warp 66.9 /
+// 35.4; two halves 64.8 / 32.8.  A third of the exponentials as a polynomial of degree 5 on the multiply-add units (61.8 / 31.5) was taken
+// back: up to 1.71e-7 from their value and 6.6e-8 in the mean square where the unit's are 1.46e-7 and 4.2e-8 to 6.0e-8, and probabilities at
+// a rounding's edge moved the layers' outputs by up to 3e-4.  Scores by 64 keys in two buffers a tile, so that a tile's products
 // and exponentials need not wait for one another, were slower (75.6 / 38.7: products of 128 x 64 read shared memory for 48 cycles and
 // compute for 32), and so was a ring of five tiles given back one by one (the loads are not what a round waits for).
 // A grid of few query blocks with many key tiles each (a portion behind a long context) leaves SMs idle, so the launcher
@@ -424,7 +425,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap kv_map, const Tc
                     for (int k = 0; k < 32; ++k) {
                         const int c = h * 64 + 2 * k;
                         const float2 arg = __ffma2_rn(make_float2(__uint_as_float(v[c]), __uint_as_float(v[c + 1])), scale2, neg_m2);
-                        const float2 pr = k % 3 == 2 ? ex2_fma2(arg) : make_float2(ex2(arg.x), ex2(arg.y));
+                        const float2 pr = make_float2(ex2(arg.x), ex2(arg.y));
                         sum2[k & 1] = __fadd2_rn(sum2[k & 1], pr);
                         __nv_bfloat162 hh = __floats2bfloat162_rn(pr.x, pr.y);
                         packed[k] = *reinterpret_cast<uint32_t*>(&hh);

@@ -182,24 +182,6 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// 2^x of two numbers on the multiply-add units, for x up to 126: x = n + f with n the nearest integer; 2^f by the polynomial of degree 5 whose
-// largest relative error over [-1/2, 1/2] is smallest among those with p(0) = 1 (a weighted least squares fit whose weights were
-// driven to equal errors), 1.7e-7 in float arithmetic; 2^n from its exponent bits.  As with ex2, x below -126 gives 0 and a NaN a NaN.
-__device__ __forceinline__ float2 ex2_fma2(float2 x) {
-    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x.x));                       // -127: its exponent bits are those of 0
-    asm("max.NaN.f32 %0, %0, 0fC2FE0000;" : "+f"(x.y));
-    const float2 magic = make_float2(12582912.f, 12582912.f);                 // 1.5 * 2^23: the sum's lowest bits are n
-    const float2 t = __fadd2_rn(x, magic);
-    const float2 f = __fadd2_rn(x, __ffma2_rn(t, make_float2(-1.f, -1.f), magic));
-    float2 p = make_float2(0.0013264727313071489f, 0.0013264727313071489f);
-    p = __ffma2_rn(p, f, make_float2(0.009671512991189957f, 0.009671512991189957f));
-    p = __ffma2_rn(p, f, make_float2(0.05550733581185341f, 0.05550733581185341f));
-    p = __ffma2_rn(p, f, make_float2(0.24022242426872253f, 0.24022242426872253f));
-    p = __ffma2_rn(p, f, make_float2(0.6931470036506653f, 0.6931470036506653f));
-    p = __ffma2_rn(p, f, make_float2(1.f, 1.f));
-    const float2 e = make_float2(__int_as_float((__float_as_int(t.x) << 23) + 0x3f800000), __int_as_float((__float_as_int(t.y) << 23) + 0x3f800000));
-    return __fmul2_rn(p, e);
-}
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

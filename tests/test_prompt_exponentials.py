@@ -1,5 +1,5 @@
-"""Exponentials of the prompt kernels, of which every third pair is made on the multiply-add units: a NaN, a score far below the row's
-largest and a row's only key, at neighbouring columns, so that both kinds are met."""
+"""Exponentials of the prompt kernels: a NaN, a score far below the row's largest and a row's only key, at neighbouring columns (they are made in
+pairs, and a tile's in two halves)."""
 import pytest
 import torch
 
@@ -49,7 +49,7 @@ def test_a_score_far_below_the_largest_has_no_weight(key):
 
 
 def test_rows_with_one_key_give_its_value():
-    """Whichever unit made the only probability of a row."""
+    """Whichever column the only probability of a row lies in."""
     q, k, v = _random(0, 1 + N)
     q[:, :, :], k[:, :, :] = 0.0, 0.0
     q[:, :, 0] = 32.0
@@ -57,3 +57,21 @@ def test_rows_with_one_key_give_its_value():
     out = _attend(q, k, v, 1.0, first=0)
     # the scores reach 6,000 in base 2, where a float's last place is 2^-11: 2^-12 in the exponent, and the two roundings to bf16
     torch.testing.assert_close(out.float(), v.repeat_interleave(H // KV, 1).float(), atol=0.0, rtol=2.0 ** -7)
+
+
+def test_a_keys_weight_does_not_depend_on_its_column():
+    """Two keys with a weight, one of weight 1; the other one's probability is the same number wherever it lies in a tile.  Of 131,072 scores some
+    have an exponential within 1e-7 of the middle between two bf16, where two ways to make it would round apart."""
+    n, g = 32768, torch.Generator().manual_seed(11)
+    q, k, v = torch.zeros(n, H, HD), torch.zeros(C + n, KV, HD), torch.zeros(C + n, KV, HD)
+    q[:, :, 0], q[:, :, 2], q[:, :, 1] = 0.5 + 7.0 * torch.rand(n, H, generator=g), torch.rand(n, H, generator=g), 1.0
+    k[:, :, 1] = -30000.0                                    # no weight
+    k[60] = 0.0                                              # weight 1, value 0
+    first = None
+    for column in (0, 1, 2, 3, 4, 5, 64, 65, 66, 67, 68, 69):
+        k2, v2 = k.clone(), v.clone()
+        k2[column, :, 0], k2[column, :, 2], k2[column, :, 1] = -1.0, -2.0 ** -7, 0.0
+        v2[column] = 1.0
+        out = _attend(q.to(DT), k2.to(DT), v2.to(DT), 0.7)
+        first = out if first is None else first
+        assert torch.equal(out, first), (column, int((out != first).any(-1).sum()))
