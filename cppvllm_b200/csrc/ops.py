@@ -935,8 +935,9 @@ def ssd_tcgen05_supported(dim: int, vdim: int) -> bool:
 def ssd_chunks(y: torch.Tensor, u: torch.Tensor, dt: torch.Tensor, log_decay: torch.Tensor, skip: torch.Tensor, state: torch.Tensor, cu_seqlens,
                state_slots, q_lens, num_heads: int, groups: int, dim: int, vdim: int, ends: Optional[torch.Tensor] = None,
                decays: Optional[torch.Tensor] = None, kernel: str = "") -> torch.Tensor:
-    """Per request and head: S <- exp(log_decay) S + dt B x^T, y = S^T C + skip_h x over the request's tokens of this step, in chunks of 64 tokens on
-    the tensor cores (128 on csrc/ssd_tcgen05.cu's kernels, see ssd_tcgen05_supported; `kernel` = "mma" | "tcgen05" fixes the choice); u bf16 [T, H vdim + 2 G dim] rows [x | B | C]; y float32 [T, H * vdim].  Portions of more than 64 tokens go through `ends`
+    """Per request and head: S <- exp(log_decay) S + dt B x^T, y = S^T C + skip_h x over the request's tokens of this step, in chunks of 64
+    tokens on the tensor cores, or of 128 by csrc/ssd_tcgen05.cu's kernels (see ssd_tcgen05_supported; `kernel` = "mma" | "tcgen05" fixes the
+    choice); u bf16 [T, H vdim + 2 G dim] rows [x | B | C]; y float32 [T, H * vdim].  Portions of more than one chunk go through `ends`
     (float32, H dim vdim per chunk of such a portion) and `decays` (float32, H per chunk)."""
     _cuda(y, u, dt, log_decay, skip, state, cu_seqlens, state_slots, ends, decays); _contig(y, u, dt, log_decay, skip, cu_seqlens, state_slots, ends, decays)
     sp, sf, n_slots = _state_args(state)
@@ -1564,27 +1565,26 @@ def experts_grouped_tcgen05(y, x, ids, weights, w_gate_up, w_down, tile_expert, 
         lib = load_library("gemm_experts")
         lib.cvb_gemm_experts_bf16.restype = c_int
         _gemm_experts = lib
-    err = _ptr(error_flag(x.device))
+    # addresses instead of views of the scratch: a view costs a microsecond, and steps of a few hundred tokens wait for the host
+    err, stream = _ptr(error_flag(x.device)), _stream()
     tile_pairs = tile[0] if tile is not None else GROUPED_TILE
-    row_of = row_token.view(-1)[:P]
-    segments = row_token.view(-1)[P:R]
-    _check(_moe_lib().cvb_sort_pairs(_ptr(segments), _ptr(row_of), _ptr(slot_of), _ptr(ids), c_int(T), c_int(E), c_int(top), c_int(tile_pairs),
-                                     c_int(identity), err, _stream()), "sort_pairs")
-    xs2, hid2, rows2 = xs.view(-1)[:P * D].view(P, D), hid.view(-1)[:P * F].view(P, F), rows.view(-1)[:P * D].view(P, D)
+    x_p, xs_p, hid_p, rows_p, slot_p = _ptr(x), _ptr(xs), _ptr(hid), _ptr(rows), _ptr(slot_of)
+    tokens_p, segments_p = _ptr(row_token), c_void_p(row_token.data_ptr() + 4 * P)
+    moe = _moe_lib()
+    _check(moe.cvb_sort_pairs(segments_p, tokens_p, slot_p, _ptr(ids), c_int(T), c_int(E), c_int(top), c_int(tile_pairs), c_int(identity), err,
+                              stream), "sort_pairs")
     if weight_on_input:     # a pair's weight scales its row on the way in
-        _check(_moe_lib().cvb_scatter_pairs_scaled_bf16(_ptr(xs2), _ptr(x), _ptr(slot_of), _ptr(weights), c_int(T), c_int(D), c_int(top),
-                                                        _stream()), "scatter_pairs_scaled")
+        _check(moe.cvb_scatter_pairs_scaled_bf16(xs_p, x_p, slot_p, _ptr(weights), c_int(T), c_int(D), c_int(top), stream), "scatter_pairs_scaled")
     else:
-        gather_rows(xs2, x, row_of)
+        _check(core().cvb_gather_rows(xs_p, x_p, tokens_p, c_int(P), c_int(D), c_int(T), c_int(dtype_code(bf)), stream), "gather_rows")
 
     def product(out, a, w, n, k, mode):
         blocks = tile[1] if tile is not None else grouped_blocks(k)
-        _check(_gemm_experts.cvb_gemm_experts_bf16(_ptr(out), _ptr(a), _ptr(w), _ptr(segments), c_int(P), c_int(n), c_int(E), c_int(k), c_int(mode),
-                                                   c_int(tile_pairs), c_int(blocks), c_float(limit), c_float(alpha), err, _stream()), "gemm_experts_bf16")
-    product(hid2, xs2, w_gate_up, F2, D, (4 if activation == "clamped" else 1) if gated else 3)
-    product(rows2, hid2, w_down, D, F, 0)
-    _check(_moe_lib().cvb_combine_pairs_bf16(_ptr(y), _ptr(rows2), _ptr(x), _ptr(slot_of), _ptr(None if weight_on_input else weights), c_int(T),
-                                             c_int(D), c_int(top), _stream()),
+        _check(_gemm_experts.cvb_gemm_experts_bf16(out, a, _ptr(w), segments_p, c_int(P), c_int(n), c_int(E), c_int(k), c_int(mode), c_int(tile_pairs),
+                                                   c_int(blocks), c_float(limit), c_float(alpha), err, stream), "gemm_experts_bf16")
+    product(hid_p, xs_p, w_gate_up, F2, D, (4 if activation == "clamped" else 1) if gated else 3)
+    product(rows_p, hid_p, w_down, D, F, 0)
+    _check(moe.cvb_combine_pairs_bf16(_ptr(y), rows_p, x_p, slot_p, _ptr(None if weight_on_input else weights), c_int(T), c_int(D), c_int(top), stream),
            "combine_pairs")
     return y
 
@@ -2426,7 +2426,7 @@ def project_rows(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, rows:
     if gemv_stream_supported(x.dtype, weight, rows):
         return gemv_stream_bf16(out, x, weight, rows, dependent=dependent)
     if rows > GEMV_MAX_ROWS or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
-        if gemm_f32_split_supported(x, weight, out):
+        if x.dtype == torch.float32 and gemm_f32_split_supported(x, weight, out):
             return gemm_f32_split(out, x, weight, dependent=dependent)
         return linear(x, weight, out=out)
     key = (weight.shape[0], weight.shape[1], rows if rows <= 2 else (8 if rows <= 8 else 16))
@@ -2598,8 +2598,10 @@ def gemm_f32_split_preferred(rows: int, n_out: int, k: int) -> bool:
 def gemm_f32_split_supported(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor) -> bool:
     """Whether a float32 product goes through the tensor cores: what the kernel takes (whole 16-byte pieces, byte offsets in 32 bits, 65,535
     tiles of 32 rows) where it is the faster one.  Everything else is the library's to compute or to refuse."""
-    return (all(t.dtype == torch.float32 and t.dim() == 2 and t.is_contiguous() for t in (x, weight, out))
-            and out.shape == (x.shape[0], weight.shape[0]) and x.shape[1] == weight.shape[1]
+    if x.dtype != torch.float32 or weight.dtype != torch.float32 or out.dtype != torch.float32 or x.dim() != 2 or weight.dim() != 2:
+        return False
+    return (out.shape == (x.shape[0], weight.shape[0]) and x.shape[1] == weight.shape[1]
+            and x.is_contiguous() and weight.is_contiguous() and out.is_contiguous()
             and SPLIT_MIN_ROWS <= x.shape[0] <= 65535 * 32 and x.shape[1] >= SPLIT_MIN_K and x.shape[1] % 4 == 0
             and max(x.numel(), weight.numel()) < 1 << 30 and (x.data_ptr() | weight.data_ptr()) % 16 == 0
             and gemm_f32_split_preferred(x.shape[0], weight.shape[0], x.shape[1]))

@@ -105,3 +105,25 @@ def test_scratch_is_as_large_as_the_pairs():
     ref = _layer(x, ids, wts, wgu, wd, "silu", 0.0, 0.0)
     err = (y.double() - ref).abs().amax(1) / ref.abs().amax(1).clamp(min=1e-3)
     assert float(err.max()) < 2.0 ** -6                        # as above
+
+
+def test_a_call_makes_no_tensors():
+    """Small steps wait for the host, where a view of the scratch costs as much as a launch's share of it."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from cppvllm_b200.csrc import ops
+    from cppvllm_b200.parts.base import Workspace
+    dev, T, top, E, D, F = torch.device("cuda:0"), 40, 2, 8, 72, 40
+    made = []
+
+    class Count(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            made.append(str(func))
+            return func(*args, **(kwargs or {}))
+    ids, wts = torch.zeros(T, top, dtype=torch.int32, device=dev), torch.rand(T, top, device=dev)
+    x, y, wgu, wd = (torch.zeros(*s, dtype=BF, device=dev) for s in ((T, D), (T, D), (E, 2 * F, D), (E, D, F)))
+    ws = Workspace(dev, T)
+    ops.routed_experts(y, x, ids, wts, wgu, wd, workspace=ws, kernel="tcgen05")       # makes the scratch
+    with Count():
+        ops.routed_experts(y, x, ids, wts, wgu, wd, workspace=ws, kernel="tcgen05")
+    ops.check_device_errors(dev)
+    assert made == []
