@@ -2,8 +2,8 @@
 //
 // The rows of X [P, K] are the steps' (token, expert) pairs sorted by expert, W holds the experts' matrices one below the
 // other (N rows of K each), and every row is multiplied by its expert's matrix:
-//   plain   C[p, :] = X[p, :] W_e^T                                      (kPlain; kRelu2: relu(T(.))^2)
-//   gated   C[p, :] = f(T(X Wg_e^T), T(X Wu_e^T)),  W_e = [Wg_e; Wu_e]   (kSwiglu, kClamped)
+//   plain   C[p, :] = X[p, :] W_e^T                                      (kExpPlain; kExpRelu2: relu(T(.))^2)
+//   gated   C[p, :] = f(T(X Wg_e^T), T(X Wu_e^T)),  W_e = [Wg_e; Wu_e]   (kExpSwiglu, kExpClamped)
 //
 // What bounds it.  Many rows per expert: the power limit.  8 experts of 512 pairs, K 4,096, 9,472 gated weight rows run at 1,385
 // TFLOP/s while the clock falls from 1.6 to 1.2 GHz (a cuBLAS product in a row on this machine: 1,383), so what is left to gain is

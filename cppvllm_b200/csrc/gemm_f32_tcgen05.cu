@@ -21,8 +21,10 @@
 //   warps 8-15  add the partial sums of the stage before (accumulators alternate) and store C.
 // With few tiles the blocks of a cluster share a tile's K and add their sums up through distributed shared memory.
 //
-// What bounds it: shared memory (a product of parts of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, and the parts have to
-// be written) and, close behind, the cuts (about six instructions an element).  449 rows by 4,096 x 1,024: 86 us as a float32
+// What bounds it: no unit alone.  At 2,048 rows by 4,096 x 4,096 the tensor pipe is active for 54 % of the cycles, shared memory (a product of
+// parts of 128 x 128 x 16 reads 8 KB in the 64 cycles it takes, and the parts have to be written) for 61, the issue slots, mostly the cuts', for
+// 45, and the cutting warps wait for their rows from the L2 or memory (W is read again by every 128 rows of A: 327 MB where 101 are
+// needed).  449 rows by 4,096 x 1,024: 86 us as a float32
 // library product, 33 with parts cut off, now 28 (134 TFLOP/s of float32 work); by 1,024 x 2,048 57, 21, now 18; 2,048 rows by 4,096 x 1,024 330,
 // 128, now 108 (159 TFLOP/s).
 // Every wait is bounded by a cycle count; one that runs out records error 5 and the block carries on to its end.  The kernel may start while
